@@ -15,6 +15,7 @@
 #include "../../include/lddmm_b200.h"
 #include "common.cuh"
 #include "cross.cuh"
+#include "gauss.cuh"
 #include "kernels.cuh"
 #include "layout.h"
 #include "lbfgs.cuh"
@@ -171,6 +172,12 @@ struct lddmm_ctx {
   PairState *st = nullptr;
   float4 *qs = nullptr, *as = nullptr, *us = nullptr, *ls = nullptr;
   double *q64 = nullptr, *p64 = nullptr;
+  // 3D Gaussian per-step sweeps (gauss.cuh): statistics of the 32-point blocks, the split
+  // items' FP64 parts and arrival counts
+  bool gauss = false;
+  float4 *gbox = nullptr, *gwa = nullptr, *gwu = nullptr;
+  double *gpart = nullptr;
+  unsigned int *gcnt = nullptr;
   float4 *dbb = nullptr, *tbb = nullptr;  // 32-element block boxes (varifold culling)
   float4 *ec = nullptr, *en = nullptr, *el = nullptr, *tc = nullptr, *tn = nullptr,
          *tl = nullptr;
@@ -251,6 +258,8 @@ lddmm_ctx::~lddmm_ctx() {
   dfree(cl_segs, stream); dfree(cl_cta_seg, stream); dfree(cl_job, stream);
   dfree(cl_job_src, stream);
   dfree(dbb, stream); dfree(tbb, stream);
+  dfree(gbox, stream); dfree(gwa, stream); dfree(gwu, stream); dfree(gpart, stream);
+  dfree(gcnt, stream);
   if (own_stream && stream) cudaStreamDestroy(stream);
 }
 
@@ -291,6 +300,26 @@ static cudaError_t launch_sweep(const Op &op, const int2 *items, int n_items, in
                 items, S);
 }
 
+// Statistics and split plan of step t's Gaussian sweep (gauss.cuh).
+static GaussStats gauss_stats(const lddmm_ctx &c, int t) {
+  const size_t nb = (size_t)c.NPtot / kSub;
+  GaussStats gs;
+  gs.box = c.gbox + 2 * nb * t;
+  gs.wa = c.gwa + nb * t;
+  gs.wu = c.gwu + nb * (t & 1);
+  gs.box_n = c.gbox + 2 * nb * (t + 1);
+  gs.wu_n = t > 0 ? c.gwu + nb * ((t - 1) & 1) : nullptr;
+  return gs;
+}
+
+// Weights of alpha at every step, once per evaluation (of u: launch_gather).
+static cudaError_t gauss_begin(lddmm_ctx &c) {
+  if (!c.gauss) return cudaSuccess;
+  const long long nb = (long long)c.T * c.NPtot / kSub;
+  return launch(gauss_alpha_kernel, (unsigned)std::min<long long>((nb + 7) / 8, 2048), 256, 0,
+                c.stream, (const float4 *)c.as, nb, c.gwa);
+}
+
 template <int D, int ORDER>
 static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
   ShootOp<D, ORDER> op;
@@ -305,6 +334,12 @@ static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
   op.vlc64 = vlc;
   op.tile_part = c.reg_part + (size_t)t * c.ntile_tot;
   op.t = t;
+  if constexpr (D == 3 && ORDER == -1) {
+    if (c.gauss)
+      return launch(gauss_shoot_kernel<kWarps>, (unsigned)(c.n_pt_items2 * c.S_shoot),
+                    kWarps * 32, 0, c.stream, op, gauss_stats(c, t), (const int2 *)c.pt_items2,
+                    SplitPlan{c.S_shoot, c.gpart, c.gcnt});
+  }
   // packed FP32x2 form of the same sweep (bitwise the same sums), on one- or two-tile
   // work items (c.tpw_shoot; the default rule and the autotuner pick it).  Two tiles
   // per item serve four rows per lane from each staged column: the Gaussian sweep,
@@ -338,6 +373,12 @@ static cudaError_t adjoint_impl(lddmm_ctx &c, int t, double *g, double *pdot) {
   op.ls_n = (t > 0) ? c.ls + (size_t)((t - 1) & 1) * c.NPtot : nullptr;
   op.pdot64 = pdot;
   op.t = t;
+  if constexpr (D == 3 && ORDER == -1) {
+    if (c.gauss)
+      return launch(gauss_adjoint_kernel<kWarps>, (unsigned)(c.n_pt_items2 * c.S_adj),
+                    kWarps * 32, 0, c.stream, op, gauss_stats(c, t), (const int2 *)c.pt_items2,
+                    SplitPlan{c.S_adj, c.gpart, c.gcnt});
+  }
   // packed FP32x2 form of the same sweep (bitwise the same sums), one- or two-tile
   // items as in shoot_impl (c.tpw_adj; Gaussian at 163,842 landmarks: 23.3 -> 22.0 ms
   // with two tiles, at 2 CTAs per SM instead of 3)
@@ -600,9 +641,14 @@ static cudaError_t launch_geometry(lddmm_ctx &c, const double *q64T) {
 static cudaError_t launch_gather(lddmm_ctx &c, const double *q64T, float4 *un, float4 *ln,
                                  double *dq_out) {
   const unsigned nb = (unsigned)(((long long)c.NPtot * kGatherLanes + 127) / 128);
-  if (c.D == 3)
-    return launch(gather_kernel<3>, nb, 128, 0, c.stream, c.pd, c.act, c.pt_pair, c.NPtot,
-                  c.adj_ptr, c.adj, c.dcdd, q64T, c.XT, c.p64, un, ln, dq_out, c.T);
+  if (c.D == 3) {
+    CUE(launch(gather_kernel<3>, nb, 128, 0, c.stream, c.pd, c.act, c.pt_pair, c.NPtot,
+               c.adj_ptr, c.adj, c.dcdd, q64T, c.XT, c.p64, un, ln, dq_out, c.T));
+    if (!c.gauss || !un) return cudaSuccess;
+    const long long nblk = c.NPtot / kSub;  // weights of the first backward step's u
+    return launch(gauss_alpha_kernel, (unsigned)((nblk + 3) / 4), 128, 0, c.stream,
+                  (const float4 *)un, nblk, c.gwu + nblk * ((c.T - 1) & 1));
+  }
   return launch(gather_kernel<2>, nb, 128, 0, c.stream, c.pd, c.act, c.pt_pair, c.NPtot,
                 c.adj_ptr, c.adj, c.dcdd, q64T, c.XT, c.p64, un, ln, dq_out, c.T);
 }
@@ -1305,10 +1351,29 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
       c.cycle_grid_lm = bc * sms;
     }
   }
+  if (c.D == 3 && c.order == -1 && cf.persistent <= 0) {
+    // 3D Gaussian per-step sweeps: S independent CTAs per 128-row item (default 8: at
+    // 9,001 / 40,962 / 163,842 landmarks 8 is within 3 % of the best of 1..32; fewer
+    // leave SMs idle at the end of a sweep, 1: 119 / 859 / 7065 us per shooting step
+    // against 47 / 510 / 6096)
+    const size_t nb = (size_t)c.NPtot / kSub;
+    if (cf.cluster_shoot <= 0) c.S_shoot = 8;
+    if (cf.cluster_adjoint <= 0) c.S_adj = 8;
+    CU(dalloc(c.stream, &c.gbox, 2 * nb * (c.T + 1)));
+    CU(dalloc(c.stream, &c.gwa, nb * c.T));
+    CU(dalloc(c.stream, &c.gwu, 2 * nb));
+    CU(dalloc(c.stream, &c.gpart, (size_t)c.n_pt_items2 * std::max(c.S_shoot, c.S_adj) *
+                                      kGaussRows * AdjointOp<3, -1>::NA));
+    CU(dalloc(c.stream, &c.gcnt, c.n_pt_items2));
+    CU(launch(gauss_box_kernel, (unsigned)((nb + 3) / 4), 128, 0, c.stream, (const float4 *)c.qs,
+              (const int *)c.pt_pair, (int)nb, c.gbox));
+    c.gauss = true;
+  }
   if (cf.autotune >= 0) {
     const int rc = autotune(c, cf);
     if (rc) return rc;
   }
+  if (c.persistent) c.gauss = false;
   *out = cp.release();
   return 0;
 }
@@ -1377,6 +1442,7 @@ extern "C" int lddmm_ctx_launch_shape(const lddmm_ctx *c, int *o, int n) {
 static cudaError_t run_eval(lddmm_ctx &c, double *g_out, double *f_out, double *vlc,
                             bool grad) {
   const int D = c.D;
+  CUE(gauss_begin(c));
   if (c.persistent) {
     CUE(c.shoot_all(c, vlc));
   } else {
@@ -1479,6 +1545,7 @@ extern "C" int lddmm_shoot(lddmm_ctx *ctx, const double *alp, double *nde_stk, d
   double *vlc = nullptr;
   CU(dalloc(c.stream, &vlc, (size_t)c.T * c.NPtot * D));
   cudaError_t e = reset_sync(c);
+  if (e == cudaSuccess) e = gauss_begin(c);
   if (e == cudaSuccess && c.persistent) e = c.shoot_all(c, vlc);
   for (int t = 0; t < c.T && e == cudaSuccess && !c.persistent; ++t)
     e = c.shoot(c, t, vlc + (size_t)t * c.NPtot * D);
@@ -1951,6 +2018,7 @@ extern "C" int lddmm_ctx_time_sweeps(lddmm_ctx *ctx, int reps, double *ms4) {
   CU(reset_sync(c));
   for (int r = 0; r < reps && err == cudaSuccess; ++r) {
     cudaEventRecord(ev[2 * nev], c.stream);
+    if (err == cudaSuccess) err = gauss_begin(c);
     if (c.persistent) {
       cudaEventRecord(ev[0], c.stream);
       err = c.shoot_all(c, nullptr);
@@ -2114,8 +2182,13 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
     *S = bS;
     *tpw = bT;
   };
-  tune_step(0, &c.S_shoot, &c.tpw_shoot, cf.cluster_shoot > 0);
-  tune_step(1, &c.S_adj, &c.tpw_adj, cf.cluster_adjoint > 0);
+  if (c.gauss) {
+    CU(gauss_begin(c));
+    CU(cudaMemsetAsync(c.gwu, 0, sizeof(float4) * 2 * c.NPtot / kSub, c.stream));
+  } else {
+    tune_step(0, &c.S_shoot, &c.tpw_shoot, cf.cluster_shoot > 0);
+    tune_step(1, &c.S_adj, &c.tpw_adj, cf.cluster_adjoint > 0);
+  }
   if (err == cudaSuccess && c.has_vfd && cf.cluster_varifold <= 0) {
     float best = 1e30f;
     int bS = c.S_vfd;
@@ -2251,6 +2324,7 @@ extern "C" int lddmm_dq_kernel(int dim, int n, const double *q, const double *l,
   CU(cudaMemcpyAsync(c.ls, hl.data(), sizeof(float4) * c.NPtot, cudaMemcpyHostToDevice, c.stream));
   CU(cudaMemcpyAsync(c.as, hr.data(), sizeof(float4) * c.NPtot, cudaMemcpyHostToDevice, c.stream));
   CU(launch_set_active(c, 1));
+  c.gauss = false;  // l and r are not a step's operands (u = l + r / 2): the general sweep
   CU(c.adjoint(c, 0, nullptr, pd));
   std::vector<double> h((size_t)c.NPtot * dim);
   CU(cudaMemcpyAsync(h.data(), pd, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c.stream));

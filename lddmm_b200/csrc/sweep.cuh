@@ -72,11 +72,12 @@ __device__ __forceinline__ void run_sub(const Op &op, const float4 (*sj)[kSub], 
 }
 
 // Warps -> CTA (shared memory) -> cluster (DSMEM) reduction of a tile's row sums and
-// the finalisation by cluster rank 0 (shared by both sweep kernels).
+// the finalisation by cluster rank 0 (shared by the sweep kernels).  v0, v1: the warp's
+// sums of rows lane and 32 + lane.
 template <class Op, int W>
 __device__ __forceinline__ void finish_tile(const Op &op, int p, int tile, int rank, int S,
-                                            const float (&hi0)[Op::NA], const float (&lo0)[Op::NA],
-                                            const float (&hi1)[Op::NA], const float (&lo1)[Op::NA]) {
+                                            const double (&v0)[Op::NA],
+                                            const double (&v1)[Op::NA]) {
   constexpr int NA = Op::NA;
   __shared__ double s_red[W][kTile][NA];
   __shared__ double s_cta[kTile][NA];
@@ -84,8 +85,8 @@ __device__ __forceinline__ void finish_tile(const Op &op, int p, int tile, int r
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int a = 0; a < NA; ++a) {
-    s_red[warp][lane][a] = (double)hi0[a] + (double)lo0[a];
-    s_red[warp][32 + lane][a] = (double)hi1[a] + (double)lo1[a];
+    s_red[warp][lane][a] = v0[a];
+    s_red[warp][32 + lane][a] = v1[a];
   }
   __syncthreads();
   double v[NA];
@@ -117,6 +118,19 @@ __device__ __forceinline__ void finish_tile(const Op &op, int p, int tile, int r
     const double tot = block_sum(e, s_scr);
     if (threadIdx.x == 0) op.write_tile(p, tile, tot);
   }
+}
+
+template <class Op, int W>
+__device__ __forceinline__ void finish_tile(const Op &op, int p, int tile, int rank, int S,
+                                            const float (&hi0)[Op::NA], const float (&lo0)[Op::NA],
+                                            const float (&hi1)[Op::NA], const float (&lo1)[Op::NA]) {
+  double v0[Op::NA], v1[Op::NA];
+#pragma unroll
+  for (int a = 0; a < Op::NA; ++a) {
+    v0[a] = (double)hi0[a] + (double)lo0[a];
+    v1[a] = (double)hi1[a] + (double)lo1[a];
+  }
+  finish_tile<Op, W>(op, p, tile, rank, S, v0, v1);
 }
 
 template <int SET, class Op>
