@@ -23,6 +23,7 @@
 // of all of space and S_B = inf: it is never skipped.
 #pragma once
 
+#include "griddesc.cuh"
 #include "kernels.cuh"
 #include "layout.h"
 #include "ops.cuh"
@@ -42,30 +43,49 @@ struct GaussStats {
   const float4 *wu;   // adjoint, per block: (sum |u|, max |u|, -, -)
   float4 *box_n;      // shooting: boxes of the next step's positions (written)
   float4 *wu_n;       // adjoint: weights of the next backward step's u (written; or null)
+  // contexts with a grid (grid.cuh): the next positions' box keys [pair][6], max |u| of the
+  // next backward step [pair] (or null)
+  unsigned *key_n, *umax_n;
 };
 
-// Union box of a row tile's blocks, its centre, and the sums of its blocks' weights.
+// Bounding box of a row tile, its centre and diagonal (each warp of a CTA holds all the
+// tile's rows, four per lane, and computes the same).
 struct GaussTile {
   float lo[3], hi[3], c[3];
   float diag2;       // squared diagonal of the box
   bool compact;
 };
 
-__device__ __forceinline__ GaussTile gauss_tile(const float4 *box, int b0, int nb) {
+__device__ __forceinline__ GaussTile gauss_tile(const float4 (&q)[4], const bool (&live)[4]) {
   GaussTile t;
+  bool fin = true;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     t.lo[d] = INFINITY;
     t.hi[d] = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float x = d == 0 ? q[r].x : d == 1 ? q[r].y : q[r].z;
+      fin &= !live[r] || isfinite(x);
+      if (live[r]) {
+        t.lo[d] = fminf(t.lo[d], x);
+        t.hi[d] = fmaxf(t.hi[d], x);
+      }
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      t.lo[d] = fminf(t.lo[d], __shfl_xor_sync(0xffffffffu, t.lo[d], off));
+      t.hi[d] = fmaxf(t.hi[d], __shfl_xor_sync(0xffffffffu, t.hi[d], off));
+    }
   }
-  for (int b = b0; b < b0 + nb; ++b) {
-    const float4 l = __ldcg(&box[2 * b]), h = __ldcg(&box[2 * b + 1]);
-    t.lo[0] = fminf(t.lo[0], l.x); t.lo[1] = fminf(t.lo[1], l.y); t.lo[2] = fminf(t.lo[2], l.z);
-    t.hi[0] = fmaxf(t.hi[0], h.x); t.hi[1] = fmaxf(t.hi[1], h.y); t.hi[2] = fmaxf(t.hi[2], h.z);
-  }
+  fin = __all_sync(0xffffffffu, fin);
   t.diag2 = 0.0f;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
+    if (!fin) {
+      t.lo[d] = -INFINITY;
+      t.hi[d] = INFINITY;
+    }
     const float e = t.hi[d] - t.lo[d];
     t.diag2 = fmaf(e, e, t.diag2);
     t.c[d] = 0.5f * (t.lo[d] + t.hi[d]);
@@ -85,9 +105,10 @@ __device__ __forceinline__ float gauss_gap2(const GaussTile &t, const float4 &lo
 
 // ------------------------------------------------------------------- statistics
 
-// Box and weight of one 32-point block, one point per lane (live: not padding).
+// Box of one 32-point block, one point per lane (live: not padding), and its part in the
+// pair's box (keys).  blk < 0: not a block of the storage order, keys only.
 __device__ __forceinline__ void gauss_block_box(float4 *box, int blk, bool live, float x,
-                                                float y, float z) {
+                                                float y, float z, unsigned *keys) {
   const bool fin = isfinite(x) && isfinite(y) && isfinite(z);
   const float v[3] = {x, y, z};
   float lo[3], hi[3];
@@ -102,8 +123,16 @@ __device__ __forceinline__ void gauss_block_box(float4 *box, int blk, bool live,
     }
   }
   if ((threadIdx.x & 31) == 0) {
-    box[2 * blk] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-    box[2 * blk + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+    if (blk >= 0) {
+      box[2 * blk] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+      box[2 * blk + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+    }
+    if (keys)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        atomicMin(&keys[d], float_key(lo[d]));
+        atomicMin(&keys[3 + d], float_key(-hi[d]));
+      }
   }
 }
 
@@ -126,8 +155,10 @@ __device__ __forceinline__ float abs_max(const float4 &a) {
 // A NaN or infinity anywhere in the block gives S = inf (fmaxf drops NaNs, sums keep them).
 __device__ __forceinline__ float or_inf(float s) { return s < INFINITY ? s : INFINITY; }
 
-// Weights of alpha at every time step (or of u): one warp per (step, block); grid-stride.
-__global__ void gauss_alpha_kernel(const float4 *as, long long nblk_tot, float4 *wa) {
+// Weights of alpha at every time step (or of u): one warp per (step, block), nblk blocks
+// per step; mx (or null): max |a| per (step, pair).
+__global__ void gauss_alpha_kernel(const float4 *as, long long nblk_tot, int nblk, float4 *wa,
+                                   const int *pt_pair, unsigned *mx, int P) {
   pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31;
@@ -135,37 +166,50 @@ __global__ void gauss_alpha_kernel(const float4 *as, long long nblk_tot, float4 
   for (long long b = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
        b < nblk_tot; b += nw) {
     const float4 a = __ldcg(&as[b * 32 + lane]);
-    const float s = warp_sum_f(abs_sum(a)), m = warp_max_f(abs_max(a));
-    if (lane == 0) wa[b] = make_float4(or_inf(s), m, 0.0f, 0.0f);
+    const float s = or_inf(warp_sum_f(abs_sum(a))), m = warp_max_f(abs_max(a));
+    if (lane == 0) {
+      wa[b] = make_float4(s, m, 0.0f, 0.0f);
+      const int t = (int)(b / nblk), p = pt_pair[(b - (long long)t * nblk) * 32];
+      if (mx && p >= 0) atomicMax(&mx[t * P + p], __float_as_uint(s < INFINITY ? m : s));
+    }
   }
 }
 
 // Boxes of the initial positions: one warp per block.
-__global__ void gauss_box_kernel(const float4 *qs, const int *pt_pair, int nblk, float4 *box) {
+__global__ void gauss_box_kernel(const float4 *qs, const int *pt_pair, int nblk, float4 *box,
+                                 unsigned *keys) {
   pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (b >= nblk) return;
   const float4 q = __ldcg(&qs[(size_t)b * 32 + lane]);
-  gauss_block_box(box, b, pt_pair[(size_t)b * 32 + lane] >= 0, q.x, q.y, q.z);
+  const int p = pt_pair[(size_t)b * 32 + lane], p0 = __shfl_sync(0xffffffffu, p, 0);
+  gauss_block_box(box, b, p >= 0, q.x, q.y, q.z, keys && p0 >= 0 ? keys + 6 * p0 : nullptr);
 }
 
-// Statistics of the block a warp has just finalised (one row per lane, whose new values
-// the lane itself wrote): the boxes of the next positions, the weights of the next u.
+// Statistics of the rows a warp has just finalised (one per lane, whose new values the
+// lane itself wrote): the boxes of the next positions, the weights of the next u; of
+// storage block blk (-1: rows of another order, only the pair's keys and maxima).  g: the
+// row's point, any valid one when not live.
 template <int D, int ORDER>
 __device__ __forceinline__ void gauss_next_stats(const ShootOp<D, ORDER> &op,
-                                                 const GaussStats &gs, int blk, int g, bool live) {
+                                                 const GaussStats &gs, int p, int blk, int g,
+                                                 bool live) {
   const float4 q = op.qs_n[g];
-  gauss_block_box(gs.box_n, blk, live, q.x, q.y, q.z);
+  gauss_block_box(gs.box_n, blk, live, q.x, q.y, q.z, gs.key_n ? gs.key_n + 6 * p : nullptr);
 }
 template <int D, int ORDER>
 __device__ __forceinline__ void gauss_next_stats(const AdjointOp<D, ORDER> &op,
-                                                 const GaussStats &gs, int blk, int g, bool) {
+                                                 const GaussStats &gs, int p, int blk, int g,
+                                                 bool live) {
   if (!op.us_n) return;
-  const float4 u = op.us_n[g];
-  const float s = warp_sum_f(abs_sum(u)), m = warp_max_f(abs_max(u));
-  if ((threadIdx.x & 31) == 0) gs.wu_n[blk] = make_float4(or_inf(s), m, 0.0f, 0.0f);
+  const float4 u = live ? op.us_n[g] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float s = or_inf(warp_sum_f(abs_sum(u))), m = warp_max_f(abs_max(u));
+  if ((threadIdx.x & 31) == 0) {
+    if (blk >= 0) gs.wu_n[blk] = make_float4(s, m, 0.0f, 0.0f);
+    if (gs.umax_n) atomicMax(&gs.umax_n[p], __float_as_uint(s < INFINITY ? m : s));
+  }
 }
 
 // ------------------------------------------------------------------- split items
@@ -178,6 +222,8 @@ __device__ __forceinline__ void gauss_next_stats(const AdjointOp<D, ORDER> &op,
 
 struct SplitPlan {
   int S;               // CTAs per item
+  int items;           // work items: items * S units, walked by the grid
+  bool one;            // all of one pair
   double *part;        // [item * S + rank][row of the item][NA]
   unsigned int *cnt;   // per item: arrivals (left at zero)
 };
@@ -241,7 +287,7 @@ __device__ __forceinline__ void finish_split(const Op &op, int p, int tile, int 
   if (mine) e = op.finalize(p, row, t);
   if (mine) {  // whole warps: the statistics of this warp's block for the next step
     const PairDesc &P = op.pd[p];
-    gauss_next_stats(op, gs, (P.pt_off + row) / kSub, P.pt_off + row, row < P.N);
+    gauss_next_stats(op, gs, p, (P.pt_off + row) / kSub, P.pt_off + row, row < P.N);
   }
   if (Op::kTileSum) {
     for (int h = 0; h < (two ? 2 : 1); ++h) {
@@ -262,24 +308,43 @@ __device__ __forceinline__ void finish_split(const Op &op, int p, int tile, int 
 template <int W>
 __global__ void __launch_bounds__(W * 32)
     gauss_shoot_kernel(const ShootOp<3, -1> op, const GaussStats gs,
-                       const int2 *__restrict__ items, const SplitPlan sp) {
+                       const int2 *__restrict__ items, const SplitPlan sp, const GridArgs ga) {
   constexpr int NA = 3;
-  const int S = sp.S;
   __shared__ __align__(16) float s_j[W][7][kSub];
-  const int item = blockIdx.x / S;
-  const int rank = blockIdx.x - item * S;
-  const int2 it = items[item];
   pdl_wait();
   pdl_trigger();
+  int skip = -1;  // pair found to have nothing to do here
+  for (int unit = blockIdx.x; unit < sp.items * sp.S; unit += gridDim.x) {
+  const int S = sp.S;
+  const int item = unit / S;
+  const int rank = unit - item * S;
+  const int2 it = items[item];
   const int p = it.x, tile = it.y;
-  if (!op.active(p)) return;  // identical for every CTA of the cluster
+  if (p == skip) continue;
+  GridDesc gd;
+  if (!op.active(p) || grid_active(ga, p, false, gd)) {
+    if (sp.one) return;
+    skip = p;
+    continue;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const PairDesc &P = op.pd[p];
   const int pt = P.pt_off, npad = P.Npad;
   const int row0 = tile * kTile;
   const bool two = row0 + kTile < npad;  // uniform over the cluster
   const int blk0 = pt / kSub, nblk = npad / kSub;
-  const GaussTile T = gauss_tile(gs.box + 2 * blk0, row0 / kSub, two ? 4 : 2);
+  // pairs with a grid come here when it cannot hold the step; their blocks have no
+  // statistics and every block is evaluated
+  const bool cull = !ga.slot || ga.slot[p] < 0;
+  float4 q[4];
+  bool live[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int row = (r < 2 || two) ? row0 + 32 * r + lane : row0 + lane;
+    live[r] = row < P.N;
+    q[r] = __ldcg(&op.qs_t[pt + row]);
+  }
+  const GaussTile T = gauss_tile(q, live);
   float S_I = 0.0f;
   for (int b = 0; b < (two ? 4 : 2); ++b) S_I += __ldcg(&gs.wa[blk0 + row0 / kSub + b].x);
   const float thr = T.diag2 - lg2f_approx(S_I) + kCullBits + lg2f_approx((float)nblk);
@@ -287,9 +352,7 @@ __global__ void __launch_bounds__(W * 32)
   double b2[4];     // |x'|^2
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    const int row = (r < 2 || two) ? row0 + 32 * r + lane : row0 + lane;
-    const float4 q = __ldcg(&op.qs_t[pt + row]);
-    const float x = q.x - T.c[0], y = q.y - T.c[1], z = q.z - T.c[2];
+    const float x = q[r].x - T.c[0], y = q[r].y - T.c[1], z = q[r].z - T.c[2];
     b2[r] = (double)x * x + (double)y * y + (double)z * z;
     const float f = T.compact ? 2.0f : 1.0f;
     q2[r][0] = make_float2(f * x, f * x);
@@ -310,8 +373,8 @@ __global__ void __launch_bounds__(W * 32)
       base += 32 * nw;
       if (base >= nblk) return nblk;
       const int sb = base + lane * nw;
-      bool keep = false;
-      if (sb < nblk) {
+      bool keep = sb < nblk;
+      if (keep && cull) {
         const float4 l = __ldcg(&gs.box[2 * (blk0 + sb)]), h = __ldcg(&gs.box[2 * (blk0 + sb) + 1]);
         const float w = __ldcg(&gs.wa[blk0 + sb].x);
         keep = !(gauss_gap2(T, l, h) >= lg2f_approx(w) + thr);
@@ -374,7 +437,7 @@ __global__ void __launch_bounds__(W * 32)
         }
       }
     } else {
-#pragma unroll 1
+#pragma unroll 2
       for (int jj = 0; jj < kSub; jj += 2) {
         float2 w[7];
 #pragma unroll
@@ -405,7 +468,9 @@ __global__ void __launch_bounds__(W * 32)
 #pragma unroll
     for (int a = 0; a < NA; ++a) v[r][a] = f * ((double)hi[r][a] + (double)lo[r][a]);
   }
+  __syncthreads();  // the previous unit's reduction is done with the shared arrays
   finish_split<ShootOp<3, -1>, W, 4>(op, p, tile, item, rank, sp, two, gs, v);
+  }
 }
 
 // --------------------------------------------------------------------- adjoint
@@ -419,20 +484,28 @@ __global__ void __launch_bounds__(W * 32)
 template <int W>
 __global__ void __launch_bounds__(W * 32)
     gauss_adjoint_kernel(const AdjointOp<3, -1> op, const GaussStats gs,
-                         const int2 *__restrict__ items, const SplitPlan sp) {
+                         const int2 *__restrict__ items, const SplitPlan sp, const GridArgs ga) {
   using Op = AdjointOp<3, -1>;
   constexpr int R = 4;    // rows per lane
   constexpr int NS = 7;   // sums per row: K u (3), s x' (3), s
   constexpr int NJ = 10;  // staged values per column: x', -|x'|^2, u, r
   __shared__ __align__(16) float s_j[W][NJ][kSub];
-  const int S = sp.S;
-  const int item = blockIdx.x / S;
-  const int rank = blockIdx.x - item * S;
-  const int2 it = items[item];
   pdl_wait();
   pdl_trigger();
+  int skip = -1;  // as in the shooting sweep
+  for (int unit = blockIdx.x; unit < sp.items * sp.S; unit += gridDim.x) {
+  const int S = sp.S;
+  const int item = unit / S;
+  const int rank = unit - item * S;
+  const int2 it = items[item];
   const int p = it.x, tile = it.y;
-  if (!op.active(p)) return;
+  if (p == skip) continue;
+  GridDesc gd;
+  if (!op.active(p) || grid_active(ga, p, true, gd)) {
+    if (sp.one) return;
+    skip = p;
+    continue;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const PairDesc &P = op.pd[p];
   const int pt = P.pt_off, npad = P.Npad;
@@ -440,7 +513,16 @@ __global__ void __launch_bounds__(W * 32)
   const bool two = row0 + kTile < npad;
   const int nbt = two ? 4 : 2;
   const int blk0 = pt / kSub, nblk = npad / kSub;
-  const GaussTile T = gauss_tile(gs.box + 2 * blk0, row0 / kSub, nbt);
+  const bool cull = !ga.slot || ga.slot[p] < 0;  // as in the shooting sweep
+  float4 q[R];
+  bool live[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int row = (r < 2 || two) ? row0 + 32 * r + lane : row0 + lane;
+    live[r] = row < P.N;
+    q[r] = __ldcg(&op.qs_t[pt + row]);
+  }
+  const GaussTile T = gauss_tile(q, live);
   // cut-offs: of K u against the tile's sum of |u|, and of s |x_i - x_j| against the same
   // products of the tile's own points a quarter of its diagonal apart
   float U_I = 0.0f, R_I = 0.0f, rm = 0.0f, um = 0.0f;
@@ -461,8 +543,8 @@ __global__ void __launch_bounds__(W * 32)
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int row = pt + ((r < 2 || two) ? row0 + 32 * r + lane : row0 + lane);
-    const float4 q = __ldcg(&op.qs_t[row]), u = __ldcg(&op.us_t[row]), a = __ldcg(&op.as_t[row]);
-    const float x[3] = {qf * (q.x - T.c[0]), qf * (q.y - T.c[1]), qf * (q.z - T.c[2])};
+    const float4 u = __ldcg(&op.us_t[row]), a = __ldcg(&op.as_t[row]);
+    const float x[3] = {qf * (q[r].x - T.c[0]), qf * (q[r].y - T.c[1]), qf * (q[r].z - T.c[2])};
     const float m[3] = {u.x - a.x, u.y - a.y, u.z - a.z}, rr[3] = {a.x, a.y, a.z};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -484,8 +566,8 @@ __global__ void __launch_bounds__(W * 32)
       base += 32 * nw;
       if (base >= nblk) return nblk;
       const int sb = base + lane * nw;
-      bool keep = false;
-      if (sb < nblk) {
+      bool keep = sb < nblk;
+      if (keep && cull) {
         const int b = blk0 + sb;
         const float4 l = __ldcg(&gs.box[2 * b]), h = __ldcg(&gs.box[2 * b + 1]);
         const float4 w = __ldcg(&gs.wu[b]), a = __ldcg(&gs.wa[b]);
@@ -561,7 +643,7 @@ __global__ void __launch_bounds__(W * 32)
         }
       }
     } else {
-#pragma unroll 1
+#pragma unroll 2
       for (int jj = 0; jj < kSub; jj += 2) {
         float2 w[NJ];
 #pragma unroll
@@ -600,7 +682,9 @@ __global__ void __launch_bounds__(W * 32)
       v[r][3 + d] = f * (x[d] * ss - ((double)hi[r][3 + d] + (double)lo[r][3 + d]));
     }
   }
+  __syncthreads();
   finish_split<Op, W, R>(op, p, tile, item, rank, sp, two, gs, v);
+  }
 }
 
 }  // namespace lddmm

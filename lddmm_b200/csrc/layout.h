@@ -41,6 +41,7 @@ struct PairDesc {
   double pd_fac;      // dq factor: pdot = pd_fac * sum(lr * W * dq_scaled)
   double dc_fac;      // varifold dc factor (without the 2 a_i): -2 / (sigma_W^2 * cscale)
   double tt;          // target self-term, FP64, computed once
+  double kscale64;    // coordinate scale of the Gaussian deformation kernel in FP64 (grid.cuh)
 };
 
 // L-BFGS + line-search state of one pair (FP64 scalars), after Cpp/src/LBFGS.cpp

@@ -1,6 +1,7 @@
 // Host runtime of the B200 LDDMM library: batch layout, device memory, kernel
 // dispatch, the objective sweep, the device L-BFGS cycle (CUDA graph) and the C ABI.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <memory>
 #include <map>
@@ -16,6 +17,7 @@
 #include "common.cuh"
 #include "cross.cuh"
 #include "gauss.cuh"
+#include "grid.cuh"
 #include "kernels.cuh"
 #include "layout.h"
 #include "lbfgs.cuh"
@@ -178,6 +180,17 @@ struct lddmm_ctx {
   float4 *gbox = nullptr, *gwa = nullptr, *gwu = nullptr;
   double *gpart = nullptr;
   unsigned int *gcnt = nullptr;
+  // gridded kernel sums of large pairs (grid.cuh)
+  bool grid = false;
+  int n_grid = 0, grid_dmax = 0;        // pairs with a grid, largest extent per axis
+  int n_gblk = 0, n_gtile[2] = {0, 0};  // 32-point blocks; spread tiles of 32 / 128 points
+  int2 *gblk = nullptr, *gtile[2] = {nullptr, nullptr};
+  int *gpairs = nullptr, *gslot = nullptr, *gord = nullptr;
+  long long *goff = nullptr, *gcap = nullptr;
+  unsigned *gkeys = nullptr, *gmax = nullptr;  // box keys [T + 1][P][6]; max |a|, |u| [2][T][P]
+  unsigned long long *graw = nullptr;
+  double *gfld = nullptr;
+  GridTables *gtab = nullptr;
   float4 *dbb = nullptr, *tbb = nullptr;  // 32-element block boxes (varifold culling)
   float4 *ec = nullptr, *en = nullptr, *el = nullptr, *tc = nullptr, *tn = nullptr,
          *tl = nullptr;
@@ -260,6 +273,9 @@ lddmm_ctx::~lddmm_ctx() {
   dfree(dbb, stream); dfree(tbb, stream);
   dfree(gbox, stream); dfree(gwa, stream); dfree(gwu, stream); dfree(gpart, stream);
   dfree(gcnt, stream);
+  dfree(gblk, stream); dfree(gtile[0], stream); dfree(gtile[1], stream); dfree(gpairs, stream);
+  dfree(gslot, stream); dfree(gord, stream); dfree(goff, stream); dfree(gcap, stream); dfree(gkeys, stream);
+  dfree(gmax, stream); dfree(graw, stream); dfree(gfld, stream); dfree(gtab, stream);
   if (own_stream && stream) cudaStreamDestroy(stream);
 }
 
@@ -269,13 +285,13 @@ lddmm_ctx::~lddmm_ctx() {
 // programmatic stream serialisation (the kernel calls pdl_wait() before touching its
 // predecessor's output) and, for the sweeps, the thread-block cluster size.
 template <typename... KArgs, typename... Args>
-static cudaError_t launch(void (*kern)(KArgs...), unsigned grid, unsigned block, int cluster,
-                          cudaStream_t stream, Args &&...args) {
-  if (grid == 0) return cudaSuccess;
+static cudaError_t launch_smem(void (*kern)(KArgs...), dim3 grid, unsigned block, int cluster,
+                               size_t smem, cudaStream_t stream, Args &&...args) {
+  if (grid.x == 0) return cudaSuccess;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -291,6 +307,12 @@ static cudaError_t launch(void (*kern)(KArgs...), unsigned grid, unsigned block,
   cfg.attrs = attr;
   cfg.numAttrs = na;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch(void (*kern)(KArgs...), unsigned grid, unsigned block, int cluster,
+                          cudaStream_t stream, Args &&...args) {
+  return launch_smem(kern, dim3(grid), block, cluster, 0, stream, std::forward<Args>(args)...);
 }
 
 template <class Op>
@@ -309,15 +331,99 @@ static GaussStats gauss_stats(const lddmm_ctx &c, int t) {
   gs.wu = c.gwu + nb * (t & 1);
   gs.box_n = c.gbox + 2 * nb * (t + 1);
   gs.wu_n = t > 0 ? c.gwu + nb * ((t - 1) & 1) : nullptr;
+  gs.key_n = c.grid ? c.gkeys + (size_t)(t + 1) * c.P * 6 : nullptr;
+  gs.umax_n = c.grid && t > 0 ? c.gmax + (size_t)(c.T + t - 1) * c.P : nullptr;
   return gs;
+}
+
+// Grid arguments of step t (slot = null: no grid).
+static GridArgs grid_args(const lddmm_ctx &c, int t) {
+  GridArgs a;
+  std::memset(&a, 0, sizeof(a));
+  if (!c.grid) return a;
+  a.pd = c.pd;
+  a.act = c.act;
+  a.blocks = c.gblk;
+  a.ord = c.gord;
+  a.pairs = c.gpairs;
+  a.slot = c.gslot;
+  a.off = c.goff;
+  a.cap = c.gcap;
+  a.box = c.gkeys + (size_t)t * c.P * 6;
+  a.amax = c.gmax + (size_t)t * c.P;
+  a.umax = c.gmax + (size_t)(c.T + t) * c.P;
+  a.raw = c.graw;
+  a.fld = c.gfld;
+  a.tab = c.gtab;
+  a.dmax = c.grid_dmax;
+  return a;
+}
+
+// CTAs of the pair sweeps: one per unit, or, where every pair has a grid and the sweep
+// usually finds nothing to do, four per SM that walk the units.
+static unsigned gauss_ctas(const lddmm_ctx &c, int units) {
+  return (unsigned)(c.n_grid == c.P && c.grid ? std::min(units, 4 * 148) : units);
+}
+
+static size_t conv_smem(const lddmm_ctx &c) {
+  return sizeof(double) * (2 * kGridMaxDim + 2 + 2 * (size_t)c.grid_dmax * (c.grid_dmax + 1));
+}
+
+// Shared-memory limits of the grid kernels, raised once per device.
+static cudaError_t grid_attributes() {
+  static std::atomic<bool> set[kMaxDevices];
+  int dev = 0;
+  CUE(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < kMaxDevices && set[dev].load()) return cudaSuccess;
+  const int cs = (int)(sizeof(double) * (2 * kGridMaxDim + 2 + 2 * kGridMaxDim * (kGridMaxDim + 1)));
+  CUE(cudaFuncSetAttribute(grid_conv_yz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
+  CUE(cudaFuncSetAttribute(grid_conv_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
+  CUE(cudaFuncSetAttribute(grid_spread_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(GridSpreadSmem<128>)));
+  CUE(cudaFuncSetAttribute(grid_spread_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(GridSpreadSmem<32>)));
+  CUE(cudaFuncSetAttribute(grid_interp_kernel<false, ShootOp<3, -1>>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(GridInterpSmem<false>)));
+  CUE(cudaFuncSetAttribute(grid_interp_kernel<true, AdjointOp<3, -1>>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(GridInterpSmem<true>)));
+  if (dev >= 0 && dev < kMaxDevices) set[dev].store(true);
+  return cudaSuccess;
+}
+
+// Spread and convolve step t's sources: a (and u) -> fields of 3 (6) components.
+static cudaError_t grid_fields(lddmm_ctx &c, int t, const float4 *a, const float4 *u) {
+  const GridArgs A = grid_args(c, t);
+  const double *q = c.q64 + (size_t)t * c.NPtot * 3;
+  const int adj = u ? 1 : 0;
+  for (int k = 0; k < 2; ++k) {
+    if (!c.n_gtile[k]) continue;
+    GridArgs B = A;
+    B.blocks = c.gtile[k];
+    CUE(launch_smem(k ? grid_spread_kernel<128> : grid_spread_kernel<32>,
+                    dim3((unsigned)c.n_gtile[k]), kGridThreads, 0,
+                    k ? sizeof(GridSpreadSmem<128>) : sizeof(GridSpreadSmem<32>), c.stream, B, a, u,
+                    q, adj));
+  }
+  const dim3 gr((unsigned)c.grid_dmax, adj ? 6u : 3u, (unsigned)c.n_grid);
+  CUE(launch_smem(grid_conv_yz_kernel, gr, kConvThreads, 0, conv_smem(c), c.stream, A, adj));
+  return launch_smem(grid_conv_x_kernel, gr, kConvThreads, 0, conv_smem(c), c.stream, A, adj);
 }
 
 // Weights of alpha at every step, once per evaluation (of u: launch_gather).
 static cudaError_t gauss_begin(lddmm_ctx &c) {
   if (!c.gauss) return cudaSuccess;
-  const long long nb = (long long)c.T * c.NPtot / kSub;
+  const int nblk = c.NPtot / kSub;
+  const long long nb = (long long)c.T * nblk;
+  if (c.grid) {
+    const int nk = c.T * c.P * 6, nm = 2 * c.T * c.P;
+    CUE(launch(grid_reset_kernel, (unsigned)std::min((nk + nm + 255) / 256, 64), 256, 0, c.stream,
+               c.gkeys + c.P * 6, nk, c.gmax, nm));
+  }
   return launch(gauss_alpha_kernel, (unsigned)std::min<long long>((nb + 7) / 8, 2048), 256, 0,
-                c.stream, (const float4 *)c.as, nb, c.gwa);
+                c.stream, (const float4 *)c.as, nb, nblk, c.gwa, (const int *)c.pt_pair,
+                c.grid ? c.gmax : nullptr, c.P);
 }
 
 template <int D, int ORDER>
@@ -335,10 +441,22 @@ static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
   op.tile_part = c.reg_part + (size_t)t * c.ntile_tot;
   op.t = t;
   if constexpr (D == 3 && ORDER == -1) {
-    if (c.gauss)
-      return launch(gauss_shoot_kernel<kWarps>, (unsigned)(c.n_pt_items2 * c.S_shoot),
-                    kWarps * 32, 0, c.stream, op, gauss_stats(c, t), (const int2 *)c.pt_items2,
-                    SplitPlan{c.S_shoot, c.gpart, c.gcnt});
+    if (c.gauss) {
+      const GaussStats gs = gauss_stats(c, t);
+      if (c.grid) {
+        op.by_group = 1;
+        op.tile_part = c.reg_part + (size_t)t * c.ngrp_tot;
+      }
+      // pairs without a grid, and those whose grid cannot hold this step
+      CUE(launch(gauss_shoot_kernel<kWarps>, gauss_ctas(c, c.n_pt_items2 * c.S_shoot), kWarps * 32,
+                 0, c.stream, op, gs, (const int2 *)c.pt_items2,
+                 SplitPlan{c.S_shoot, c.n_pt_items2, c.P == 1, c.gpart, c.gcnt}, grid_args(c, t)));
+      if (!c.grid) return cudaSuccess;
+      CUE(grid_fields(c, t, op.as_t, nullptr));
+      return launch_smem(grid_interp_kernel<false, ShootOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
+                         InterpShape<false>::kWarps * 32, 0, sizeof(GridInterpSmem<false>), c.stream, op,
+                         grid_args(c, t), op.q64_t, gs);
+    }
   }
   // packed FP32x2 form of the same sweep (bitwise the same sums), on one- or two-tile
   // work items (c.tpw_shoot; the default rule and the autotuner pick it).  Two tiles
@@ -374,10 +492,17 @@ static cudaError_t adjoint_impl(lddmm_ctx &c, int t, double *g, double *pdot) {
   op.pdot64 = pdot;
   op.t = t;
   if constexpr (D == 3 && ORDER == -1) {
-    if (c.gauss)
-      return launch(gauss_adjoint_kernel<kWarps>, (unsigned)(c.n_pt_items2 * c.S_adj),
-                    kWarps * 32, 0, c.stream, op, gauss_stats(c, t), (const int2 *)c.pt_items2,
-                    SplitPlan{c.S_adj, c.gpart, c.gcnt});
+    if (c.gauss) {
+      const GaussStats gs = gauss_stats(c, t);
+      CUE(launch(gauss_adjoint_kernel<kWarps>, gauss_ctas(c, c.n_pt_items2 * c.S_adj), kWarps * 32,
+                 0, c.stream, op, gs, (const int2 *)c.pt_items2,
+                 SplitPlan{c.S_adj, c.n_pt_items2, c.P == 1, c.gpart, c.gcnt}, grid_args(c, t)));
+      if (!c.grid) return cudaSuccess;
+      CUE(grid_fields(c, t, op.as_t, op.us_t));
+      return launch_smem(grid_interp_kernel<true, AdjointOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
+                         InterpShape<true>::kWarps * 32, 0, sizeof(GridInterpSmem<true>), c.stream, op,
+                         grid_args(c, t), (const double *)(c.q64 + (size_t)t * c.NPtot * D), gs);
+    }
   }
   // packed FP32x2 form of the same sweep (bitwise the same sums), one- or two-tile
   // items as in shoot_impl (c.tpw_adj; Gaussian at 163,842 landmarks: 23.3 -> 22.0 ms
@@ -647,14 +772,16 @@ static cudaError_t launch_gather(lddmm_ctx &c, const double *q64T, float4 *un, f
     if (!c.gauss || !un) return cudaSuccess;
     const long long nblk = c.NPtot / kSub;  // weights of the first backward step's u
     return launch(gauss_alpha_kernel, (unsigned)((nblk + 3) / 4), 128, 0, c.stream,
-                  (const float4 *)un, nblk, c.gwu + nblk * ((c.T - 1) & 1));
+                  (const float4 *)un, nblk, (int)nblk, c.gwu + nblk * ((c.T - 1) & 1),
+                  (const int *)c.pt_pair,
+                  c.grid ? c.gmax + (size_t)(2 * c.T - 1) * c.P : nullptr, c.P);
   }
   return launch(gather_kernel<2>, nb, 128, 0, c.stream, c.pd, c.act, c.pt_pair, c.NPtot,
                 c.adj_ptr, c.adj, c.dcdd, q64T, c.XT, c.p64, un, ln, dq_out, c.T);
 }
 
 static cudaError_t launch_objective(lddmm_ctx &c, PairState *st, double *f_out) {
-  const int groups = c.persistent ? kGroup : 0;
+  const int groups = c.persistent || c.grid ? kGroup : 0;
   return launch(objective_kernel, (unsigned)c.P, 512, 0, c.stream, c.pd, c.act, c.reg_part,
                 groups ? c.ngrp_tot : c.ntile_tot, c.vfd_part, c.T, st, f_out, groups);
 }
@@ -854,6 +981,123 @@ static cudaError_t run_eval(lddmm_ctx &c, double *g_out, double *f_out, double *
 
 static int autotune(lddmm_ctx &c, const lddmm_config &cf);
 
+// Landmarks in k-d order: split at the median of the longest axis, at multiples of 128 and
+// then of 32 points, so that consecutive tiles of that size are compact whatever the order
+// of the mesh's vertices (a tile's grid work grows with its extent).
+static void kd_order(const double *x, int *idx, int lo, int hi);
+
+// Chooses the pairs whose Gaussian kernel sums run on a grid and allocates the grids.
+//
+// Cost per time step (shooting and adjoint), in SM clocks, measured: 0.32 N^2 for the pair
+// sweeps (40,962 landmarks: 1.92 ms); on the grid 5,000 per landmark and the convolutions,
+// 9 fields x 3 axes x about 53 taps per node at 64 per clock (20,011 landmarks: 0.35 ms
+// against 0.46).  The grid must win by a quarter: from about 20,000 landmarks on for a
+// unit shape at kernel width 0.3.  The grids of a context are bounded to 4 GB, largest
+// pairs first; each is 1.7 times the nodes of the initial box (extents up to 1.35 times).
+static void kd_order(const double *x, int *idx, int lo, int hi) {
+  while (hi - lo > 32) {
+    const int unit = hi - lo > 128 ? 128 : 32;
+    const int mid = lo + std::max(unit, ((hi - lo) / 2 + unit / 2) / unit * unit);
+    double l[3], h[3];
+    for (int d = 0; d < 3; ++d) l[d] = h[d] = x[(size_t)idx[lo] * 3 + d];
+    for (int k = lo + 1; k < hi; ++k)
+      for (int d = 0; d < 3; ++d) {
+        l[d] = std::min(l[d], x[(size_t)idx[k] * 3 + d]);
+        h[d] = std::max(h[d], x[(size_t)idx[k] * 3 + d]);
+      }
+    int ax = 0;
+    for (int d = 1; d < 3; ++d)
+      if (h[d] - l[d] > h[ax] - l[ax]) ax = d;
+    if (mid >= hi) return;
+    std::nth_element(idx + lo, idx + mid, idx + hi, [&](int a, int b) {
+      const double u = x[(size_t)a * 3 + ax], v = x[(size_t)b * 3 + ax];
+      return u < v || (u == v && a < b);
+    });
+    kd_order(x, idx, lo, mid);
+    lo = mid;
+  }
+}
+
+static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
+  constexpr long long kGridBytes = 4ll << 30;
+  std::vector<int> order(c.P), pairs, slot(c.P, -1);
+  for (int p = 0; p < c.P; ++p) order[p] = p;
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return c.hpd[a].N > c.hpd[b].N; });
+  std::vector<long long> off, cap;
+  long long total = 0;
+  for (int p : order) {
+    const PairDesc &P = c.hpd[p];
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    bool fin = true;
+    for (int i = 0; i < P.N; ++i)
+      for (int d = 0; d < 3; ++d) {
+        const double x = probs[p].ini_nde[(size_t)i * 3 + d] * P.kscale64;
+        fin &= std::isfinite(x);
+        lo[d] = std::min(lo[d], x);
+        hi[d] = std::max(hi[d], x);
+      }
+    double nodes = 1.0, nmax = 0.0;
+    for (int d = 0; d < 3; ++d) {
+      const double n = std::floor((hi[d] - lo[d]) / kGridH) + kWin + 2;
+      nodes *= n;
+      nmax = std::max(nmax, n);
+    }
+    if (!fin || !(nmax <= 0.9 * kGridMaxDim)) continue;
+    const double pair = 0.32 * P.N * (double)P.N;
+    const double grid = 5000.0 * P.N + 9.0 * 3.0 * std::min(nmax, 53.0) / 64.0 * nodes;
+    const long long cp = (long long)(1.7 * nodes);
+    if (pair < 1.25 * grid || (total + cp) * 6 * 16 > kGridBytes) continue;
+    slot[p] = (int)pairs.size();
+    pairs.push_back(p);
+    off.push_back(total);
+    cap.push_back(cp);
+    total += cp;
+    c.grid_dmax = std::max(c.grid_dmax, std::min(kGridMaxDim, (int)std::ceil(1.35 * nmax)));
+  }
+  c.n_grid = (int)pairs.size();
+  if (!c.n_grid) return 0;
+  std::vector<int2> blk, tile[2];
+  for (int p : pairs) {
+    const int nb = c.hpd[p].Npad / 32;
+    for (int k = 0; k < nb; ++k) blk.push_back(make_int2(p, k));
+    const int big = c.hpd[p].N >= 100000 ? 1 : 0;  // 128-point spread tiles
+    for (int k = 0; k < nb; k += big ? 4 : 1) tile[big].push_back(make_int2(p, k));
+  }
+  c.n_gblk = (int)blk.size();
+  std::vector<int> ord(c.NPtot, 0);
+  for (int p : pairs) {
+    int *o = &ord[c.hpd[p].pt_off];
+    for (int i = 0; i < c.hpd[p].N; ++i) o[i] = i;
+    kd_order(probs[p].ini_nde, o, 0, c.hpd[p].N);
+  }
+  auto put = [&](auto **d, const auto &h) -> cudaError_t {
+    CUE(dalloc(c.stream, d, h.size()));
+    return cudaMemcpyAsync(*d, h.data(), sizeof(h[0]) * h.size(), cudaMemcpyHostToDevice,
+                           c.stream);
+  };
+  CU(grid_attributes());
+  CU(put(&c.gblk, blk));
+  for (int k = 0; k < 2; ++k) {
+    c.n_gtile[k] = (int)tile[k].size();
+    CU(put(&c.gtile[k], tile[k]));
+  }
+  CU(put(&c.gpairs, pairs));
+  CU(put(&c.gslot, slot));
+  CU(put(&c.gord, ord));
+  CU(put(&c.goff, off));
+  CU(put(&c.gcap, cap));
+  CU(put(&c.gtab, std::vector<GridTables>(1, grid_tables())));
+  CU(dalloc(c.stream, &c.gkeys, (size_t)(c.T + 1) * c.P * 6));
+  CU(cudaMemsetAsync(c.gkeys, 0xff, sizeof(unsigned) * (size_t)(c.T + 1) * c.P * 6, c.stream));
+  CU(dalloc(c.stream, &c.gmax, (size_t)2 * c.T * c.P));
+  CU(dalloc(c.stream, &c.graw, (size_t)total * 6));
+  CU(dalloc(c.stream, &c.gfld, (size_t)total * 6));
+  CU(cudaStreamSynchronize(c.stream));  // the host arrays go out of scope
+  c.grid = true;
+  return 0;
+}
+
 extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm_config *cfg,
                                 lddmm_ctx **out) {
   if (!out || !probs || num <= 0) {
@@ -930,6 +1174,7 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     P.dt = a.time_stp;
     P.dis_wgt = a.dis_wgt;
     def_kernel_scales(a.knl_order, a.dim, a.knl_width, &P.kscale, &P.pd_fac);
+    P.kscale64 = a.knl_order == -1 ? std::sqrt(1.4426950408889634) / a.knl_width : P.kscale;
     if (c.has_vfd) cen_kernel_scales(a.cen_knl_type, a.cen_knl_width, &P.cscale, &P.dc_fac);
     pt += P.Npad;
     el += P.Edpad;
@@ -1365,15 +1610,17 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     CU(dalloc(c.stream, &c.gpart, (size_t)c.n_pt_items2 * std::max(c.S_shoot, c.S_adj) *
                                       kGaussRows * AdjointOp<3, -1>::NA));
     CU(dalloc(c.stream, &c.gcnt, c.n_pt_items2));
-    CU(launch(gauss_box_kernel, (unsigned)((nb + 3) / 4), 128, 0, c.stream, (const float4 *)c.qs,
-              (const int *)c.pt_pair, (int)nb, c.gbox));
     c.gauss = true;
+    const int rc = setup_grid(c, probs);
+    if (rc) return rc;
+    CU(launch(gauss_box_kernel, (unsigned)((nb + 3) / 4), 128, 0, c.stream, (const float4 *)c.qs,
+              (const int *)c.pt_pair, (int)nb, c.gbox, c.gkeys));
   }
   if (cf.autotune >= 0) {
     const int rc = autotune(c, cf);
     if (rc) return rc;
   }
-  if (c.persistent) c.gauss = false;
+  if (c.persistent) c.gauss = c.grid = false;
   *out = cp.release();
   return 0;
 }
@@ -2324,7 +2571,7 @@ extern "C" int lddmm_dq_kernel(int dim, int n, const double *q, const double *l,
   CU(cudaMemcpyAsync(c.ls, hl.data(), sizeof(float4) * c.NPtot, cudaMemcpyHostToDevice, c.stream));
   CU(cudaMemcpyAsync(c.as, hr.data(), sizeof(float4) * c.NPtot, cudaMemcpyHostToDevice, c.stream));
   CU(launch_set_active(c, 1));
-  c.gauss = false;  // l and r are not a step's operands (u = l + r / 2): the general sweep
+  c.gauss = c.grid = false;  // l and r are not a step's operands (u = l + r / 2): the general sweep
   CU(c.adjoint(c, 0, nullptr, pd));
   std::vector<double> h((size_t)c.NPtot * dim);
   CU(cudaMemcpyAsync(h.data(), pd, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c.stream));

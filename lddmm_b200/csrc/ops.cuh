@@ -37,6 +37,7 @@ struct ShootOp {
   const double *x64;   // FP64 alpha (trial point), variable layout
   double *vlc64;       // optional velocity output       [NPtot * D]
   double *tile_part;   // energy partial per i-tile of this step
+  int by_group = 0;    // tile_part in 16-row groups (contexts with a grid, grid.cuh)
   int t;
   // bases for the persistent multi-step sweep (set_step derives the fields above)
   const float4 *qs0, *as0;
@@ -179,6 +180,11 @@ struct ShootOp {
     return finalize(p, row, v, F);
   }
   __device__ void write_tile(int p, int tile, double v) const {
+    if (by_group) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) write_group(p, 4 * tile + k, k ? 0.0 : v);
+      return;
+    }
     tile_part[pd[p].itile_off + tile] = v;
   }
   __device__ void write_group(int p, int grp, double v) const {

@@ -49,3 +49,57 @@ def test_gauss_sweeps_keep_nan():
     with api.Context(P, persistent=-1) as ctx:
         f, g = ctx.objgrd(a)
     assert np.isnan(f[0]) and np.isnan(g).any()
+
+
+def _grid_problem(n, width, seed):
+    P = _problem(n, width, seed)
+    P.cen_width = 0.1
+    return P
+
+
+@pytest.mark.parametrize("n", [40000, 40962])
+def test_gridded_sums_against_fp64(n):
+    """A pair large enough for the gridded kernel sums (csrc/grid.cuh), 40,000 landmarks
+    leaving a partial 32-point tile's worth of padding and 40,962 an odd tile count:
+    velocities and costate steps of a row sample against FP64 pair sums.  The grid's kernel
+    is within 3.4e-11 of the Gaussian and 2.5e-9 of its derivative, far below the FP32
+    rounding of the pair sweeps, so 1e-7 of the largest value bounds what the FP32 momenta
+    leave."""
+    import ctypes as C
+
+    import torch
+
+    from lddmm_b200 import _lib, api
+
+    P = _grid_problem(n, 0.3, 5)
+    rng = np.random.default_rng(n)
+    a = rng.normal(size=(P.T, n, 3)) * 0.001 + 0.0005 * P.ini_nde
+    with api.Context(P) as ctx:
+        (q, v), = ctx.shoot(a.reshape(-1))
+        d = torch.from_numpy(a.reshape(-1)).cuda()
+        f, g, pst = torch.empty(1, dtype=torch.float64, device="cuda"), d.clone(), d.clone()
+        args = [C.c_void_p(x.data_ptr()) for x in (d, f, g, pst)]
+        _lib.check(_lib.lib.lddmm_objgrd_costate(ctx.handle, *args))
+        f2, g2 = ctx.objgrd(a.reshape(-1))
+        g, pst = (x.cpu().numpy().reshape(a.shape) for x in (g, pst))
+        assert f2[0] == f.item() and np.array_equal(g2.reshape(a.shape), g)
+        big, _ = ctx.objgrd(a.reshape(-1) * 4000)  # outgrows its grid: the pair sweeps
+        assert np.isfinite(big[0])
+        a[1, 3, 0] = np.inf
+        assert not np.isfinite(ctx.objgrd(a.reshape(-1))[0][0])
+    rows = rng.integers(0, n, 40)
+    w2 = P.knl_width ** 2
+    a[1, 3, 0] = 0.0
+    for t in range(P.T):
+        d = q[t][rows][:, None] - q[t][None]
+        K = np.exp(-(d ** 2).sum(-1) / w2)
+        if t != 1:  # row 3's momentum was replaced at step 1
+            assert np.max(np.abs(K @ a[t] - v[t][rows])) < 1e-7 * np.max(np.abs(v[t]))
+            u = a[t] - pst[t]
+            assert np.max(np.abs(P.time_stp * K @ u - g[t][rows])) < 1e-7 * np.max(np.abs(g[t]))
+        if t == 2:
+            l = 0.5 * a[t] - pst[t]
+            lr = l[rows] @ a[t].T + a[t][rows] @ l.T
+            dq = -2 / w2 * ((K * lr)[..., None] * d).sum(1)
+            step = pst[t][rows] - pst[t - 1][rows]
+            assert np.max(np.abs(P.time_stp * dq - step)) < 1e-7 * np.max(np.abs(pst[t]))
