@@ -38,6 +38,7 @@ constexpr int kGridMaxDim = 112;  // nodes per axis: a plane of doubles fits sha
 constexpr int kGridKZ = 16;       // z nodes handled at once in registers
 constexpr int kGridThreads = 128;
 constexpr int kConvThreads = 256;
+constexpr int kInterpWarps = 4;
 
 // Window values (and derivatives) on one axis of point pt (of npts) at scaled coordinate
 // x: val[node * npts + pt], and the window's first node relative to the grid, kept inside
@@ -75,22 +76,30 @@ __global__ void grid_reset_kernel(unsigned *keys, int nkeys, unsigned *mx, int n
     else mx[i - nkeys] = 0u;
 }
 
+// FP64 tensor-core product of 8 x 4 and 4 x 8: a = A[lane / 4][lane % 4], b = B[lane % 4]
+// [lane / 4], d = D[lane / 4][2 (lane % 4) + 0, 1].
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+  asm volatile(
+      "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
 // ------------------------------------------------------------------------ spread
 //
 // A CTA takes a tile of 32 or 128 points that are close in space (k-d order of the initial
-// positions): thread = a line of
-// nodes along z of the tile's bounding grid, which it sums over the points in registers,
-// so that a node receives one atomic per tile instead of one per point.  Bound by FP64
-// FMA issue (3 per node and point).
+// positions).  For a plane m of x nodes and 8 rows n of y nodes,
+//   S_c(n, k) = sum_p [psi_m psi_n a_c](p) psi_k(p)
+// is an (8 x points) x (points x 16 z nodes) product for each of the 3 momenta
+// components, on the FP64 tensor cores: the left operand is formed in registers, the
+// right one holds the points' z windows.  A node receives one atomic per tile.
 
 template <int TPTS>
 struct GridSpreadSmem {
   double w[2][kWin][TPTS];        // x and y windows
-  double zw[TPTS][kGridKZ];       // z windows over the current nodes, zero outside
   double z[kWin][TPTS];
+  double zw[TPTS][kGridKZ + 4];   // z windows over the current nodes, zero outside
   float a[6][TPTS];
-  unsigned long long st[kGridThreads][kGridKZ + 1];  // sums of a pass, for atomics along z
-  int ln[kGridThreads];           // first node of the pass's lines
   int o[3][TPTS];
   int lo[3], hi[3];
 };
@@ -104,7 +113,7 @@ __global__ void __launch_bounds__(kGridThreads)
   const int2 it = A.blocks[blockIdx.x];
   pdl_wait();
   pdl_trigger();
-  const int p = it.x, tid = threadIdx.x;
+  const int p = it.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (!A.act[p]) return;
   GridDesc g;
   if (!grid_active(A, p, adj != 0, g)) return;
@@ -112,7 +121,6 @@ __global__ void __launch_bounds__(kGridThreads)
   const int row0 = it.y * 32;
   const int npt = min(TPTS, P.N - row0);
   if (npt <= 0) return;
-  const int slot = A.slot[p];
   if (tid < 3) {
     sm.lo[tid] = 1 << 20;
     sm.hi[tid] = -1;
@@ -131,7 +139,7 @@ __global__ void __launch_bounds__(kGridThreads)
   __syncthreads();
   for (int i = tid; i < 3 * TPTS; i += kGridThreads) {
     const int axis = i / TPTS, pt = i - axis * TPTS;
-    const int src = min(pt, npt - 1);
+    const int src = min(pt, npt - 1);  // padding repeats the last point, with a = 0
     const double x = __ldcg(&q64[(size_t)(P.pt_off + ord[src]) * 3 + axis]) * P.kscale64;
     grid_windows<false>(A.tab, x, pt, TPTS, g.f[axis], g.n[axis],
                         axis == 2 ? &sm.z[0][0] : &sm.w[axis][0][0], nullptr, sm.o[axis]);
@@ -140,63 +148,48 @@ __global__ void __launch_bounds__(kGridThreads)
     atomicMax(&sm.hi[axis], o + kWin);
   }
   __syncthreads();
-  const int lx = sm.lo[0], ly = sm.lo[1], lz = sm.lo[2];
-  const int nx = sm.hi[0] - lx, ny = sm.hi[1] - ly, nlines = nx * ny;
-  unsigned long long *raw = A.raw + A.off[slot] * 6;
-  for (int z0 = lz; z0 < sm.hi[2]; z0 += kGridKZ) {
+  unsigned long long *raw = A.raw + A.off[A.slot[p]] * 6;
+  const int hx = sm.hi[0], hy = sm.hi[1], hz = sm.hi[2];
+  const int kr = lane & 3, kq = lane >> 2;
+  const int npt4 = (npt + 3) & ~3;
+  const double sca = scalbn(1.0, grid_scale_exp(P.N, __ldcg(&A.amax[p])));
+  const double scu = s1 ? scalbn(1.0, grid_scale_exp(P.N, __ldcg(&A.umax[p]))) : 0.0;
+  for (int z0 = sm.lo[2]; z0 < hz; z0 += kGridKZ) {
     for (int i = tid; i < TPTS * kGridKZ; i += kGridThreads) {
       const int pt = i / kGridKZ, k = i - pt * kGridKZ;
       const int q = z0 + k - sm.o[2][pt];
-      sm.zw[pt][k] = (q >= 0 && q < kWin && pt < npt) ? sm.z[q][pt] : 0.0;
+      sm.zw[pt][k] = (q >= 0 && q < kWin) ? sm.z[q][pt] : 0.0;
     }
     __syncthreads();
-    for (int c0 = 0; c0 < (s1 ? 6 : 3); c0 += 3) {
-      const int ex = grid_scale_exp(P.N, c0 ? __ldcg(&A.umax[p]) : __ldcg(&A.amax[p]));
-      const double sc = scalbn(1.0, ex);
-      for (int l0 = 0; l0 < nlines; l0 += kGridThreads) {
-        const int ln = l0 + tid;
-        const int m = lx + ln / ny, n = ly + ln % ny;
-        double acc[3][kGridKZ];
+    const int nchunk = (hy - sm.lo[1] + 7) / 8;
+    for (int u = warp; u < (hx - sm.lo[0]) * nchunk; u += kGridThreads / 32) {
+      const int m = sm.lo[0] + u / nchunk, n0 = sm.lo[1] + (u % nchunk) * 8, n = n0 + kq;
+      for (int c0 = 0; c0 < (s1 ? 6 : 3); c0 += 3) {
+        double d[3][4] = {};
+        for (int pt = kr; pt < npt4; pt += 4) {
+          const unsigned i = m - sm.o[0][pt], j = n - sm.o[1][pt];
+          if (!__any_sync(0xffffffffu, i < kWin && j < kWin)) continue;
+          const double w = i < kWin && j < kWin ? sm.w[0][i][pt] * sm.w[1][j][pt] : 0.0;
+          const double b0 = sm.zw[pt][kq], b1 = sm.zw[pt][8 + kq];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int k = 0; k < kGridKZ; ++k) acc[c][k] = 0.0;
-        if (ln < nlines) {
-#pragma unroll 1
-          for (int pt = 0; pt < npt; ++pt) {
-            const unsigned i = m - sm.o[0][pt], j = n - sm.o[1][pt];
-            if (i >= kWin || j >= kWin) continue;
-            const double w = sm.w[0][i][pt] * sm.w[1][j][pt];
-            const double w0 = w * sm.a[c0][pt], w1 = w * sm.a[c0 + 1][pt],
-                         w2 = w * sm.a[c0 + 2][pt];
-#pragma unroll
-            for (int k = 0; k < kGridKZ; k += 2) {
-              const double2 z = *reinterpret_cast<const double2 *>(&sm.zw[pt][k]);
-              acc[0][k] = fma(w0, z.x, acc[0][k]);
-              acc[1][k] = fma(w1, z.x, acc[1][k]);
-              acc[2][k] = fma(w2, z.x, acc[2][k]);
-              acc[0][k + 1] = fma(w0, z.y, acc[0][k + 1]);
-              acc[1][k + 1] = fma(w1, z.y, acc[1][k + 1]);
-              acc[2][k + 1] = fma(w2, z.y, acc[2][k + 1]);
-            }
+          for (int c = 0; c < 3; ++c) {
+            const double x = w * sm.a[c0 + c][pt];
+            dmma(d[c][0], d[c][1], x, b0);
+            dmma(d[c][2], d[c][3], x, b1);
           }
         }
-        // neighbouring threads add neighbouring z nodes
-        const int nl = min(kGridThreads, nlines - l0), nk = min(kGridKZ, sm.hi[2] - z0);
+        const double sc = c0 ? scu : sca;
+        if (n < hy) {
+          unsigned long long *dst =
+              raw + c0 * g.nodes + ((size_t)m * g.n[1] + n) * g.n[2] + z0;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          __syncthreads();  // the previous pass's or component's atomics have read st and ln
-          if (c == 0) sm.ln[tid] = (m * g.n[1] + n) * g.n[2];
+          for (int c = 0; c < 3; ++c)
 #pragma unroll
-          for (int k = 0; k < kGridKZ; ++k)
-            sm.st[tid][k] = (unsigned long long)__double2ll_rn(acc[c][k] * sc);
-          __syncthreads();
-          unsigned long long *dst = raw + (c0 + c) * g.nodes + z0;
-          for (int i = tid; i < nl * kGridKZ; i += kGridThreads) {
-            const int l = i / kGridKZ, k = i - l * kGridKZ;
-            const unsigned long long v = sm.st[l][k];
-            if (k < nk && v) atomicAdd(dst + sm.ln[l] + k, v);
-          }
+            for (int k = 0; k < 4; ++k) {
+              const int z = (k >> 1) * 8 + kr * 2 + (k & 1);
+              const long long v = __double2ll_rn(d[c][k] * sc);
+              if (z0 + z < hz && v) atomicAdd(dst + (size_t)c * g.nodes + z, (unsigned long long)v);
+            }
         }
       }
     }
@@ -324,33 +317,30 @@ __global__ void __launch_bounds__(kConvThreads) grid_conv_x_kernel(const GridArg
 
 // ------------------------------------------------------------------- interpolate
 //
-// CTA = one tile of 32 points, lane = point; the warps take the x planes of the
-// tile's bounding grid in turn.  A warp copies 8 or 16 rows x 16 z nodes of a plane to its
-// shared-memory buffer (all its loads in flight at once) and sums them against the lanes'
-// windows, the z windows in registers; the node values are read by all lanes at the same
-// address.  Then the rows are finalised as after a pair sweep.  Bound by FP64 FMA issue.
-
-template <bool ADJ>
-struct InterpShape {  // warps per tile, y rows per copy, CTAs per SM
-  static constexpr int kWarps = ADJ ? 4 : 8, kRows = ADJ ? 8 : 16, kCtas = ADJ ? 3 : 2;
-};
+// CTA = one tile of 32 points; the warps take the x planes of the tile's bounding grid in
+// turn.  A warp copies 8 y rows x 16 z nodes of a plane to its shared-memory buffer (all
+// its loads in flight at once); the sums over z are (8 points x 16 z nodes) x (16 x 8
+// rows) products on the FP64 tensor cores, the points' z windows in registers.  Each sum
+// is then weighted with the point's x and y windows.  Node values read through broadcast
+// loads into plain FMAs were held by the shared-memory pipe instead (twice the FMA time).
 
 template <bool ADJ>
 struct GridInterpSmem {
-  double2 f[InterpShape<ADJ>::kWarps][InterpShape<ADJ>::kRows][ADJ ? 6 : 3][kGridKZ / 2];  // reused for the sums
+  double f[kInterpWarps][ADJ ? 6 : 3][8][kGridKZ + 4];
   double w[3][kWin][32];
   double dw[ADJ ? 3 : 1][ADJ ? kWin : 1][32];
+  float cf[ADJ ? 6 : 1][32];   // m and r of the points
   int o[3][32];
+  double red[kInterpWarps][ADJ ? 6 : 3][32];
 };
 
 template <bool ADJ, class Op>
-__global__ void __launch_bounds__(InterpShape<ADJ>::kWarps * 32, InterpShape<ADJ>::kCtas)
+__global__ void __launch_bounds__(kInterpWarps * 32, ADJ ? 2 : 4)
     grid_interp_kernel(const Op op, const GridArgs A, const double *__restrict__ q64,
                        const GaussStats gs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GridInterpSmem<ADJ> &sm = *reinterpret_cast<GridInterpSmem<ADJ> *>(smem_raw);
   constexpr int NV = ADJ ? 6 : 3, NC = ADJ ? 6 : 3;
-  constexpr int kInterpWarps = InterpShape<ADJ>::kWarps, kInterpRows = InterpShape<ADJ>::kRows;
   const int2 it = A.blocks[blockIdx.x];
   pdl_wait();
   pdl_trigger();
@@ -363,9 +353,12 @@ __global__ void __launch_bounds__(InterpShape<ADJ>::kWarps * 32, InterpShape<ADJ
   // a partial tile's idle lanes repeat its last row (and are not finalised)
   const bool live = lane < npt;
   const int row = npt > 0 ? A.ord[P.pt_off + row0 + min(lane, npt - 1)] : 0;
-  double out[NV];
+  const int kr = lane & 3, kq = lane >> 2;
+  double out[4][NV];  // points 8 r + lane / 4, this lane's share of the y rows
 #pragma unroll
-  for (int k = 0; k < NV; ++k) out[k] = 0.0;
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[r][k] = 0.0;
   if (npt > 0) {
     if (tid < 96) {
       const int axis = tid >> 5;
@@ -373,112 +366,138 @@ __global__ void __launch_bounds__(InterpShape<ADJ>::kWarps * 32, InterpShape<ADJ
           __ldcg(&q64[(size_t)(P.pt_off + row) * 3 + axis]) * P.kscale64;
       grid_windows<ADJ>(A.tab, x, lane, 32, g.f[axis], g.n[axis], &sm.w[axis][0][0],
                         &sm.dw[ADJ ? axis : 0][0][0], sm.o[axis]);
-    }
-    double cm[3], cr[3];  // adjoint: coefficients of R and U in the row's scalar field
-    if constexpr (ADJ) {
-      const int gr = P.pt_off + row;
-      const float4 u = __ldcg(&op.us_t[gr]), a = __ldcg(&op.as_t[gr]);
-      cm[0] = (double)u.x - a.x; cm[1] = (double)u.y - a.y; cm[2] = (double)u.z - a.z;
-      cr[0] = a.x; cr[1] = a.y; cr[2] = a.z;
+    } else if constexpr (ADJ) {
+      if (tid < 128) {
+        const int gr = P.pt_off + row;
+        const float4 u = __ldcg(&op.us_t[gr]), a = __ldcg(&op.as_t[gr]);
+        sm.cf[0][lane] = u.x - a.x; sm.cf[1][lane] = u.y - a.y; sm.cf[2][lane] = u.z - a.z;
+        sm.cf[3][lane] = a.x; sm.cf[4][lane] = a.y; sm.cf[5][lane] = a.z;
+      }
     }
     __syncthreads();
-    int o[3], lo[3], hi[3];
+    // windows of the tile and of its four groups of eight points
+    int lo[3], hi[3], glo[2][4], ghi[2][4];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      o[d] = sm.o[d][lane];
-      lo[d] = __reduce_min_sync(0xffffffffu, o[d]);
-      hi[d] = __reduce_max_sync(0xffffffffu, o[d]) + kWin;
+      const int o = sm.o[d][lane];
+      int l = o, h = o;
+#pragma unroll
+      for (int off = 1; off < 8; off <<= 1) {
+        l = min(l, __shfl_xor_sync(0xffffffffu, l, off));
+        h = max(h, __shfl_xor_sync(0xffffffffu, h, off));
+      }
+      if (d < 2)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          glo[d][r] = __shfl_sync(0xffffffffu, l, 8 * r);
+          ghi[d][r] = __shfl_sync(0xffffffffu, h, 8 * r) + kWin;
+        }
+      lo[d] = __reduce_min_sync(0xffffffffu, o);
+      hi[d] = __reduce_max_sync(0xffffffffu, o) + kWin;
     }
     lo[2] &= ~1;  // 16-byte aligned pairs of z nodes
     const double *F = A.fld + A.off[A.slot[p]] * 6;
+    const int nchunk = (hi[1] - lo[1] + 7) / 8;
     for (int z0 = lo[2]; z0 < hi[2]; z0 += kGridKZ) {
-      double wz[kGridKZ], dz[ADJ ? kGridKZ : 1];
+      double az[4][4], adz[ADJ ? 4 : 1][ADJ ? 4 : 1];
       const int nk2 = min(kGridKZ, g.n[2] - z0) / 2;  // pairs of nodes of the grid from z0 on
 #pragma unroll
-      for (int k = 0; k < kGridKZ; ++k) {
-        const int q = z0 + k - o[2];
-        const bool in = q >= 0 && q < kWin;
-        wz[k] = in ? sm.w[2][q][lane] : 0.0;
-        if (ADJ) dz[k] = in ? sm.dw[2][q][lane] : 0.0;
-      }
-      for (int m = lo[0] + warp; m < hi[0]; m += kInterpWarps) {
-        const unsigned qx = m - o[0];
-        const double wx = qx < kWin ? sm.w[0][qx][lane] : 0.0;
-        const double dx = ADJ && qx < kWin ? sm.dw[0][qx][lane] : 0.0;
-        for (int n0 = lo[1]; n0 < hi[1]; n0 += kInterpRows) {
-          const int nr = min(kInterpRows, hi[1] - n0);
-          __syncwarp();
-          {
-            constexpr int PER = NC * (kGridKZ / 2);  // pairs per row
-            const double *f = F + ((size_t)m * g.n[1] + n0) * g.n[2] + z0;
-            double2 v[(kInterpRows * PER + 31) / 32];
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-            for (int k = 0; k < (kInterpRows * PER + 31) / 32; ++k) {
-              const int i = k * 32 + lane, r = i / PER, q = i - r * PER, c = q / (kGridKZ / 2),
-                        z = q - c * (kGridKZ / 2);
-              v[k] = make_double2(0.0, 0.0);
-              if (r < nr && z < nk2)
-                v[k] = __ldcg(reinterpret_cast<const double2 *>(
-                    f + (size_t)c * g.nodes + (size_t)r * g.n[2] + 2 * z));
-            }
+        for (int s = 0; s < 4; ++s) {
+          const int pt = 8 * r + kq, q = z0 + 4 * s + kr - sm.o[2][pt];
+          const bool in = q >= 0 && q < kWin;
+          az[r][s] = in ? sm.w[2][q][pt] : 0.0;
+          if constexpr (ADJ) adz[r][s] = in ? sm.dw[2][q][pt] : 0.0;
+        }
+      for (int u = warp; u < (hi[0] - lo[0]) * nchunk; u += kInterpWarps) {
+        const int m = lo[0] + u / nchunk, n0 = lo[1] + (u % nchunk) * 8;
+        const int nr = min(8, hi[1] - n0);
+        __syncwarp();
+        {
+          constexpr int PER = 8 * (kGridKZ / 2), NL = NC * PER / 32;
+          const double *f = F + ((size_t)m * g.n[1] + n0) * g.n[2] + z0;
+          double2 v[NL];
 #pragma unroll
-            for (int k = 0; k < (kInterpRows * PER + 31) / 32; ++k) {
-              const int i = k * 32 + lane;
-              if (i < kInterpRows * PER) (&sm.f[warp][0][0][0])[i] = v[k];
-            }
+          for (int k = 0; k < NL; ++k) {
+            const int i = k * 32 + lane, c = i / PER, r = (i / 8) & 7, z = i & 7;
+            v[k] = make_double2(0.0, 0.0);
+            if (r < nr && z < nk2)
+              v[k] = __ldcg(reinterpret_cast<const double2 *>(
+                  f + (size_t)c * g.nodes + (size_t)r * g.n[2] + 2 * z));
           }
-          __syncwarp();
-          for (int r = 0; r < nr; ++r) {
-            const unsigned qy = n0 + r - o[1];
-            const bool in = qx < kWin && qy < kWin;
-            const double wy = in ? sm.w[1][qy][lane] : 0.0;
-            const double w = wx * wy;
-            if constexpr (!ADJ) {
-              double s[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-              for (int k = 0; k < kGridKZ / 2; ++k)
+          for (int k = 0; k < NL; ++k) {
+            const int i = k * 32 + lane, c = i / PER, r = (i / 8) & 7, z = i & 7;
+            *reinterpret_cast<double2 *>(&sm.f[warp][c][r][2 * z]) = v[k];
+          }
+        }
+        __syncwarp();
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                  const double2 v = sm.f[warp][r][c][k];
-                  s[c] = fma(wz[2 * k], v.x, s[c]);
-                  s[c] = fma(wz[2 * k + 1], v.y, s[c]);
-                }
+        for (int r = 0; r < 4; ++r) {
+          if (m < glo[0][r] || m >= ghi[0][r] || n0 + 8 <= glo[1][r] || n0 >= ghi[1][r]) continue;
+          const int pt = 8 * r + kq;
+          const unsigned qx = m - sm.o[0][pt];
+          const double wx = qx < kWin ? sm.w[0][qx][pt] : 0.0;
+          double wy[2], sv[NC][2];
 #pragma unroll
-              for (int c = 0; c < 3; ++c) out[c] = fma(w, s[c], out[c]);
-            } else {
-              const double dy = in ? sm.dw[1][qy][lane] : 0.0;
-              double s[3] = {0.0, 0.0, 0.0}, ph = 0.0, pd = 0.0;
+          for (int e = 0; e < 2; ++e) {
+            const unsigned qy = n0 + 2 * kr + e - sm.o[1][pt];
+            wy[e] = qy < kWin ? sm.w[1][qy][pt] : 0.0;
+          }
 #pragma unroll
-              for (int k = 0; k < kGridKZ / 2; ++k) {
-                double e0 = 0.0, e1 = 0.0;
+          for (int c = 0; c < NC; ++c) {
+            sv[c][0] = sv[c][1] = 0.0;
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                  const double2 v = sm.f[warp][r][d][k], y = sm.f[warp][r][3 + d][k];
-                  e0 = fma(cr[d], y.x, fma(cm[d], v.x, e0));
-                  e1 = fma(cr[d], y.y, fma(cm[d], v.y, e1));
-                  s[d] = fma(wz[2 * k], y.x, s[d]);
-                  s[d] = fma(wz[2 * k + 1], y.y, s[d]);
-                }
-                ph = fma(wz[2 * k], e0, ph);
-                ph = fma(wz[2 * k + 1], e1, ph);
-                pd = fma(dz[2 * k], e0, pd);
-                pd = fma(dz[2 * k + 1], e1, pd);
+            for (int s = 0; s < 4; ++s)
+              dmma(sv[c][0], sv[c][1], az[r][s], sm.f[warp][c][kq][4 * s + kr]);
+          }
+          if constexpr (!ADJ) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              out[r][c] = fma(wx, fma(wy[0], sv[c][0], wy[1] * sv[c][1]), out[r][c]);
+          } else {
+            const double dx = qx < kWin ? sm.dw[0][qx][pt] : 0.0;
+            double ph[2] = {0.0, 0.0}, pd[2] = {0.0, 0.0};
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+              const double cf = sm.cf[c][pt];
+              double dv[2] = {0.0, 0.0};
+#pragma unroll
+              for (int s = 0; s < 4; ++s)
+                dmma(dv[0], dv[1], adz[r][s], sm.f[warp][c][kq][4 * s + kr]);
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                ph[e] = fma(cf, sv[c][e], ph[e]);
+                pd[e] = fma(cf, dv[e], pd[e]);
               }
-#pragma unroll
-              for (int c = 0; c < 3; ++c) out[c] = fma(w, s[c], out[c]);
-              out[3] = fma(dx * wy, ph, out[3]);
-              out[4] = fma(wx * dy, ph, out[4]);
-              out[5] = fma(w, pd, out[5]);
             }
+            double dy[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const unsigned qy = n0 + 2 * kr + e - sm.o[1][pt];
+              dy[e] = qy < kWin ? sm.dw[1][qy][pt] : 0.0;
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              out[r][c] = fma(wx, fma(wy[0], sv[3 + c][0], wy[1] * sv[3 + c][1]), out[r][c]);
+            out[r][3] = fma(dx, fma(wy[0], ph[0], wy[1] * ph[1]), out[r][3]);
+            out[r][4] = fma(wx, fma(dy[0], ph[0], dy[1] * ph[1]), out[r][4]);
+            out[r][5] = fma(wx, fma(wy[0], pd[0], wy[1] * pd[1]), out[r][5]);
           }
         }
       }
     }
   }
-  __syncthreads();
-  double(*red)[NV][32] = reinterpret_cast<double(*)[NV][32]>(&sm.f[0][0][0][0]);
 #pragma unroll
-  for (int k = 0; k < NV; ++k) red[warp][k][lane] = out[k];
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      double x = out[r][k];
+      x += __shfl_xor_sync(0xffffffffu, x, 1);
+      x += __shfl_xor_sync(0xffffffffu, x, 2);
+      if (kr == 0) sm.red[warp][k][8 * r + kq] = x;
+    }
   __syncthreads();
   if (warp) return;
   double v[NV];
@@ -486,7 +505,7 @@ __global__ void __launch_bounds__(InterpShape<ADJ>::kWarps * 32, InterpShape<ADJ
   for (int k = 0; k < NV; ++k) {
     v[k] = 0.0;
 #pragma unroll
-    for (int w = 0; w < kInterpWarps; ++w) v[k] += red[w][k][lane];
+    for (int w = 0; w < kInterpWarps; ++w) v[k] += sm.red[w][k][lane];
     if (ADJ && k >= 3) v[k] *= -0.5 / 0.69314718055994530942;
   }
   double e = live ? op.finalize(p, row, v) : 0.0;

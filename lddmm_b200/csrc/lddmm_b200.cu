@@ -454,7 +454,7 @@ static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
       if (!c.grid) return cudaSuccess;
       CUE(grid_fields(c, t, op.as_t, nullptr));
       return launch_smem(grid_interp_kernel<false, ShootOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
-                         InterpShape<false>::kWarps * 32, 0, sizeof(GridInterpSmem<false>), c.stream, op,
+                         kInterpWarps * 32, 0, sizeof(GridInterpSmem<false>), c.stream, op,
                          grid_args(c, t), op.q64_t, gs);
     }
   }
@@ -500,7 +500,7 @@ static cudaError_t adjoint_impl(lddmm_ctx &c, int t, double *g, double *pdot) {
       if (!c.grid) return cudaSuccess;
       CUE(grid_fields(c, t, op.as_t, op.us_t));
       return launch_smem(grid_interp_kernel<true, AdjointOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
-                         InterpShape<true>::kWarps * 32, 0, sizeof(GridInterpSmem<true>), c.stream, op,
+                         kInterpWarps * 32, 0, sizeof(GridInterpSmem<true>), c.stream, op,
                          grid_args(c, t), (const double *)(c.q64 + (size_t)t * c.NPtot * D), gs);
     }
   }
@@ -989,11 +989,13 @@ static void kd_order(const double *x, int *idx, int lo, int hi);
 // Chooses the pairs whose Gaussian kernel sums run on a grid and allocates the grids.
 //
 // Cost per time step (shooting and adjoint), in SM clocks, measured: 0.32 N^2 for the pair
-// sweeps (40,962 landmarks: 1.92 ms); on the grid 5,000 per landmark and the convolutions,
-// 9 fields x 3 axes x about 53 taps per node at 64 per clock (20,011 landmarks: 0.35 ms
-// against 0.46).  The grid must win by a quarter: from about 20,000 landmarks on for a
-// unit shape at kernel width 0.3.  The grids of a context are bounded to 4 GB, largest
-// pairs first; each is 1.7 times the nodes of the initial box (extents up to 1.35 times).
+// sweeps (40,962 landmarks: 1.92 ms); on the grid 2,500 per landmark, the latency of four
+// dependent launches per sweep (22 M: 80 us of 148 SMs) and the convolutions, 9 fields x
+// 3 axes x about 53 taps per node at 64 per clock (20,011 landmarks: 0.28 ms against 0.46,
+// 40,962: 0.42, 163,842: 1.27 against 32).  The grid must win by a tenth: from about
+// 15,000 landmarks on for a unit shape at kernel width 0.3.  The grids of a context are
+// bounded to 4 GB, largest pairs first; each is 1.7 times the nodes of the initial box
+// (extents up to 1.35 times).
 static void kd_order(const double *x, int *idx, int lo, int hi) {
   while (hi - lo > 32) {
     const int unit = hi - lo > 128 ? 128 : 32;
@@ -1045,9 +1047,9 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
     }
     if (!fin || !(nmax <= 0.9 * kGridMaxDim)) continue;
     const double pair = 0.32 * P.N * (double)P.N;
-    const double grid = 5000.0 * P.N + 9.0 * 3.0 * std::min(nmax, 53.0) / 64.0 * nodes;
+    const double grid = 22e6 + 2500.0 * P.N + 9.0 * 3.0 * std::min(nmax, 53.0) / 64.0 * nodes;
     const long long cp = (long long)(1.7 * nodes);
-    if (pair < 1.25 * grid || (total + cp) * 6 * 16 > kGridBytes) continue;
+    if (pair < 1.1 * grid || (total + cp) * 6 * 16 > kGridBytes) continue;
     slot[p] = (int)pairs.size();
     pairs.push_back(p);
     off.push_back(total);
