@@ -152,6 +152,10 @@ __device__ __forceinline__ float abs_sum(const float4 &a) {
 __device__ __forceinline__ float abs_max(const float4 &a) {
   return fmaxf(fabsf(a.x), fmaxf(fabsf(a.y), fabsf(a.z)));
 }
+// log2 of a tile's weight; -inf (nothing is skipped) when it is not finite.
+__device__ __forceinline__ float lg2_finite(float s) {
+  return lg2f_approx(s < INFINITY ? s : 0.0f);
+}
 // A NaN or infinity anywhere in the block gives S = inf (fmaxf drops NaNs, sums keep them).
 __device__ __forceinline__ float or_inf(float s) { return s < INFINITY ? s : INFINITY; }
 
@@ -212,6 +216,10 @@ __device__ __forceinline__ void gauss_next_stats(const AdjointOp<D, ORDER> &op,
   }
 }
 
+template <int D, char CT, char DT>
+__device__ __forceinline__ void gauss_next_stats(const VarifoldOp<D, CT, DT> &,
+                                                 const GaussStats &, int, int, int, bool) {}
+
 // ------------------------------------------------------------------- split items
 //
 // The columns of an item are dealt to S independent CTAs (not a cluster: clusters are
@@ -236,7 +244,7 @@ __device__ __forceinline__ void finish_split(const Op &op, int p, int tile, int 
                                              const GaussStats &gs,
                                              const double (&v)[R][Op::NA]) {
   constexpr int NA = Op::NA, ROWS = R * 32;
-  static_assert(ROWS == W * 32, "one thread per row");
+  static_assert(ROWS <= W * 32, "one thread per row");
   __shared__ double s_red[W][32][NA];
   __shared__ double s_scr[W];
   __shared__ int s_last;
@@ -258,7 +266,7 @@ __device__ __forceinline__ void finish_split(const Op &op, int p, int tile, int 
       }
     }
   }
-  const bool mine = tid < kTile || two;
+  const bool mine = tid < ROWS && (tid < kTile || two);
   if (sp.S > 1) {
     double *slot = sp.part + (size_t)item * sp.S * ROWS * NA;
     if (mine)
@@ -306,7 +314,7 @@ __device__ __forceinline__ void finish_split(const Op &op, int p, int tile, int 
 // duplicated: 7 shared-memory loads of 16 bytes serve 16 pairs of a lane.
 
 template <int W>
-__global__ void __launch_bounds__(W * 32)
+__global__ void __launch_bounds__(W * 32, 4)
     gauss_shoot_kernel(const ShootOp<3, -1> op, const GaussStats gs,
                        const int2 *__restrict__ items, const SplitPlan sp, const GridArgs ga) {
   constexpr int NA = 3;
@@ -347,7 +355,7 @@ __global__ void __launch_bounds__(W * 32)
   const GaussTile T = gauss_tile(q, live);
   float S_I = 0.0f;
   for (int b = 0; b < (two ? 4 : 2); ++b) S_I += __ldcg(&gs.wa[blk0 + row0 / kSub + b].x);
-  const float thr = T.diag2 - lg2f_approx(S_I) + kCullBits + lg2f_approx((float)nblk);
+  const float thr = T.diag2 - lg2_finite(S_I) + kCullBits + lg2f_approx((float)nblk);
   float2 q2[4][3];  // compact: (2 x', 2 x'); else (x, x)
   double b2[4];     // |x'|^2
 #pragma unroll
@@ -536,8 +544,8 @@ __global__ void __launch_bounds__(W * 32)
   }
   const float mm = um + rm;  // bounds |m| = |u - r|
   const float bits = T.diag2 + kCullBits + lg2f_approx((float)nblk);
-  const float thr_u = bits - lg2f_approx(U_I);
-  const float thr_s = bits + 2.0f - 0.5f * lg2f_approx(T.diag2) - lg2f_approx(mm * R_I + rm * U_I);
+  const float thr_u = bits - lg2_finite(U_I);
+  const float thr_s = bits + 2.0f - 0.5f * lg2f_approx(T.diag2) - lg2_finite(mm * R_I + rm * U_I);
   float2 q2[R][3], mi[R][3], ri[R][3];
   const float qf = T.compact ? 2.0f : 1.0f;
 #pragma unroll

@@ -25,6 +25,7 @@
 #include "persist.cuh"
 #include "plan.h"
 #include "sweep.cuh"
+#include "vfd.cuh"
 
 using namespace lddmm;
 
@@ -178,8 +179,8 @@ struct lddmm_ctx {
   // items' FP64 parts and arrival counts
   bool gauss = false;
   float4 *gbox = nullptr, *gwa = nullptr, *gwu = nullptr;
-  double *gpart = nullptr;
-  unsigned int *gcnt = nullptr;
+  double *gpart = nullptr, *vpart = nullptr;  // vpart, vcnt: the split varifold sweep's
+  unsigned int *gcnt = nullptr, *vcnt = nullptr;
   // gridded kernel sums of large pairs (grid.cuh)
   bool grid = false;
   int n_grid = 0, grid_dmax = 0;        // pairs with a grid, largest extent per axis
@@ -272,7 +273,7 @@ lddmm_ctx::~lddmm_ctx() {
   dfree(cl_job_src, stream);
   dfree(dbb, stream); dfree(tbb, stream);
   dfree(gbox, stream); dfree(gwa, stream); dfree(gwu, stream); dfree(gpart, stream);
-  dfree(gcnt, stream);
+  dfree(gcnt, stream); dfree(vpart, stream); dfree(vcnt, stream);
   dfree(gblk, stream); dfree(gtile[0], stream); dfree(gtile[1], stream); dfree(gpairs, stream);
   dfree(gslot, stream); dfree(gord, stream); dfree(goff, stream); dfree(gcap, stream); dfree(gkeys, stream);
   dfree(gmax, stream); dfree(graw, stream); dfree(gfld, stream); dfree(gtab, stream);
@@ -671,6 +672,10 @@ static cudaError_t varifold_impl(lddmm_ctx &c) {
   op.ow2 = c.ow2;
   op.dbb = c.dbb;
   op.tbb = c.tbb;
+  if constexpr (D == 3 && CT == 'G' && DT == 'B')
+    return launch(vfd_split_kernel<kWarps>, (unsigned)(c.n_el_items * c.S_vfd), kWarps * 32, 0,
+                  c.stream, op, (const int2 *)c.el_items,
+                  SplitPlan{c.S_vfd, c.n_el_items, c.P == 1, c.vpart, c.vcnt});
   return launch(sweep_packed_kernel<VarifoldOp<D, CT, DT>, kWarps>,
                 (unsigned)(c.n_el_items * c.S_vfd), kWarps * 32, c.S_vfd, c.stream, op,
                 (const int2 *)c.el_items, c.S_vfd);
@@ -903,6 +908,50 @@ static int default_cluster(int n_items, int sms = 148) {
   return S;
 }
 
+// Points in k-d order: split at the median of the longest axis, at multiples of 128 and
+// then of 32 points, so that consecutive tiles of that size are compact whatever the order
+// of the mesh's vertices or elements.
+static void kd_order(const double *x, int *idx, int lo, int hi) {
+  while (hi - lo > 32) {
+    const int unit = hi - lo > 128 ? 128 : 32;
+    const int mid = lo + std::max(unit, ((hi - lo) / 2 + unit / 2) / unit * unit);
+    double l[3], h[3];
+    for (int d = 0; d < 3; ++d) l[d] = h[d] = x[(size_t)idx[lo] * 3 + d];
+    for (int k = lo + 1; k < hi; ++k)
+      for (int d = 0; d < 3; ++d) {
+        l[d] = std::min(l[d], x[(size_t)idx[k] * 3 + d]);
+        h[d] = std::max(h[d], x[(size_t)idx[k] * 3 + d]);
+      }
+    int ax = 0;
+    for (int d = 1; d < 3; ++d)
+      if (h[d] - l[d] > h[ax] - l[ax]) ax = d;
+    if (mid >= hi) return;
+    std::nth_element(idx + lo, idx + mid, idx + hi, [&](int a, int b) {
+      const double u = x[(size_t)a * 3 + ax], v = x[(size_t)b * 3 + ax];
+      return u < v || (u == v && a < b);
+    });
+    kd_order(x, idx, lo, mid);
+    lo = mid;
+  }
+}
+
+// Summed extent of the bounding boxes of consecutive 32-element blocks.
+static double block_extent(const std::vector<double> &cen, int n, const std::vector<int> *order) {
+  double sum = 0.0;
+  for (int b0 = 0; b0 < n; b0 += 32) {
+    double l[3] = {INFINITY, INFINITY, INFINITY}, h[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int k = b0; k < std::min(b0 + 32, n); ++k) {
+      const int e = order ? (*order)[k] : k;
+      for (int d = 0; d < 3; ++d) {
+        l[d] = std::min(l[d], cen[(size_t)e * 3 + d]);
+        h[d] = std::max(h[d], cen[(size_t)e * 3 + d]);
+      }
+    }
+    sum += (h[0] - l[0]) + (h[1] - l[1]) + (h[2] - l[2]);
+  }
+  return sum;
+}
+
 // Storage order of a 3D surface's elements for the varifold sweep, whose distance
 // culling tests 32-element blocks by their bounding boxes: blocks of nearby elements
 // make small boxes.  Returns the elements sorted along a Morton (Z-order) curve of
@@ -939,22 +988,20 @@ static std::vector<int> spatial_order(const std::vector<double> &cen, int n) {
   std::vector<int> perm(n);
   for (int e = 0; e < n; ++e) perm[e] = e;
   std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return code[a] < code[b]; });
-  auto extent = [&](const std::vector<int> *order) {
-    double sum = 0.0;
-    for (int b0 = 0; b0 < n; b0 += 32) {
-      double l[3] = {INFINITY, INFINITY, INFINITY}, h[3] = {-INFINITY, -INFINITY, -INFINITY};
-      for (int k = b0; k < std::min(b0 + 32, n); ++k) {
-        const int e = order ? (*order)[k] : k;
-        for (int d = 0; d < 3; ++d) {
-          l[d] = std::min(l[d], cen[(size_t)e * 3 + d]);
-          h[d] = std::max(h[d], cen[(size_t)e * 3 + d]);
-        }
-      }
-      sum += (h[0] - l[0]) + (h[1] - l[1]) + (h[2] - l[2]);
-    }
-    return sum;
-  };
-  if (extent(&perm) < 0.8 * extent(nullptr)) return perm;
+  if (block_extent(cen, n, &perm) < 0.8 * block_extent(cen, n, nullptr)) return perm;
+  return {};
+}
+
+// The same for vfd_split_kernel, in k-d order: its 64-row tiles are also more compact, which
+// a Morton curve's jumps prevent (0.9: icosphere faces come in an order as good).
+static std::vector<int> kd_spatial_order(const std::vector<double> &cen, int n) {
+  if (n < 64) return {};
+  for (double x : cen)
+    if (!std::isfinite(x)) return {};
+  std::vector<int> perm(n);
+  for (int e = 0; e < n; ++e) perm[e] = e;
+  kd_order(cen.data(), perm.data(), 0, n);
+  if (block_extent(cen, n, &perm) < 0.9 * block_extent(cen, n, nullptr)) return perm;
   return {};
 }
 
@@ -981,11 +1028,6 @@ static cudaError_t run_eval(lddmm_ctx &c, double *g_out, double *f_out, double *
 
 static int autotune(lddmm_ctx &c, const lddmm_config &cf);
 
-// Landmarks in k-d order: split at the median of the longest axis, at multiples of 128 and
-// then of 32 points, so that consecutive tiles of that size are compact whatever the order
-// of the mesh's vertices (a tile's grid work grows with its extent).
-static void kd_order(const double *x, int *idx, int lo, int hi);
-
 // Chooses the pairs whose Gaussian kernel sums run on a grid and allocates the grids.
 //
 // Cost per time step (shooting and adjoint), in SM clocks, measured: 0.32 N^2 for the pair
@@ -996,30 +1038,6 @@ static void kd_order(const double *x, int *idx, int lo, int hi);
 // 15,000 landmarks on for a unit shape at kernel width 0.3.  The grids of a context are
 // bounded to 4 GB, largest pairs first; each is 1.7 times the nodes of the initial box
 // (extents up to 1.35 times).
-static void kd_order(const double *x, int *idx, int lo, int hi) {
-  while (hi - lo > 32) {
-    const int unit = hi - lo > 128 ? 128 : 32;
-    const int mid = lo + std::max(unit, ((hi - lo) / 2 + unit / 2) / unit * unit);
-    double l[3], h[3];
-    for (int d = 0; d < 3; ++d) l[d] = h[d] = x[(size_t)idx[lo] * 3 + d];
-    for (int k = lo + 1; k < hi; ++k)
-      for (int d = 0; d < 3; ++d) {
-        l[d] = std::min(l[d], x[(size_t)idx[k] * 3 + d]);
-        h[d] = std::max(h[d], x[(size_t)idx[k] * 3 + d]);
-      }
-    int ax = 0;
-    for (int d = 1; d < 3; ++d)
-      if (h[d] - l[d] > h[ax] - l[ax]) ax = d;
-    if (mid >= hi) return;
-    std::nth_element(idx + lo, idx + mid, idx + hi, [&](int a, int b) {
-      const double u = x[(size_t)a * 3 + ax], v = x[(size_t)b * 3 + ax];
-      return u < v || (u == v && a < b);
-    });
-    kd_order(x, idx, lo, mid);
-    lo = mid;
-  }
-}
-
 static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
   constexpr long long kGridBytes = 4ll << 30;
   std::vector<int> order(c.P), pairs, slot(c.P, -1);
@@ -1254,9 +1272,9 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
           for (int k = 0; k < 3; ++k) sum += a.ini_nde[(size_t)a.dfm_elm_vtx[(size_t)e * 3 + k] * 3 + d];
           cen[(size_t)e * 3 + d] = sum / 3.0;
         }
-      dperm = spatial_order(cen, P.Ed);
-      tperm = spatial_order(std::vector<double>(a.tgt_cen_pos, a.tgt_cen_pos + (size_t)P.Et * 3),
-                            P.Et);
+      const auto order = c.ct == 'G' && c.dt == 'B' ? kd_spatial_order : spatial_order;
+      dperm = order(cen, P.Ed);
+      tperm = order(std::vector<double>(a.tgt_cen_pos, a.tgt_cen_pos + (size_t)P.Et * 3), P.Et);
     }
     if (!dperm.empty()) {
       dslot.resize(P.Ed);
@@ -1414,7 +1432,9 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
           hi[d] = std::max(hi[d], fin ? x[d] : INFINITY);
         }
       }
-      h_tbb[2 * b] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+      float area = 0.0f;  // the block's weight, for the distance test of vfd_split_kernel
+      for (int k = 32 * b; k < 32 * b + 32; ++k) area += std::fabs(h_tc[k].w);
+      h_tbb[2 * b] = make_float4(lo[0], lo[1], lo[2], std::isfinite(area) ? area : INFINITY);
       h_tbb[2 * b + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
     }
     CU(cudaMemcpyAsync(c.tbb, h_tbb.data(), sizeof(float4) * h_tbb.size(),
@@ -1495,6 +1515,10 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     for (int s = 8; s >= 1 && !S; --s)
       if (c.n_el_items <= c.vfd_clusters(s)) S = s;
     if (S) c.S_vfd = S;
+  }
+  if (c.D == 3 && c.ct == 'G' && c.dt == 'B' && c.has_vfd) {
+    CU(dalloc(c.stream, &c.vpart, (size_t)c.n_el_items * 8 * kTile * 8));
+    CU(dalloc(c.stream, &c.vcnt, c.n_el_items));
   }
   // two-tile work items for the Gaussian per-step sweeps, one tile for the Matern ones
   c.tpw_shoot = c.tpw_adj = (c.order == -1) ? 2 : 1;

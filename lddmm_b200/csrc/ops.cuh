@@ -799,8 +799,11 @@ __global__ void geometry_kernel(const PairDesc *__restrict__ pd, const int *__re
         hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], off));
       }
     }
+    float area = live ? ec[g].w : 0.0f;  // the block's weight (written by this lane above)
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) area += __shfl_xor_sync(0xffffffffu, area, off);
     if (threadIdx.x % 32 == 0) {
-      bbox[2 * (g / 32)] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+      bbox[2 * (g / 32)] = make_float4(lo[0], lo[1], lo[2], area < INFINITY ? area : INFINITY);
       bbox[2 * (g / 32) + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
     }
   }

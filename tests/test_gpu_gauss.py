@@ -103,3 +103,19 @@ def test_gridded_sums_against_fp64(n):
             dq = -2 / w2 * ((K * lr)[..., None] * d).sum(1)
             step = pst[t][rows] - pst[t - 1][rows]
             assert np.max(np.abs(P.time_stp * dq - step)) < 1e-7 * np.max(np.abs(pst[t]))
+
+
+@pytest.mark.parametrize("n,cw", [(40, 0.1), (66, 0.5), (1500, 1.0), (1500, 0.3), (1500, 0.1),
+                                  (1500, 0.02)])
+def test_split_varifold_sweep_against_the_oracle(oracle, n, cw):
+    """csrc/vfd.cuh: element tiles that are compact against the centre kernel's width, near
+    ones and wide ones (double-single differences), one 64-element tile and a partial last
+    one; value and gradient."""
+    from lddmm_b200 import api
+
+    P = _problem(n, 0.3, n + 1)
+    P.cen_width = cw
+    v, dq = api.varifold(P, P.ini_nde)
+    vo, go = oracle.varifold(P, P.ini_nde)
+    assert abs(v - vo) <= TOL * abs(vo)
+    assert rel(dq, go) < TOL
