@@ -94,123 +94,145 @@ __global__ void tri_input_kernel(const float *tri7, int B, int Et, int Etp, bf16
   const long long M = (long long)B * Etp;
   if (r >= M) return;
   const int p = (int)(r / Etp), e = (int)(r - (long long)p * Etp);
+  __align__(16) bf16 h[kTriIn];
 #pragma unroll
   for (int c = 0; c < kTriIn; ++c) {
     float v = 0.0f;
     if (e < Et && c < 7) v = tri7[((size_t)p * Et + e) * 7 + c];
-    const bf16 h = __float2bfloat16_rn(v);
-    xt[r * kTriIn + c] = h;
-    xtT[(size_t)c * M + r] = h;
+    h[c] = __float2bfloat16_rn(v);
+    xtT[(size_t)c * M + r] = h[c];
   }
+  uint4 *row = reinterpret_cast<uint4 *>(xt + r * kTriIn);
+  row[0] = reinterpret_cast<const uint4 *>(h)[0];
+  row[1] = reinterpret_cast<const uint4 *>(h)[1];
 }
 
-// g[p][c] = max over the pair's Et real rows of h2 (lowest row wins ties); arg = row
-__global__ void maxpool_kernel(const float *h2, int Et, int Etp, float *g, int *arg) {
+// g[p][c] = max over the pair's Et real rows of h2 (lowest row wins ties); arg = row.
+// kPoolSplit CTAs per pair meet in a 64-bit atomic maximum of (ordered value, ~row), which
+// does not depend on the order of arrival; one CTA per pair took 100 us for 8 pairs.
+constexpr int kPoolSplit = 16;
+__global__ void maxpool_part_kernel(const float *h2, int Et, int Etp, unsigned long long *key) {
   const int p = blockIdx.x, c = threadIdx.x & 63, part = threadIdx.x >> 6;  // 4 parts
-  __shared__ float s_v[4][64];
-  __shared__ int s_i[4][64];
+  const int e0 = (int)((long long)Et * blockIdx.y / kPoolSplit);
+  const int e1 = (int)((long long)Et * (blockIdx.y + 1) / kPoolSplit);
   float best = -INFINITY;
-  int bi = 0;
-  for (int e = part; e < Et; e += 4) {
+  int bi = -1;
+#pragma unroll 8
+  for (int e = e0 + part; e < e1; e += 4) {
     const float v = h2[((size_t)p * Etp + e) * kTriH + c];
     if (v > best) {
       best = v;
       bi = e;
     }
   }
-  s_v[part][c] = best;
-  s_i[part][c] = bi;
-  __syncthreads();
-  if (part == 0) {
-    for (int k = 1; k < 4; ++k)
-      if (s_v[k][c] > best || (s_v[k][c] == best && s_i[k][c] < bi)) {
-        best = s_v[k][c];
-        bi = s_i[k][c];
-      }
-    g[p * kTriH + c] = best;
-    arg[p * kTriH + c] = bi;
-  }
+  if (bi < 0) return;  // no value above -inf
+  const unsigned b = __float_as_uint(best);
+  const unsigned o = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  atomicMax(&key[p * kTriH + c], ((unsigned long long)o << 32) | (0xffffffffu - (unsigned)bi));
+}
+
+__global__ void maxpool_kernel(const unsigned long long *key, int n, float *g, int *arg) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const unsigned o = (unsigned)(key[k] >> 32);
+  const bool any = key[k] != 0ull;
+  g[k] = any ? __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o) : -INFINITY;
+  arg[k] = any ? (int)(0xffffffffu - (unsigned)key[k]) : 0;
 }
 
 // The k nearest target triangles of every source landmark: for pair p and landmark i,
 // the indices of the k closest triangle centres in ascending order of the squared
 // distance, computed in FP32 as ((cx - qx)^2 + (cy - qy)^2) + (cz - qz)^2 with every
-// operation rounded (no contraction), ties to the lower index.  One warp per (pair,
-// landmark): lane l keeps the sorted list of its k best among triangles l, l + 32, ...
-// in shared memory, then the warp merges the 32 lists in k rounds of a (distance,
-// index) argmin.  Requires k <= Et.
-constexpr int kKnnWarps = 4;
+// operation rounded (no contraction), ties to the lower index.  Requires k <= Et.
+// One warp per (pair, landmark), k <= 32: lane r holds the r-th nearest so far.  The
+// centres go through shared memory once per CTA (coalesced, 16 landmarks share them); 32
+// candidates are tested per step against the k-th distance, and the few that pass (about
+// k (1 + ln(Et / k)) per landmark: 150 of 5,120 at k = 24) are inserted with shuffles, in
+// increasing index order.  A sorted list per lane in shared memory instead took 32 times
+// as many insertions: 1.40 ms for 8 pairs x 2,562 landmarks.
+constexpr int kKnnWarps = 16, kKnnChunk = 2048;
 __global__ void __launch_bounds__(kKnnWarps * 32)
     knn_kernel(const float *tri7, int B, int Et, const float *xyz, int N, int k, int *nbr) {
-  __shared__ float s_d[kKnnWarps][kMaxLocal][32];
-  __shared__ int s_i[kKnnWarps][kMaxLocal][32];
+  __shared__ float s_c[3][kKnnChunk];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long item = (long long)blockIdx.x * kKnnWarps + warp;
-  if (item >= (long long)B * N) return;  // warp-uniform
-  const int p = (int)(item / N), i = (int)(item - (long long)p * N);
-  const float qx = xyz[i * 3], qy = xyz[i * 3 + 1], qz = xyz[i * 3 + 2];
+  const int per = (N + kKnnWarps - 1) / kKnnWarps;  // CTAs per pair
+  const int p = blockIdx.x / per, i = (blockIdx.x - p * per) * kKnnWarps + warp;
+  const bool on = i < N;  // warp-uniform
+  const int q = on ? i : N - 1;
+  const float qx = xyz[q * 3], qy = xyz[q * 3 + 1], qz = xyz[q * 3 + 2];
   const float *tp = tri7 + (size_t)p * Et * 7;
-  float(*ld)[32] = s_d[warp];
-  int(*li)[32] = s_i[warp];
-  int cnt = 0;
-  for (int j = lane; j < Et; j += 32) {
-    const float dx = __fsub_rn(tp[j * 7], qx), dy = __fsub_rn(tp[j * 7 + 1], qy),
-                dz = __fsub_rn(tp[j * 7 + 2], qz);
-    const float d =
-        __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-    if (cnt < k || d < ld[cnt - 1][lane]) {
-      // this lane's candidates come in increasing index, so an equal distance stays
-      // behind the entries already kept
-      int pos = cnt < k ? cnt : k - 1;
-      while (pos > 0 && ld[pos - 1][lane] > d) {
-        ld[pos][lane] = ld[pos - 1][lane];
-        li[pos][lane] = li[pos - 1][lane];
-        --pos;
+  float ld = INFINITY, thr = INFINITY;
+  int li = 0, cnt = 0;
+  for (int c0 = 0; c0 < Et; c0 += kKnnChunk) {
+    const int nc = min(kKnnChunk, Et - c0);
+    __syncthreads();
+    for (int j = threadIdx.x; j < nc * 7; j += kKnnWarps * 32) {
+      const int e = j / 7, f = j - 7 * e;
+      const float v = tp[(size_t)c0 * 7 + j];
+      if (f < 3) s_c[f][e] = v;
+    }
+    __syncthreads();
+    if (!on) continue;
+    for (int j0 = 0; j0 < nc; j0 += 32) {
+      const int j = j0 + lane;
+      float d = INFINITY;
+      if (j < nc) {
+        const float dx = __fsub_rn(s_c[0][j], qx), dy = __fsub_rn(s_c[1][j], qy),
+                    dz = __fsub_rn(s_c[2][j], qz);
+        d = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
       }
-      ld[pos][lane] = d;
-      li[pos][lane] = j;
-      if (cnt < k) ++cnt;
+      unsigned m = __ballot_sync(0xffffffffu, j < nc && (cnt < k || d < thr));
+      while (m) {
+        const int src = __ffs(m) - 1;
+        m &= m - 1u;
+        const float c = __shfl_sync(0xffffffffu, d, src);
+        if (cnt == k && !(c < thr)) continue;
+        // after the entries that are no farther (an equal distance came with a lower index)
+        const int pos = __popc(__ballot_sync(0xffffffffu, lane < cnt && !(ld > c)));
+        const float ud = __shfl_up_sync(0xffffffffu, ld, 1);
+        const int ui = __shfl_up_sync(0xffffffffu, li, 1);
+        if (lane > pos) {
+          ld = ud;
+          li = ui;
+        } else if (lane == pos) {
+          ld = c;
+          li = c0 + j0 + src;
+        }
+        cnt = min(cnt + 1, k);
+        if (cnt == k) thr = __shfl_sync(0xffffffffu, ld, k - 1);
+      }
     }
   }
-  int h = 0;  // head of this lane's list
-  for (int r = 0; r < k; ++r) {
-    float bd = h < cnt ? ld[h][lane] : INFINITY;
-    int bi = h < cnt ? li[h][lane] : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float od = __shfl_xor_sync(0xffffffffu, bd, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (od < bd || (od == bd && oi < bi)) {
-        bd = od;
-        bi = oi;
-      }
-    }
-    if (h < cnt && li[h][lane] == bi) ++h;  // indices are distinct: one lane advances
-    if (lane == 0) nbr[item * k + r] = bi;
-  }
+  if (on && lane < k) nbr[((size_t)p * N + i) * k + lane] = li;
+}
+
+// CTAs of knn_kernel for B pairs.
+unsigned knn_grid(int B, int N) {
+  return (unsigned)B * (unsigned)((N + kKnnWarps - 1) / kKnnWarps);
 }
 
 // xp [B * Np][pt_in] = (q_i, g_p, local features, 0) and its transpose: here every
-// column but the local features' (k neighbours x 7, written by local_input_kernel)
+// column but the local features' (k neighbours x 7, written by local_input_kernel).  One
+// thread per entry, of xp and of its transpose, so that both are written in order.
 __global__ void point_input_kernel(const float *xyz, int N, int Np, int B, const float *g,
                                    int k, int pt_in, bf16 *xp, bf16 *xpT) {
-  const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long M = (long long)B * Np;
-  if (r >= M) return;
-  const int p = (int)(r / Np), i = (int)(r - (long long)p * Np);
+  const long long M = (long long)B * Np, idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= M * pt_in) return;
   const int lo = 3 + kTriH, hi = 3 + kTriH + 7 * k;
-  for (int c = 0; c < pt_in; ++c) {
-    if (c == lo) c = hi;  // the local columns
-    if (c >= pt_in) break;
+  auto value = [&](long long r, int c) {
+    const int p = (int)(r / Np), i = (int)(r - (long long)p * Np);
     float v = 0.0f;
     if (i < N) {
       if (c < 3) v = xyz[i * 3 + c];
-      else if (c < 3 + kTriH) v = g[p * kTriH + c - 3];
+      else if (c < lo) v = g[p * kTriH + c - 3];
     }
-    const bf16 h = __float2bfloat16_rn(v);
-    xp[r * pt_in + c] = h;
-    xpT[(size_t)c * M + r] = h;
-  }
+    return __float2bfloat16_rn(v);
+  };
+  const long long r = idx / pt_in;
+  const int c = (int)(idx - r * pt_in);
+  if (c < lo || c >= hi) xp[idx] = value(r, c);
+  const int ct = (int)(idx / M);
+  if (ct < lo || ct >= hi) xpT[idx] = value(idx - (long long)ct * M, ct);
 }
 
 // The local columns of xp / xpT: neighbour n of row r (thread n M + r, rows fastest, so
@@ -291,7 +313,14 @@ __global__ void rowsum_kernel(const bf16 *xT, long long M, float *out) {
   __shared__ float s[kThreads / 32];
   const bf16 *row = xT + (size_t)blockIdx.x * M;
   float acc = 0.0f;
-  for (long long k = threadIdx.x; k < M; k += kThreads) acc += __bfloat162float(row[k]);
+  // 16 bytes per load: M is a multiple of 16
+  for (long long k = threadIdx.x; k < M / 8; k += kThreads) {
+    const uint4 u = reinterpret_cast<const uint4 *>(row)[k];
+    const unsigned w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      acc += __uint_as_float(w[j] << 16) + __uint_as_float(w[j] & 0xffff0000u);
+  }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = acc;
   __syncthreads();
@@ -302,25 +331,28 @@ __global__ void rowsum_kernel(const bf16 *xT, long long M, float *out) {
   }
 }
 
-// pair sums of the first point layer's pre-activation gradient, then through the g
-// columns of P1: dg[p][c] = sum_o (sum_{i of p} da1[p][i][o]) Wt_P1[o][3 + c];
-// block per pair, threads over o
-__global__ void dg_kernel(const bf16 *da1T, long long M, int Np, const float *wt_p1, int pt_in,
-                          float *dg) {
-  const int p = blockIdx.x;
-  __shared__ float s_o[kPtH];
-  for (int o = threadIdx.x; o < kPtH; o += blockDim.x) {
-    const bf16 *row = da1T + (size_t)o * M + (size_t)p * Np;
-    float a = 0.0f;
-    for (int i = 0; i < Np; ++i) a += __bfloat162float(row[i]);
-    s_o[o] = a;
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < kTriH; c += blockDim.x) {
-    float a = 0.0f;
-    for (int o = 0; o < kPtH; ++o) a = fmaf(s_o[o], wt_p1[o * pt_in + 3 + c], a);
-    dg[p * kTriH + c] = a;
-  }
+// pair sums of the first point layer's pre-activation gradient: s[p][o] = sum_{i of p}
+// da1[p][i][o], one warp per (p, o)
+__global__ void pair_sum_kernel(const bf16 *da1T, long long M, int Np, float *s) {
+  const int p = blockIdx.x, lane = threadIdx.x & 31;
+  const int o = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const unsigned *row =
+      reinterpret_cast<const unsigned *>(da1T + (size_t)o * M + (size_t)p * Np);  // Np % 16 == 0
+  float a = 0.0f;
+#pragma unroll 8
+  for (int i = lane; i < Np / 2; i += 32)
+    a += __uint_as_float(row[i] << 16) + __uint_as_float(row[i] & 0xffff0000u);
+  for (int k = 16; k > 0; k >>= 1) a += __shfl_xor_sync(0xffffffffu, a, k);
+  if (lane == 0) s[p * kPtH + o] = a;
+}
+
+// the same through the g columns of P1: dg[p][c] = sum_o s[p][o] Wt_P1[o][3 + c]
+__global__ void dg_kernel(const float *s, const float *wt_p1, int pt_in, float *dg) {
+  const int p = blockIdx.x, c = threadIdx.x;
+  float a = 0.0f;
+#pragma unroll 8
+  for (int o = 0; o < kPtH; ++o) a = fmaf(s[p * kPtH + o], wt_p1[o * pt_in + 3 + c], a);
+  dg[p * kTriH + c] = a;
 }
 
 // the max-pool's gradient: dh2 is zero except at each (pair, channel)'s argmax row
@@ -403,6 +435,8 @@ struct lddmm_ws {
        *dh2T = nullptr, *dh1T = nullptr;
   float *pre_h1 = nullptr, *h2 = nullptr, *g = nullptr, *dg = nullptr;
   int *arg = nullptr;
+  unsigned long long *pool = nullptr;
+  float *psum = nullptr;
   bf16 *xp = nullptr, *xpT = nullptr, *a1 = nullptr, *a1T = nullptr, *a2 = nullptr,
        *a2T = nullptr, *dy = nullptr, *dyT = nullptr, *da2 = nullptr, *da2T = nullptr,
        *da1 = nullptr, *da1T = nullptr;
@@ -634,14 +668,17 @@ int forward(lddmm_ws &w, const float *tri7, int B, int Et, const int *nbr_in = n
   a.out = w.h2;
   a.ldo = kTriH;
   WCU(gemm(w, a, 1));
-  maxpool_kernel<<<B, 256, 0, w.stream>>>(w.h2, Et, Etp, w.g, w.arg);
+  WCU(cudaMemsetAsync(w.pool, 0, sizeof(unsigned long long) * B * kTriH, w.stream));
+  maxpool_part_kernel<<<dim3(B, kPoolSplit), 256, 0, w.stream>>>(w.h2, Et, Etp, w.pool);
+  maxpool_kernel<<<(B * kTriH + kThreads - 1) / kThreads, kThreads, 0, w.stream>>>(
+      w.pool, B * kTriH, w.g, w.arg);
   const int *nbr = nbr_in ? nbr_in : w.nbr;
   if (w.local_k > 0 && !nbr_in) {
-    const long long items = (long long)B * w.N;
-    knn_kernel<<<(unsigned)((items + kKnnWarps - 1) / kKnnWarps), kKnnWarps * 32, 0,
-                 w.stream>>>(tri7, B, Et, w.xyz, w.N, w.local_k, w.nbr);
+    knn_kernel<<<knn_grid(B, w.N), kKnnWarps * 32, 0, w.stream>>>(
+        tri7, B, Et, w.xyz, w.N, w.local_k, w.nbr);
   }
-  point_input_kernel<<<(unsigned)((Mp + kThreads - 1) / kThreads), kThreads, 0, w.stream>>>(
+  point_input_kernel<<<(unsigned)((Mp * w.pt_in + kThreads - 1) / kThreads), kThreads, 0,
+                       w.stream>>>(
       w.xyz, w.N, w.Np, B, w.g, w.local_k, w.pt_in, w.xp, w.xpT);
   if (w.local_k > 0) {
     const long long n = Mp * w.local_k;
@@ -726,8 +763,8 @@ int backward(lddmm_ws &w, int B, int Et, const float *labels, float label_weight
   WCU(gemm(w, a, 1));
   // P1 (its input gradient is needed only in the g columns, summed over each pair)
   WCU(weight_grad(w, w.L[2], w.da1T, w.xpT, Mp));
-  dg_kernel<<<B, 256, 0, w.stream>>>(w.da1T, Mp, w.Np, w.params + w.L[2].w_off, w.pt_in,
-                                     w.dg);
+  pair_sum_kernel<<<dim3(B, kPtH / 8), 256, 0, w.stream>>>(w.da1T, Mp, w.Np, w.psum);
+  dg_kernel<<<B, kTriH, 0, w.stream>>>(w.psum, w.params + w.L[2].w_off, w.pt_in, w.dg);
   WCU(cudaMemsetAsync(w.dh2, 0, sizeof(bf16) * Mt * kTriH, w.stream));
   WCU(cudaMemsetAsync(w.dh2T, 0, sizeof(bf16) * Mt * kTriH, w.stream));
   unpool_kernel<<<(B * kTriH + kThreads - 1) / kThreads, kThreads, 0, w.stream>>>(
@@ -873,6 +910,8 @@ extern "C" int lddmm_ws_create_ex(int n_src, const double *src_nde, int time_ste
   WCU(W.alloc(&W.g, (size_t)batch_max * kTriH));
   WCU(W.alloc(&W.dg, (size_t)batch_max * kTriH));
   WCU(W.alloc(&W.arg, (size_t)batch_max * kTriH));
+  WCU(W.alloc(&W.pool, (size_t)batch_max * kTriH));
+  WCU(W.alloc(&W.psum, (size_t)batch_max * kPtH));
   WCU(W.alloc(&W.xp, Mp * W.pt_in));
   WCU(W.alloc(&W.xpT, Mp * W.pt_in));
   WCU(W.alloc(&W.nbr, (size_t)batch_max * n_src * std::max(local_k, 1)));
@@ -956,9 +995,8 @@ extern "C" int lddmm_ws_neighbours(lddmm_ws *w, const float *d_tri7, int pairs, 
   }
   int rc = check_batch(*w, pairs, tri_num);
   if (rc) return rc;
-  const long long items = (long long)pairs * w->N;
-  knn_kernel<<<(unsigned)((items + kKnnWarps - 1) / kKnnWarps), kKnnWarps * 32, 0,
-               w->stream>>>(d_tri7, pairs, tri_num, w->xyz, w->N, w->local_k, d_nbr);
+  knn_kernel<<<knn_grid(pairs, w->N), kKnnWarps * 32, 0, w->stream>>>(
+      d_tri7, pairs, tri_num, w->xyz, w->N, w->local_k, d_nbr);
   WCU(cudaGetLastError());
   WCU(cudaStreamSynchronize(w->stream));
   return 0;
