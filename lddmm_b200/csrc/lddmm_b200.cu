@@ -150,6 +150,7 @@ struct lddmm_ctx {
   // persistent multi-step sweeps (one cooperative launch per direction)
   bool persistent = false;
   int pers_ctas = 0;          // CTAs of the persistent kernels (one share of work each)
+  bool pers_one = false;      // ... as one cluster
   // cluster form of the persistent sweeps (persist.cuh persistent_cluster_kernel):
   // pers_kind 1 runs it, on pers_cl_ctas CTAs in clusters of pers_C; 0 the L2 form
   int pers_kind = 0, pers_C = 0, pers_cl_ctas = 0;
@@ -233,6 +234,7 @@ struct lddmm_ctx {
   cudaError_t (*adjoint)(lddmm_ctx &, int t, double *g, double *pdot) = nullptr;
   cudaError_t (*shoot_all)(lddmm_ctx &, double *vlc) = nullptr;
   cudaError_t (*adjoint_all)(lddmm_ctx &, double *g) = nullptr;
+  bool (*pers_one_ok)(int G) = nullptr;
   int (*pers_blocks)(int which) = nullptr;  // resident CTAs per SM of the persistent kernels
   // co-resident clusters of C CTAs of the cluster-form persistent kernels (min of both)
   int (*pers_clusters)(int C, int grid) = nullptr;
@@ -552,6 +554,9 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
   plan.unit_parts = c.unit_parts;
   plan.part = c.seg_part;
   plan.cnt = c.unit_cnt;
+  if (c.pers_one)  // one cluster: stream serialisation like every other sweep
+    return launch(persistent_sweep_kernel<Op, true>, (unsigned)c.pers_ctas, kPersistWarps * 32,
+                  c.pers_ctas, c.stream, op, plan, T, dir, c.sync);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)c.pers_ctas);
   cfg.blockDim = dim3(kPersistWarps * 32);
@@ -561,7 +566,33 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, persistent_sweep_kernel<Op>, op, plan, T, dir, c.sync);
+  return cudaLaunchKernelEx(&cfg, persistent_sweep_kernel<Op, false>, op, plan, T, dir, c.sync);
+}
+
+// Whether one cluster of G CTAs can run both persistent sweeps.
+template <int D, int ORDER>
+static bool pers_one_impl(int G) {
+  if (G > kOneCluster) return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)G);
+  cfg.blockDim = dim3(kPersistWarps * 32);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)G;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int a = 0, b = 0;
+  const auto ks = persistent_sweep_kernel<ShootOp<D, ORDER>, true>;
+  const auto ka = persistent_sweep_kernel<AdjointOp<D, ORDER>, true>;
+  const cudaFuncAttribute np = cudaFuncAttributeNonPortableClusterSizeAllowed;
+  const bool ok = cudaFuncSetAttribute(ks, np, 1) == cudaSuccess &&
+                  cudaFuncSetAttribute(ka, np, 1) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&a, ks, &cfg) == cudaSuccess &&
+                  cudaOccupancyMaxActiveClusters(&b, ka, &cfg) == cudaSuccess && a > 0 && b > 0;
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 
 template <int D, int ORDER>
@@ -649,9 +680,9 @@ static int pers_blocks_impl(int which) {
   int n = 0;
   cudaError_t e = (which == 0)
       ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, persistent_sweep_kernel<ShootOp<D, ORDER>>, kPersistWarps * 32, 0)
+            &n, persistent_sweep_kernel<ShootOp<D, ORDER>, false>, kPersistWarps * 32, 0)
       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, persistent_sweep_kernel<AdjointOp<D, ORDER>>, kPersistWarps * 32, 0);
+            &n, persistent_sweep_kernel<AdjointOp<D, ORDER>, false>, kPersistWarps * 32, 0);
   return e == cudaSuccess ? n : 0;
 }
 
@@ -696,6 +727,7 @@ static void set_def(lddmm_ctx &c) {
   c.shoot_all = shoot_all_impl<D, ORDER>;
   c.adjoint_all = adjoint_all_impl<D, ORDER>;
   c.pers_blocks = pers_blocks_impl<D, ORDER>;
+  c.pers_one_ok = pers_one_impl<D, ORDER>;
   c.pers_clusters = pers_clusters_impl<D, ORDER>;
   c.probe_cluster = probe_cluster_impl<D, ORDER>;
 }
@@ -791,24 +823,37 @@ static cudaError_t launch_objective(lddmm_ctx &c, PairState *st, double *f_out) 
                 groups ? c.ngrp_tot : c.ntile_tot, c.vfd_part, c.T, st, f_out, groups);
 }
 
-// FP64 alpha (variable layout) -> FP32 point layout used by the sweeps.
-__global__ void alpha_to_f32_kernel(const PairDesc *__restrict__ pd, int P, const double *x,
-                                    float4 *as, int NPtot, int D, int T) {
+// Start of every entry point, in one launch: the trial point x (variable layout) copied to
+// XT and to the sweeps' FP32 point layout, every pair active, the persistent kernels'
+// barrier words and the split row groups' arrival counts cleared (after a clean launch they
+// are zero already, after a timed-out one they are not).
+__global__ void trial_begin_kernel(const PairDesc *__restrict__ pd, int P, const double *x,
+                                   double *xt, float4 *as, int NPtot, int D, int T, long long nvar,
+                                   int *act, StepSync *sy, unsigned int *cnt, int ncnt) {
   pdl_wait();
   pdl_trigger();
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  // locate the pair (P is small; linear scan)
-  int p = 0;
-  while (p + 1 < P && v >= pd[p + 1].var_off) ++p;
+  const long long nthr = (long long)gridDim.x * blockDim.x;
+  for (long long k = v; k < P; k += nthr) act[k] = 1;
+  for (long long k = v; k < ncnt; k += nthr) cnt[k] = 0u;
+  if (v == 0) sy->arrive = sy->error = sy->depart = 0u;
+  if (v >= nvar) return;
+  int p = 0, q = P - 1;  // the pair: the last one whose variables begin at or before v
+  while (p < q) {
+    const int m = (p + q + 1) / 2;
+    if (pd[m].var_off <= v) p = m;
+    else q = m - 1;
+  }
   const PairDesc &Q = pd[p];
-  if (v >= Q.var_off + Q.var_num) return;
+  const double y = x[v];
+  if (x != xt) xt[v] = y;
   const long long w = v - Q.var_off;
   const long long nd = (long long)Q.N * D;
   const int t = (int)(w / nd);
   const long long rem = w - (long long)t * nd;
   const int i = (int)(rem / D), d = (int)(rem - (long long)i * D);
   if (t >= T) return;
-  reinterpret_cast<float *>(as)[((size_t)t * NPtot + Q.pt_off + i) * 4 + d] = (float)x[v];
+  reinterpret_cast<float *>(as)[((size_t)t * NPtot + Q.pt_off + i) * 4 + d] = (float)y;
 }
 
 __global__ void set_int_kernel(int *a, int n, int v) {
@@ -1544,6 +1589,7 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     if (c.persistent) {
       const HostPlan h = plan_sweeps(uni, c.hpd, cap);
       c.pers_ctas = (int)h.cta_seg.size() - 1;
+      c.pers_one = c.pers_one_ok(c.pers_ctas);
       c.n_segs = (int)h.segs.size();
       c.n_slots = h.slots;
       CU(dalloc(c.stream, &c.segs, c.n_segs));
@@ -1740,12 +1786,24 @@ static cudaError_t run_eval(lddmm_ctx &c, double *g_out, double *f_out, double *
   return cudaSuccess;
 }
 
-static cudaError_t load_trial(lddmm_ctx &c, const double *d_alp, bool host) {
-  CUE(cudaMemcpyAsync(c.XT, d_alp, sizeof(double) * c.nvar,
-                      host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, c.stream));
-  const long long n = c.nvar;
-  return launch(alpha_to_f32_kernel, (unsigned)((n + 255) / 256), 256, 0, c.stream, c.pd, c.P,
-                (const double *)c.XT, c.as, c.NPtot, c.D, c.T);
+// Trial point, activity and synchronisation words of a new call (trial_begin_kernel).
+static cudaError_t begin_trial(lddmm_ctx &c, const double *alp, bool host) {
+  const double *src = alp;
+  if (host) {
+    CUE(cudaMemcpyAsync(c.XT, alp, sizeof(double) * c.nvar, cudaMemcpyHostToDevice, c.stream));
+    src = c.XT;
+  }
+  const long long n = std::max<long long>(c.nvar, 1);
+  return launch(trial_begin_kernel, (unsigned)((n + 255) / 256), 256, 0, c.stream, c.pd, c.P, src,
+                c.XT, c.as, c.NPtot, c.D, c.T, c.nvar, c.act, c.sync, c.unit_cnt,
+                c.unit_cnt ? c.n_units : 0);
+}
+
+// Waits for the stream; LDDMM_ERR_TIMEOUT when a persistent sweep's barrier gave up.
+static int finish_call(lddmm_ctx &c) {
+  if (c.persistent) return check_sync(c);  // its read-back waits
+  CU(cudaStreamSynchronize(c.stream));
+  return 0;
 }
 
 extern "C" int lddmm_objgrd_device(lddmm_ctx *ctx, const double *d_alp, double *d_fcn,
@@ -1756,15 +1814,9 @@ extern "C" int lddmm_objgrd_device(lddmm_ctx *ctx, const double *d_alp, double *
   }
   lddmm_ctx &c = *ctx;
   CU(cudaSetDevice(c.device));
-  CU(reset_sync(c));
-  CU(launch_set_active(c, c.P));
-  CU(load_trial(c, d_alp, false));
+  CU(begin_trial(c, d_alp, false));
   CU(run_eval(c, d_grd ? d_grd : c.GT, d_fcn, nullptr, true));
-  if (!async) {
-    CU(cudaStreamSynchronize(c.stream));
-    return check_sync(c);
-  }
-  return 0;
+  return async ? 0 : finish_call(c);
 }
 
 extern "C" int lddmm_objgrd_costate(lddmm_ctx *ctx, const double *d_alp, double *d_fcn,
@@ -1775,17 +1827,14 @@ extern "C" int lddmm_objgrd_costate(lddmm_ctx *ctx, const double *d_alp, double 
   }
   lddmm_ctx &c = *ctx;
   CU(cudaSetDevice(c.device));
-  CU(reset_sync(c));
-  CU(launch_set_active(c, c.P));
-  CU(load_trial(c, d_alp, false));
+  CU(begin_trial(c, d_alp, false));
   // the adjoint launches of this evaluation take the output pointer by value; every
   // other evaluation (and every captured graph) sees none
   c.pst_out = d_pst;
   const cudaError_t e = run_eval(c, d_grd ? d_grd : c.GT, d_fcn, nullptr, true);
   c.pst_out = nullptr;
   CU(e);
-  CU(cudaStreamSynchronize(c.stream));
-  return check_sync(c);
+  return finish_call(c);
 }
 
 extern "C" int lddmm_objgrd(lddmm_ctx *ctx, const double *alp, double *fcn, double *grd) {
@@ -1795,9 +1844,7 @@ extern "C" int lddmm_objgrd(lddmm_ctx *ctx, const double *alp, double *fcn, doub
   }
   lddmm_ctx &c = *ctx;
   CU(cudaSetDevice(c.device));
-  CU(reset_sync(c));
-  CU(launch_set_active(c, c.P));
-  CU(load_trial(c, alp, true));
+  CU(begin_trial(c, alp, true));
   CU(run_eval(c, c.GT, c.f_dev, nullptr, grd != nullptr));
   CU(cudaMemcpyAsync(fcn, c.f_dev, sizeof(double) * c.P, cudaMemcpyDeviceToHost, c.stream));
   if (grd) CU(cudaMemcpyAsync(grd, c.GT, sizeof(double) * c.nvar, cudaMemcpyDeviceToHost, c.stream));
@@ -1813,12 +1860,10 @@ extern "C" int lddmm_shoot(lddmm_ctx *ctx, const double *alp, double *nde_stk, d
   lddmm_ctx &c = *ctx;
   const int D = c.D;
   CU(cudaSetDevice(c.device));
-  CU(launch_set_active(c, c.P));
-  CU(load_trial(c, alp, true));
+  CU(begin_trial(c, alp, true));
   double *vlc = nullptr;
   CU(dalloc(c.stream, &vlc, (size_t)c.T * c.NPtot * D));
-  cudaError_t e = reset_sync(c);
-  if (e == cudaSuccess) e = gauss_begin(c);
+  cudaError_t e = gauss_begin(c);
   if (e == cudaSuccess && c.persistent) e = c.shoot_all(c, vlc);
   for (int t = 0; t < c.T && e == cudaSuccess && !c.persistent; ++t)
     e = c.shoot(c, t, vlc + (size_t)t * c.NPtot * D);
@@ -2101,7 +2146,6 @@ static int lbfgs_run(lddmm_ctx &c, const lddmm_opt *opt, const double *alp, bool
   o.rec_cap = std::min(opt->itr_max + 1, 100001);
   CU(cudaSetDevice(c.device));
   CU(ensure_lbfgs_buffers(c, o.mem_num, o.rec_cap));
-  CU(reset_sync(c));
   // initial state: every pair evaluates its starting point
   std::vector<PairState> hs(c.P);
   for (auto &s : hs) {
@@ -2111,8 +2155,7 @@ static int lbfgs_run(lddmm_ctx &c, const lddmm_opt *opt, const double *alp, bool
     s.newIdx = -1;
   }
   CU(cudaMemcpyAsync(c.st, hs.data(), sizeof(PairState) * c.P, cudaMemcpyHostToDevice, c.stream));
-  CU(launch_set_active(c, c.P));
-  CU(load_trial(c, alp, host));
+  CU(begin_trial(c, alp, host));
   CU(cudaMemcpyAsync(c.X, c.XT, sizeof(double) * c.nvar, cudaMemcpyDeviceToDevice, c.stream));
   // safety bound on cycles: every iteration takes at most bisMax + epdMax + 2
   // evaluations (>= 62); the per-pair state machine ends well before this.

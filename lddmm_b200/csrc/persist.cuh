@@ -287,11 +287,22 @@ __device__ __forceinline__ void persist_load_round(const Op &op, const int4 *seg
   __syncthreads();
 }
 
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Op: the sweep interface of sweep.cuh plus set_step(t) (pointers of time step t) and
 // write_group(p, k, v) (row-group partial of a kTileSum op).
 // dir = +1 runs t = 0..T-1, dir = -1 runs t = T-1..0.
 // Two CTAs per SM (<= 128 registers), 16 warps per SM.
-template <class Op>
+// ONE: the whole grid is one thread-block cluster (at most kOneCluster CTAs: small pairs),
+// whose hardware barrier replaces the grid barrier's atomics and polls: 3.3 -> 2.3 us per
+// shooting step of 200 points.  It waits without a bound, but a cluster is co-resident by
+// definition and every CTA of it reaches every barrier.
+constexpr int kOneCluster = 16;
+
+template <class Op, bool ONE>
 __global__ void __launch_bounds__(kPersistWarps * 32, 2)
     persistent_sweep_kernel(Op op, SweepPlan plan, int T, int dir, StepSync *sy) {
   constexpr int JW = Op::JW;
@@ -377,9 +388,13 @@ __global__ void __launch_bounds__(kPersistWarps * 32, 2)
         }
       }
     }
-    if (!grid_barrier(sy, (unsigned)(s + 1) * gridDim.x, (unsigned)s)) return;
+    if (ONE) {
+      if (s + 1 < T) cluster_sync_all();
+    } else if (!grid_barrier(sy, (unsigned)(s + 1) * gridDim.x, (unsigned)s)) {
+      return;
+    }
   }
-  grid_depart(sy);
+  if (!ONE) grid_depart(sy);
   stamp_exit(sy, dir > 0 ? 0 : 1);
   pdl_trigger();
 }
@@ -420,11 +435,6 @@ __device__ __forceinline__ unsigned int cluster_nctas() {
   unsigned int n;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
   return n;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned int count) {
