@@ -99,8 +99,8 @@ struct DefKernel {
 //           interpolation of K0 and K1 in double precision, within 2.1e-9.
 // Relative error against double-precision K0 / K1 stays below 1e-6 over x in [1e-8, 90].
 // Bound by FMA issue (18 and 28 per point); a trapezoid rule with 14 exponentials for 2 < x
-// <= 10 and an asymptotic series beyond took 7.6 instead of 5.6 us per shooting step of 500
-// points.
+// <= 10 and an asymptotic series beyond took 7.55 instead of 6.73 us per shooting step of 500
+// points and 8.54 instead of 7.43 per adjoint step.
 __device__ __forceinline__ float lg2f_approx(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

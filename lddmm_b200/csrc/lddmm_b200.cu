@@ -150,7 +150,8 @@ struct lddmm_ctx {
   // persistent multi-step sweeps (one cooperative launch per direction)
   bool persistent = false;
   int pers_ctas = 0;          // CTAs of the persistent kernels (one share of work each)
-  bool pers_one = false;      // ... as one cluster
+  // small form (pers_kind 2): CTAs per pair, threads, points of the largest pair
+  int small_C = 0, small_threads = 0, small_np = 0;
   // cluster form of the persistent sweeps (persist.cuh persistent_cluster_kernel):
   // pers_kind 1 runs it, on pers_cl_ctas CTAs in clusters of pers_C; 0 the L2 form
   int pers_kind = 0, pers_C = 0, pers_cl_ctas = 0;
@@ -234,7 +235,7 @@ struct lddmm_ctx {
   cudaError_t (*adjoint)(lddmm_ctx &, int t, double *g, double *pdot) = nullptr;
   cudaError_t (*shoot_all)(lddmm_ctx &, double *vlc) = nullptr;
   cudaError_t (*adjoint_all)(lddmm_ctx &, double *g) = nullptr;
-  bool (*pers_one_ok)(int G) = nullptr;
+  bool (*small_ok)(int C, int threads, int np) = nullptr;
   int (*pers_blocks)(int which) = nullptr;  // resident CTAs per SM of the persistent kernels
   // co-resident clusters of C CTAs of the cluster-form persistent kernels (min of both)
   int (*pers_clusters)(int C, int grid) = nullptr;
@@ -547,6 +548,10 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
     cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, persistent_cluster_kernel<Op>, op, cp, T, dir, c.sync);
   }
+  if (c.pers_kind == 2)  // one cluster per pair: stream serialisation like the other sweeps
+    return launch_smem(small_sweep_kernel<Op>, dim3((unsigned)(c.P * c.small_C)),
+                       (unsigned)c.small_threads, c.small_C, small_smem<Op>(c.small_np), c.stream,
+                       op, c.small_C, c.small_np, T, dir, c.sync);
   SweepPlan plan;
   plan.units = c.units;
   plan.segs = c.segs;
@@ -554,9 +559,6 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
   plan.unit_parts = c.unit_parts;
   plan.part = c.seg_part;
   plan.cnt = c.unit_cnt;
-  if (c.pers_one)  // one cluster: stream serialisation like every other sweep
-    return launch(persistent_sweep_kernel<Op, true>, (unsigned)c.pers_ctas, kPersistWarps * 32,
-                  c.pers_ctas, c.stream, op, plan, T, dir, c.sync);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)c.pers_ctas);
   cfg.blockDim = dim3(kPersistWarps * 32);
@@ -566,33 +568,39 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, persistent_sweep_kernel<Op, false>, op, plan, T, dir, c.sync);
+  return cudaLaunchKernelEx(&cfg, persistent_sweep_kernel<Op>, op, plan, T, dir, c.sync);
 }
 
-// Whether one cluster of G CTAs can run both persistent sweeps.
+// Whether clusters of C CTAs of the small form can run both persistent sweeps.
 template <int D, int ORDER>
-static bool pers_one_impl(int G) {
-  if (G > kOneCluster) return false;
+static bool small_ok_impl(int C, int threads, int np) {
+  const auto ks = small_sweep_kernel<ShootOp<D, ORDER>>;
+  const auto ka = small_sweep_kernel<AdjointOp<D, ORDER>>;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)G);
-  cfg.blockDim = dim3(kPersistWarps * 32);
+  cfg.gridDim = dim3((unsigned)C);
+  cfg.blockDim = dim3((unsigned)threads);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)G;
+  attr[0].val.clusterDim.x = (unsigned)C;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  const cudaFuncAttribute np16 = cudaFuncAttributeNonPortableClusterSizeAllowed,
+                          dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
   int a = 0, b = 0;
-  const auto ks = persistent_sweep_kernel<ShootOp<D, ORDER>, true>;
-  const auto ka = persistent_sweep_kernel<AdjointOp<D, ORDER>, true>;
-  const cudaFuncAttribute np = cudaFuncAttributeNonPortableClusterSizeAllowed;
-  const bool ok = cudaFuncSetAttribute(ks, np, 1) == cudaSuccess &&
-                  cudaFuncSetAttribute(ka, np, 1) == cudaSuccess &&
-                  cudaOccupancyMaxActiveClusters(&a, ks, &cfg) == cudaSuccess &&
-                  cudaOccupancyMaxActiveClusters(&b, ka, &cfg) == cudaSuccess && a > 0 && b > 0;
+  bool ok = cudaFuncSetAttribute(ks, np16, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(ka, np16, 1) == cudaSuccess &&
+            cudaFuncSetAttribute(ks, dyn, (int)small_smem<ShootOp<D, ORDER>>(kSmallMax)) ==
+                cudaSuccess &&
+            cudaFuncSetAttribute(ka, dyn, (int)small_smem<AdjointOp<D, ORDER>>(kSmallMax)) ==
+                cudaSuccess;
+  cfg.dynamicSmemBytes = small_smem<ShootOp<D, ORDER>>(np);
+  ok = ok && cudaOccupancyMaxActiveClusters(&a, ks, &cfg) == cudaSuccess;
+  cfg.dynamicSmemBytes = small_smem<AdjointOp<D, ORDER>>(np);
+  ok = ok && cudaOccupancyMaxActiveClusters(&b, ka, &cfg) == cudaSuccess;
   if (!ok) cudaGetLastError();
-  return ok;
+  return ok && a > 0 && b > 0;
 }
 
 template <int D, int ORDER>
@@ -680,9 +688,9 @@ static int pers_blocks_impl(int which) {
   int n = 0;
   cudaError_t e = (which == 0)
       ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, persistent_sweep_kernel<ShootOp<D, ORDER>, false>, kPersistWarps * 32, 0)
+            &n, persistent_sweep_kernel<ShootOp<D, ORDER>>, kPersistWarps * 32, 0)
       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, persistent_sweep_kernel<AdjointOp<D, ORDER>, false>, kPersistWarps * 32, 0);
+            &n, persistent_sweep_kernel<AdjointOp<D, ORDER>>, kPersistWarps * 32, 0);
   return e == cudaSuccess ? n : 0;
 }
 
@@ -727,7 +735,7 @@ static void set_def(lddmm_ctx &c) {
   c.shoot_all = shoot_all_impl<D, ORDER>;
   c.adjoint_all = adjoint_all_impl<D, ORDER>;
   c.pers_blocks = pers_blocks_impl<D, ORDER>;
-  c.pers_one_ok = pers_one_impl<D, ORDER>;
+  c.small_ok = small_ok_impl<D, ORDER>;
   c.pers_clusters = pers_clusters_impl<D, ORDER>;
   c.probe_cluster = probe_cluster_impl<D, ORDER>;
 }
@@ -1589,7 +1597,6 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     if (c.persistent) {
       const HostPlan h = plan_sweeps(uni, c.hpd, cap);
       c.pers_ctas = (int)h.cta_seg.size() - 1;
-      c.pers_one = c.pers_one_ok(c.pers_ctas);
       c.n_segs = (int)h.segs.size();
       c.n_slots = h.slots;
       CU(dalloc(c.stream, &c.segs, c.n_segs));
@@ -1653,6 +1660,26 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
           c.pers_C = 0;
         }
         CU(cudaMemsetAsync(c.sync, 0, sizeof(StepSync), c.stream));
+      }
+      if (cf.persistent == 0) {
+        // the small form: one cluster per pair of at most 512 points, beyond which a CTA's
+        // rows no longer fit its threads (at 500 points it ties with the L2 form, at 200 it
+        // takes three quarters of the time); no more CTAs than the smallest pair has 16-row
+        // groups (a CTA's energy partial takes one's place).  Autotuning times all forms
+        int np = 0, ng = kSmallCtas;
+        for (const PairDesc &d : c.hpd) {
+          np = std::max(np, d.Npad);
+          ng = std::min(ng, d.Npad / kGroup);
+        }
+        const int C = ng >= 16 ? 16 : ng >= 8 ? 8 : 4;
+        const int threads = pad_to((np + C - 1) / C * kSmallLanes, 32);
+        if (np <= kSmallMax && threads <= kSmallMax && 2 * threads >= np &&
+            c.small_ok(C, threads, np)) {
+          c.small_C = C;
+          c.small_threads = threads;
+          c.small_np = np;
+          c.pers_kind = 2;
+        }
       }
       if (cf.persistent == 2 && c.pers_C == 0) {
         set_err("the cluster form of the persistent sweeps is not available for this batch "
@@ -1748,7 +1775,7 @@ extern "C" int lddmm_ctx_launch_config(const lddmm_ctx *c, int *o) {
 extern "C" int lddmm_ctx_launch_shape(const lddmm_ctx *c, int *o, int n) {
   if (!c || !o || n < 0) return LDDMM_ERR_ARG;
   const long long v[11] = {c->S_shoot, c->S_adj, c->S_vfd, c->tpw_shoot, c->tpw_adj,
-                           c->persistent ? 1 + c->pers_kind : 0, c->pers_C, c->pers_cl_ctas,
+                           c->persistent ? (c->pers_kind == 1 ? 2 : 1) : 0, c->pers_C, c->pers_cl_ctas,
                            c->pers_ctas, c->pers_cl_share, c->pers_l2_share};
   const int k = std::min(n, 11);
   for (int i = 0; i < k; ++i) o[i] = (int)v[i];
@@ -2529,10 +2556,11 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
       }, ms);
     };
     err = reset_sync(c);
-    float mk[2] = {1e30f, 1e30f};
-    const int k0 = cf.persistent == 2 ? 1 : 0;
-    const int k1 = (cf.persistent == 1 || !c.pers_C) ? 0 : 1;
-    for (int kind = k0; kind <= k1 && err == cudaSuccess; ++kind) {
+    float mk[3] = {1e30f, 1e30f, 1e30f};
+    for (int kind = 0; kind <= 2 && err == cudaSuccess; ++kind) {
+      if (kind == 0 && cf.persistent == 2) continue;
+      if (kind == 1 && (cf.persistent == 1 || !c.pers_C)) continue;
+      if (kind == 2 && !c.small_C) continue;
       c.pers_kind = kind;
       err = time_loops(&mk[kind]);
     }
@@ -2544,7 +2572,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
         return rc;
       }
     }
-    c.pers_kind = (mk[1] < mk[0]) ? 1 : 0;
+    c.pers_kind = (int)(std::min_element(mk, mk + 3) - mk);
     if (err == cudaSuccess && cf.persistent == 0) {
       float ms = 0.0f;
       err = time_median(c, e0, e1, reps, [&]() {
@@ -2553,7 +2581,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
         for (int t = c.T - 1; t >= 0 && e == cudaSuccess; --t) e = c.adjoint(c, t, c.GT, nullptr);
         return e;
       }, &ms);
-      if (err == cudaSuccess && ms < std::min(mk[0], mk[1])) c.persistent = false;
+      if (err == cudaSuccess && ms < mk[c.pers_kind]) c.persistent = false;
     }
   }
   cudaEventDestroy(e0);

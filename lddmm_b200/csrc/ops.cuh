@@ -143,6 +143,59 @@ struct ShootOp {
 #pragma unroll
     for (int d = 0; d < D; ++d) acc[d] = __ffma2_rn(K, aj[d], acc[d]);
   }
+  // ---- raw operands of a point (small_sweep_kernel): q, a; q comes from the step before
+  static constexpr int NRAW = 2, RAW_DYN0 = 0, RAW_DYN = 1;
+  // the row's recursion in registers: x = q_t; a step's outputs wait in out for small_flush
+  struct Small {
+    double x[3], out[6];
+  };
+  __device__ void small_init(int p, int row, Small &S) const {
+#pragma unroll
+    for (int d = 0; d < D; ++d) S.x[d] = __ldcg(&q64_t[((size_t)pd[p].pt_off + row) * D + d]);
+  }
+  __device__ void small_a(int p, int row, double (&a)[3]) const {  // a_t
+    const double *x = x64 + pd[p].var_off + ((size_t)t * pd[p].N + row) * D;
+#pragma unroll
+    for (int d = 0; d < D; ++d) a[d] = __ldcg(&x[d]);
+  }
+  __device__ double small_step(const PairDesc &P, const double (&v)[NA], const double (&a)[3],
+                               Small &S, float4 (&nx)[1]) const {
+    double e = 0.0;
+    float q[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      S.x[d] += P.dt * v[d];
+      e += a[d] * v[d];
+      q[d] = (float)(S.x[d] * P.kscale);
+      S.out[d] = S.x[d];
+      S.out[3 + d] = v[d];
+    }
+    nx[0] = make_float4(q[0], q[1], q[2], 0.0f);
+    return e;
+  }
+  __device__ void small_flush(const PairDesc &P, int row, const Small &S, const float4 (&nx)[1],
+                              bool) const {
+    const size_t g = (size_t)P.pt_off + row;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      q64_n[g * D + d] = S.out[d];
+      if (vlc64) vlc64[g * D + d] = S.out[3 + d];
+    }
+    qs_n[g] = nx[0];
+  }
+  __device__ void load_raw(int p, int j, int k, float4 &x) const {
+    const int g = pd[p].pt_off + j;
+    x = __ldcg(k == 0 ? &qs_t[g] : &as_t[g]);
+  }
+  static __device__ __forceinline__ void raw_i(const float4 (&r)[NRAW], IData &I) {
+    I.x = r[0].x;
+    I.y = r[0].y;
+    I.z = r[0].z;
+  }
+  static __device__ __forceinline__ void raw_j(const float4 (&r)[NRAW], float4 (&w)[JW]) {
+    w[0] = r[0];
+    w[1] = r[1];
+  }
   // finalize operands (loaded before the row sums are complete): q_t and a_t of the row
   struct FData {
     double q[3], a[3];
@@ -372,6 +425,70 @@ struct AdjointOp {
     for (int d = 0; d < D; ++d) {
       acc[d] = __ffma2_rn(K, uj[d], acc[d]);
       acc[D + d] = __ffma2_rn(sv, dq[d], acc[D + d]);
+    }
+  }
+  // ---- raw operands of a point (small_sweep_kernel): u, l from the step before; q, r
+  static constexpr int NRAW = 4, RAW_DYN0 = 0, RAW_DYN = 2;
+  struct Small {  // x = p
+    double x[3], out[6];
+  };
+  __device__ void small_init(int p, int row, Small &S) const {
+#pragma unroll
+    for (int d = 0; d < D; ++d) S.x[d] = __ldcg(&p64[((size_t)pd[p].pt_off + row) * D + d]);
+  }
+  __device__ void small_a(int p, int row, double (&a)[3]) const {  // a_{t-1}
+    const double *x = x64 + pd[p].var_off + ((size_t)max(t - 1, 0) * pd[p].N + row) * D;
+#pragma unroll
+    for (int d = 0; d < D; ++d) a[d] = __ldcg(&x[d]);
+  }
+  __device__ double small_step(const PairDesc &P, const double (&v)[NA], const double (&a)[3],
+                               Small &S, float4 (&nx)[2]) const {
+    float u[3] = {0.0f, 0.0f, 0.0f}, l[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      S.out[d] = P.dt * v[d];
+      S.out[3 + d] = S.x[d];
+      S.x[d] -= P.dt * (P.pd_fac * v[D + d]);
+      u[d] = (float)(a[d] - S.x[d]);
+      l[d] = (float)(0.5 * a[d] - S.x[d]);
+    }
+    nx[0] = make_float4(u[0], u[1], u[2], 0.0f);
+    nx[1] = make_float4(l[0], l[1], l[2], 0.0f);
+    return 0.0;
+  }
+  __device__ void small_flush(const PairDesc &P, int row, const Small &S, const float4 (&)[2],
+                              bool last) const {
+    const size_t o = P.var_off + ((size_t)t * P.N + row) * D;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      if (g64) g64[o + d] = S.out[d];
+      if (pst64) pst64[o + d] = S.out[3 + d];
+      if (last) p64[((size_t)P.pt_off + row) * D + d] = S.x[d];
+    }
+  }
+  __device__ void load_raw(int p, int j, int k, float4 &x) const {
+    const int g = pd[p].pt_off + j;
+    x = __ldcg(k == 0 ? &us_t[g] : k == 1 ? &ls_t[g] : k == 2 ? &qs_t[g] : &as_t[g]);
+  }
+  static __device__ __forceinline__ void raw_i(const float4 (&r)[NRAW], IData &I) {
+    const float l[3] = {r[1].x, r[1].y, r[1].z}, q[3] = {r[2].x, r[2].y, r[2].z},
+                a[3] = {r[3].x, r[3].y, r[3].z};
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      I.q[d] = q[d];
+      I.l[d] = l[d];
+      I.r[d] = a[d];
+    }
+  }
+  static __device__ __forceinline__ void raw_j(const float4 (&x)[NRAW], float4 (&w)[JW]) {
+    const float4 u = x[0], l = x[1], q = x[2], r = x[3];
+    if (D == 3) {
+      w[0] = make_float4(q.x, q.y, q.z, u.x);
+      w[1] = make_float4(u.y, u.z, l.x, l.y);
+      w[JW - 1] = make_float4(l.z, r.x, r.y, r.z);
+    } else {
+      w[0] = make_float4(q.x, q.y, u.x, u.y);
+      w[1] = make_float4(l.x, l.y, r.x, r.y);
     }
   }
   // finalize operands loaded before the row sums are complete: p of the row and, when

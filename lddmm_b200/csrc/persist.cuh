@@ -296,13 +296,7 @@ __device__ __forceinline__ void cluster_sync_all() {
 // write_group(p, k, v) (row-group partial of a kTileSum op).
 // dir = +1 runs t = 0..T-1, dir = -1 runs t = T-1..0.
 // Two CTAs per SM (<= 128 registers), 16 warps per SM.
-// ONE: the whole grid is one thread-block cluster (at most kOneCluster CTAs: small pairs),
-// whose hardware barrier replaces the grid barrier's atomics and polls: 3.3 -> 2.3 us per
-// shooting step of 200 points.  It waits without a bound, but a cluster is co-resident by
-// definition and every CTA of it reaches every barrier.
-constexpr int kOneCluster = 16;
-
-template <class Op, bool ONE>
+template <class Op>
 __global__ void __launch_bounds__(kPersistWarps * 32, 2)
     persistent_sweep_kernel(Op op, SweepPlan plan, int T, int dir, StepSync *sy) {
   constexpr int JW = Op::JW;
@@ -388,13 +382,9 @@ __global__ void __launch_bounds__(kPersistWarps * 32, 2)
         }
       }
     }
-    if (ONE) {
-      if (s + 1 < T) cluster_sync_all();
-    } else if (!grid_barrier(sy, (unsigned)(s + 1) * gridDim.x, (unsigned)s)) {
-      return;
-    }
+    if (!grid_barrier(sy, (unsigned)(s + 1) * gridDim.x, (unsigned)s)) return;
   }
-  if (!ONE) grid_depart(sy);
+  grid_depart(sy);
   stamp_exit(sy, dir > 0 ? 0 : 1);
   pdl_trigger();
 }
@@ -578,6 +568,159 @@ __global__ void __launch_bounds__(kPersistWarps * 32, 2)
   }
   cluster_sync_all();  // no CTA leaves while a peer may still read its slots
   grid_depart(sy);
+  stamp_exit(sy, dir > 0 ? 0 : 1);
+  pdl_trigger();
+}
+
+// ---------------------------------------------------------------------------------
+// Small form of the persistent sweeps, for pairs of at most 512 (padded) points: one
+// thread-block cluster per pair.  Every CTA holds all points' raw operands in shared
+// memory (two buffers, by step parity) and owns a range of rows, 16 lanes per row; a
+// finalised row's new operands go straight into every CTA's buffer of the next step
+// (distributed shared memory), and the hardware cluster barrier ends the step: no operand
+// of the recursion passes through L2 between steps, and there is no atomic to poll.
+// Operands that do not depend on the step before (a; q and r in the adjoint) are loaded
+// during the sums.  The cluster barrier waits without a bound, but a cluster is co-resident
+// by definition and every CTA of it reaches every barrier.
+// Bound by the step's own latency (a chain of shared loads, exponential, shuffles, FP64
+// finalise and cluster barrier); 16 lanes per row is the most that a block of 512 threads
+// gives 512 points in 16 CTAs.  Us per step, L2 form -> this form: 200 points (2D, Gaussian)
+// shooting 3.30 -> 2.42, adjoint 3.66 -> 2.76; 500 points (2D, Matern of order 3) 6.73 ->
+// 6.70 and 7.43 -> 7.47: the two meet at its largest pairs.
+
+constexpr int kSmallMax = 512;      // padded points of a pair; threads per CTA
+constexpr int kSmallCtas = 16;      // CTAs per cluster
+constexpr int kSmallLanes = 16;     // lanes per row
+
+template <class Op>
+__host__ __device__ constexpr size_t small_smem(int npad) {
+  return sizeof(float4) * 2 * Op::NRAW * npad;
+}
+
+template <class Op>
+__global__ void __launch_bounds__(kSmallMax, 1)
+    small_sweep_kernel(Op op, int C, int npmax, int T, int dir, StepSync *sy) {
+  constexpr int NA = Op::NA, NR = Op::NRAW, ND = Op::RAW_DYN, L = kSmallLanes;
+  static_assert(Op::RAW_DYN0 == 0, "dynamic operands first");
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  float4 *sj = reinterpret_cast<float4 *>(s_raw);  // [buffer][operand][point]
+  __shared__ double s_e[2][kSmallMax / L];
+  pdl_wait();
+  stamp_entry(sy, dir > 0 ? 0 : 1);
+  const int p = blockIdx.x / C, rank = blockIdx.x - p * C;
+  if (!op.active(p)) return;  // uniform over the cluster
+  const int tid = threadIdx.x, sub = tid % L, nth = blockDim.x;
+  const PairDesc P = op.pd[p];
+  const int N = P.N, npad = P.Npad, ngrp = npad / kGroup;
+  const int R = (N + C - 1) / C, r0 = rank * R;  // this CTA's rows
+  const int rows = max(0, min(R, N - r0)), lrow = tid / L;
+  const bool mine = lrow < rows, owner = mine && sub == 0;
+  const int row = r0 + lrow;
+  auto step_of = [&](int s) { return dir > 0 ? s : T - 1 - s; };
+  Op o = op;
+  float4 st[2][NR - ND];  // independent operands of points tid and tid + nth (npad <= 2 nth)
+  auto fetch = [&](int s) {
+    o.set_step(step_of(s));
+#pragma unroll
+    for (int k = ND; k < NR; ++k) {
+      if (tid < npad) o.load_raw(p, tid, k, st[0][k - ND]);
+      if (tid + nth < npad) o.load_raw(p, tid + nth, k, st[1][k - ND]);
+    }
+  };
+  auto put = [&](float4 *buf) {
+#pragma unroll
+    for (int k = ND; k < NR; ++k) {
+      if (tid < npad) buf[k * npmax + tid] = st[0][k - ND];
+      if (tid + nth < npad) buf[k * npmax + tid + nth] = st[1][k - ND];
+    }
+  };
+  fetch(0);
+  for (int j = tid; j < npad; j += nth)
+#pragma unroll
+    for (int k = 0; k < ND; ++k) {
+      float4 x;
+      o.load_raw(p, j, k, x);
+      sj[k * npmax + j] = x;
+      // padding keeps its (zero) operands in both buffers
+      if (j >= N) sj[(NR + k) * npmax + j] = x;
+    }
+  put(sj);
+  typename Op::Small S;
+  double a[3] = {0.0, 0.0, 0.0}, an[3] = {0.0, 0.0, 0.0};
+  if (mine) {
+    o.small_init(p, row, S);
+    o.small_a(p, row, a);
+  }
+  if (T > 1) fetch(1);
+  float4 nx[ND];
+#pragma unroll
+  for (int k = 0; k < ND; ++k) nx[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  // results of the step before: its energy partial in the place of one of the pair's
+  // 16-row groups (one per CTA), and the rows' stores
+  auto flush = [&](int s) {
+    o.set_step(step_of(s));
+    if (owner) o.small_flush(P, row, S, nx, s == T - 1);
+    if (Op::kTileSum && tid == 0) {
+      double e = 0.0;
+      for (int k = 0; k < rows; ++k) e += s_e[s & 1][k];
+      o.write_group(p, rank, e);
+      if (rank == 0)
+        for (int k = C; k < ngrp; ++k) o.write_group(p, k, 0.0);
+    }
+  };
+  cluster_sync_all();  // every CTA of the cluster runs before the first remote store
+  for (int s = 0; s < T; ++s) {
+    const int cur = s & 1;
+    const float4 *c = sj + (size_t)cur * NR * npmax;
+    float4 *nxt = sj + (size_t)(cur ^ 1) * NR * npmax;
+    if (s > 0) flush(s - 1);
+    if (s + 1 < T) {
+      put(nxt);
+      o.set_step(step_of(s + 1));
+      if (mine) o.small_a(p, row, an);
+      if (s + 2 < T) fetch(s + 2);
+    }
+    double v[NA];
+    {
+      typename Op::IData I;
+      float4 x[NR];
+#pragma unroll
+      for (int k = 0; k < NR; ++k) x[k] = c[k * npmax + (mine ? row : 0)];
+      Op::raw_i(x, I);
+      float acc[NA];  // npad / 16 <= 32 plain FP32 terms
+#pragma unroll
+      for (int q = 0; q < NA; ++q) acc[q] = 0.0f;
+      if (mine)
+#pragma unroll 4
+        for (int j = sub; j < npad; j += L) {
+          float4 w[Op::JW];
+#pragma unroll
+          for (int k = 0; k < NR; ++k) x[k] = c[k * npmax + j];
+          Op::raw_j(x, w);
+          o.template pair<0>(I, w, acc);
+        }
+#pragma unroll
+      for (int q = 0; q < NA; ++q) {
+        v[q] = acc[q];
+#pragma unroll
+        for (int off = L / 2; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
+      }
+    }
+    if (mine) {  // the same in every lane of the row, so that each can serve one CTA
+      const double e = o.small_step(P, v, a, S, nx);
+      if (Op::kTileSum && owner) s_e[cur][lrow] = e;
+    }
+    if (s + 1 < T) {
+#pragma unroll
+      for (int k = 0; k < ND; ++k)
+        if (mine && sub < C)  // lane `sub` serves cluster CTA `sub`
+          *cg::this_cluster().map_shared_rank(&nxt[k * npmax + row], sub) = nx[k];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) a[d] = an[d];
+    }
+    cluster_sync_all();
+  }
+  flush(T - 1);
   stamp_exit(sy, dir > 0 ? 0 : 1);
   pdl_trigger();
 }

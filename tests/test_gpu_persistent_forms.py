@@ -62,3 +62,26 @@ def test_cluster_form_lbfgs_follows_the_l2_form():
     # between any two launch shapes)
     r = np.abs(traces[0][:9, 0] - traces[1][:9, 0]) / np.abs(traces[0][:9, 0])
     assert r.max() < 1e-5, r.max()
+
+
+@pytest.mark.parametrize("order,width", [(-1, 0.5), (3, 0.15)])
+@pytest.mark.parametrize("sizes", [(5,), (64,), (65, 300), (128,), (129,), (257,), (500, 496),
+                                   (512,), (513,)])
+def test_small_pairs_against_the_oracle(oracle, sizes, order, width):
+    """The small form's edges: pairs that give 4, 8 and 16 CTAs, one row to a full block of
+    rows per CTA, two pairs of unequal size, 512 points (its last) and 513 (another form); the
+    2D Matern width puts its Bessel arguments on both sides of 2.  Tolerance 1e-5, that of
+    every FP32 sum of the library."""
+    from lddmm_b200 import api, problem
+
+    Ps = [problem.circle_to_square(n, 40, width) for n in sizes]
+    for P in Ps:
+        P.knl_order = order
+    alp = [np.random.default_rng(P.nde_num).normal(size=P.var_num) * 0.02 for P in Ps]
+    with api.Context(Ps, autotune=False) as ctx:
+        f, g = ctx.objgrd(np.concatenate(alp))
+    g = np.split(g, np.cumsum([P.var_num for P in Ps])[:-1])
+    for k, P in enumerate(Ps):
+        fo, go = oracle.objgrd(P, alp[k])
+        assert abs(f[k] - fo) <= TOL * abs(fo)
+        assert rel(g[k], go) < TOL
