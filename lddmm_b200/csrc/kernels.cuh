@@ -32,49 +32,89 @@ enum KernelFamily : int {
 template <int ORDER>
 struct DefKernel;
 
+// One value or a packed pair: the same operations in the same order, so that the packed
+// sweeps are bitwise the scalar ones.
+__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ void vdup(float c, float &v) { v = c; }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ void vdup(float c, float2 &v) { v = make_float2(c, c); }
+
 template <>
 struct DefKernel<-1> {
+  static constexpr int kUnroll = 2;  // j pairs unrolled in the persistent sweeps
   static __device__ __forceinline__ float val(float nr2) { return ex2f(nr2); }
   static __device__ __forceinline__ void val_w(float nr2, float &K, float &W) {
     K = ex2f(nr2);
     W = K;
   }
+  static __device__ __forceinline__ float2 val2(float2 r2) {
+    return make_float2(ex2f(-r2.x), ex2f(-r2.y));
+  }
+  static __device__ __forceinline__ void val_w2(float2 r2, float2 &K, float2 &W) {
+    K = val2(r2);
+    W = K;
+  }
 };
 
 // Matern kernels take the NEGATED squared scaled distance for symmetry with the
-// Gaussian (the pair loops produce -r2 with free negation modifiers).
+// Gaussian (the pair loops produce -r2 with free negation modifiers); the packed forms
+// take the squared distance.
 template <int ORDER>
 struct DefKernel {
-  static __device__ __forceinline__ float poly_k(float d) {
-    if (ORDER == 0) return 1.0f;
-    if (ORDER == 1) return 1.0f + d;
-    if (ORDER == 2) return fmaf(d, fmaf(d, 1.0f / 3.0f, 1.0f), 1.0f);
-    if (ORDER == 3) return fmaf(d, fmaf(d, fmaf(d, 1.0f / 15.0f, 0.4f), 1.0f), 1.0f);
-    return fmaf(d, fmaf(d, fmaf(d, fmaf(d, 1.0f / 105.0f, 2.0f / 21.0f), 3.0f / 7.0f), 1.0f), 1.0f);
+  static constexpr int kUnroll = 2;
+  // e times the polynomials in d = r ln 2
+  template <class V>
+  static __device__ __forceinline__ V times_k(V e, V r) {
+    if (ORDER == 0) return e;
+    V l, c[5];
+    vdup(kLn2, l);
+    const float k[5][5] = {{1.0f}, {1.0f, 1.0f}, {1.0f, 1.0f, 1.0f / 3.0f},
+                           {1.0f, 1.0f, 0.4f, 1.0f / 15.0f},
+                           {1.0f, 1.0f, 3.0f / 7.0f, 2.0f / 21.0f, 1.0f / 105.0f}};
+#pragma unroll
+    for (int n = 0; n <= ORDER; ++n) vdup(k[ORDER][n], c[n]);
+    if (ORDER == 1) return vmul(e, vfma(r, l, c[0]));
+    const V d = vmul(r, l);
+    V s = c[ORDER];
+#pragma unroll
+    for (int n = ORDER - 1; n >= 0; --n) s = vfma(d, s, c[n]);
+    return vmul(e, s);
   }
-  static __device__ __forceinline__ float poly_w(float d) {
-    if (ORDER <= 1) return 1.0f;
-    if (ORDER == 2) return 1.0f + d;
-    if (ORDER == 3) return fmaf(d, d + 3.0f, 3.0f);
-    return fmaf(d, fmaf(d, d + 6.0f, 15.0f), 15.0f);
+  template <class V>
+  static __device__ __forceinline__ V times_w(V e, V r) {
+    if (ORDER <= 1) return e;
+    V l, a, b;
+    vdup(kLn2, l);
+    vdup(ORDER == 2 ? 1.0f : ORDER == 3 ? 3.0f : 6.0f, a);
+    V s = vfma(r, l, a);
+    if (ORDER >= 3) {
+      const V d = vmul(r, l);
+      vdup(ORDER == 3 ? 3.0f : 15.0f, b);
+      s = vfma(d, s, b);
+      if (ORDER == 4) s = vfma(d, s, b);
+    }
+    return vmul(e, s);
   }
   static __device__ __forceinline__ float val(float nr2) {
     const float r = sqrtf_approx(-nr2);
-    const float e = ex2f(-r);
-    if (ORDER == 0) return e;
-    return e * poly_k(r * kLn2);
+    return times_k(ex2f(-r), r);
   }
   static __device__ __forceinline__ void val_w(float nr2, float &K, float &W) {
-    const float r = sqrtf_approx(-nr2);
-    const float e = ex2f(-r);
-    if (ORDER == 0) {
-      K = e;
-      W = 0.0f;
-      return;
-    }
-    const float d = r * kLn2;
-    K = e * poly_k(d);
-    W = (ORDER == 1) ? e : e * poly_w(d);
+    const float r = sqrtf_approx(-nr2), e = ex2f(-r);
+    K = times_k(e, r);
+    W = ORDER == 0 ? 0.0f : times_w(e, r);
+  }
+  static __device__ __forceinline__ float2 val2(float2 r2) {
+    const float2 r = make_float2(sqrtf_approx(r2.x), sqrtf_approx(r2.y));
+    return times_k(make_float2(ex2f(-r.x), ex2f(-r.y)), r);
+  }
+  static __device__ __forceinline__ void val_w2(float2 r2, float2 &K, float2 &W) {
+    const float2 r = make_float2(sqrtf_approx(r2.x), sqrtf_approx(r2.y)),
+                 e = make_float2(ex2f(-r.x), ex2f(-r.y));
+    K = times_k(e, r);
+    W = ORDER == 0 ? make_float2(0.0f, 0.0f) : times_w(e, r);
   }
 };
 
@@ -160,6 +200,7 @@ __device__ __forceinline__ void bessel_p01(float x, float &p0, float &p1) {
 
 template <int ORDER>
 struct MaternBessel2D {
+  static constexpr int kUnroll = 1;  // of about 200 instructions each
   // K_n(x) of the family in terms of p0, p1 and x^2
   template <int N>
   static __device__ __forceinline__ float form(float p0, float p1, float x2) {
@@ -183,6 +224,13 @@ struct MaternBessel2D {
     K = form<ORDER>(p0, p1, -nr2);
     W = (ORDER == 0) ? 0.0f : form<(ORDER > 0 ? ORDER - 1 : 0)>(p0, p1, -nr2) *
                                   (1.0f / (2.0f * (ORDER > 0 ? ORDER : 1)));
+  }
+  static __device__ __forceinline__ float2 val2(float2 r2) {
+    return make_float2(val(-r2.x), val(-r2.y));
+  }
+  static __device__ __forceinline__ void val_w2(float2 r2, float2 &K, float2 &W) {
+    val_w(-r2.x, K.x, W.x);
+    val_w(-r2.y, K.y, W.y);
   }
 };
 

@@ -553,7 +553,7 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
                        (unsigned)c.small_threads, c.small_C, small_smem<Op>(c.small_np), c.stream,
                        op, c.small_C, c.small_np, T, dir, c.sync);
   SweepPlan plan;
-  plan.units = c.units;
+  plan.units = c.pt_items;
   plan.segs = c.segs;
   plan.cta_seg = c.cta_seg;
   plan.unit_parts = c.unit_parts;
@@ -1595,14 +1595,14 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     CU(dalloc(c.stream, &c.sync, 1));
     CU(cudaMemsetAsync(c.sync, 0, sizeof(StepSync), c.stream));
     if (c.persistent) {
-      const HostPlan h = plan_sweeps(uni, c.hpd, cap);
+      const HostPlan h = plan_sweeps(pti, c.hpd, cap);
       c.pers_ctas = (int)h.cta_seg.size() - 1;
       c.n_segs = (int)h.segs.size();
       c.n_slots = h.slots;
       CU(dalloc(c.stream, &c.segs, c.n_segs));
       CU(dalloc(c.stream, &c.cta_seg, h.cta_seg.size()));
       CU(dalloc(c.stream, &c.unit_parts, h.unit_parts.size()));
-      CU(dalloc(c.stream, &c.seg_part, (size_t)std::max(c.n_slots, 1) * kGroup * kPartNA));
+      CU(dalloc(c.stream, &c.seg_part, (size_t)std::max(c.n_slots, 1) * kTile * kPartNA));
       CU(dalloc(c.stream, &c.unit_cnt, std::max(c.n_units, 1)));
       CU(cudaMemcpyAsync(c.segs, h.segs.data(), sizeof(int4) * h.segs.size(),
                          cudaMemcpyHostToDevice, c.stream));
@@ -1615,7 +1615,7 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
       for (int k = 0; k < c.pers_ctas; ++k) {
         long long sh = 0;
         for (int q = h.cta_seg[k]; q < h.cta_seg[k + 1]; ++q) sh += h.segs[q].z - h.segs[q].y;
-        l2_share = std::max(l2_share, sh);
+        l2_share = std::max(l2_share, sh * (kTile / kGroup));  // in 16-row entries
       }
       ClusterHostPlan best;
       int bestC = 0, best_ncl = 0;
@@ -1646,11 +1646,9 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
                            cudaMemcpyHostToDevice, c.stream));
         c.pers_cl_share = best.max_share;
         c.pers_l2_share = l2_share;
-        // default: the cluster form unless its balance is clearly worse than the L2
-        // form's (it saves the L2 round trips of the split row groups every step)
-        c.pers_kind = cf.persistent == 2  ? 1
-                      : cf.persistent == 1 ? 0
-                                           : ((best.max_share * 100 <= l2_share * 115) ? 1 : 0);
+        // the cluster form only where it is asked for: the L2 form's 64-row tiles take 0.52
+        // to 0.82 of its time per step over 300 to 5000 points (3D, both directions)
+        c.pers_kind = cf.persistent == 2 ? 1 : 0;
         // the runtime must accept a cooperative launch of these clusters
         cudaError_t pe = c.probe_cluster(c);
         if (pe == cudaSuccess) pe = cudaStreamSynchronize(c.stream);
@@ -2559,7 +2557,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
     float mk[3] = {1e30f, 1e30f, 1e30f};
     for (int kind = 0; kind <= 2 && err == cudaSuccess; ++kind) {
       if (kind == 0 && cf.persistent == 2) continue;
-      if (kind == 1 && (cf.persistent == 1 || !c.pers_C)) continue;
+      if (kind == 1 && cf.persistent != 2) continue;
       if (kind == 2 && !c.small_C) continue;
       c.pers_kind = kind;
       err = time_loops(&mk[kind]);

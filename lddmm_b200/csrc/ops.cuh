@@ -93,6 +93,7 @@ struct ShootOp {
   // (ax,ax,ay,ay).
   static constexpr bool kPacked = true;
   static constexpr int JWP = (D == 3) ? 3 : 2;
+  static constexpr int kUnroll = DefKernelOf<D, ORDER>::type::kUnroll;
   struct IData2 {
     float2 q[D];  // (row0, row1)
   };
@@ -138,8 +139,7 @@ struct ShootOp {
       const float2 dd = __fadd2_rn(I.q[d], mq[d]);
       r2 = __ffma2_rn(dd, dd, r2);
     }
-    const float2 K = make_float2(DefKernelOf<D, ORDER>::type::val(-r2.x),
-                                 DefKernelOf<D, ORDER>::type::val(-r2.y));
+    const float2 K = DefKernelOf<D, ORDER>::type::val2(r2);
 #pragma unroll
     for (int d = 0; d < D; ++d) acc[d] = __ffma2_rn(K, aj[d], acc[d]);
   }
@@ -360,6 +360,7 @@ struct AdjointOp {
   // each value twice: -q, u, l, r (3D: 6 float4, 2D: 4).
   static constexpr bool kPacked = true;
   static constexpr int JWP = (D == 3) ? 6 : 4;
+  static constexpr int kUnroll = DefKernelOf<D, ORDER>::type::kUnroll;
   struct IData2 {
     float2 q[D], l[D], r[D];  // (row0, row1)
   };
@@ -375,23 +376,22 @@ struct AdjointOp {
     }
   }
   __device__ void load_j2(int p, int j, float4 (&w)[JWP]) const {
-    const int g = pd[p].pt_off + j;
-    const float4 q = __ldcg(&qs_t[g]), u = __ldcg(&us_t[g]), l = __ldcg(&ls_t[g]),
-                 r = __ldcg(&as_t[g]);
-    // value k of the 4D-padded list (-q, u, l, r) sits at float pair k of w
-    float v[4 * D];
-    const float qq[3] = {q.x, q.y, q.z}, uu[3] = {u.x, u.y, u.z}, ll[3] = {l.x, l.y, l.z},
-                rr[3] = {r.x, r.y, r.z};
+    float4 v[JW];
+    load_j(p, j, v);
+    // value k of the 4D list (-q, u, l, r) sits at float pair k of w
+    float x[4 * D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      v[d] = -qq[d];
-      v[D + d] = uu[d];
-      v[2 * D + d] = ll[d];
-      v[3 * D + d] = rr[d];
+    for (int k = 0; k < JW; ++k) {
+      x[4 * k] = v[k].x;
+      x[4 * k + 1] = v[k].y;
+      x[4 * k + 2] = v[k].z;
+      x[4 * k + 3] = v[k].w;
     }
 #pragma unroll
+    for (int d = 0; d < D; ++d) x[d] = -x[d];
+#pragma unroll
     for (int k = 0; k < JWP; ++k)
-      w[k] = make_float4(v[2 * k], v[2 * k], v[2 * k + 1], v[2 * k + 1]);
+      w[k] = make_float4(x[2 * k], x[2 * k], x[2 * k + 1], x[2 * k + 1]);
   }
   template <int SET>
   __device__ __forceinline__ void pair2(const IData2 &I, const float4 (&w)[JWP],
@@ -411,10 +411,8 @@ struct AdjointOp {
       dq[d] = __fadd2_rn(I.q[d], mq[d]);
       r2 = __ffma2_rn(dq[d], dq[d], r2);
     }
-    float Kx, Wx, Ky, Wy;
-    DefKernelOf<D, ORDER>::type::val_w(-r2.x, Kx, Wx);
-    DefKernelOf<D, ORDER>::type::val_w(-r2.y, Ky, Wy);
-    const float2 K = make_float2(Kx, Ky), Wt = make_float2(Wx, Wy);
+    float2 K, Wt;
+    DefKernelOf<D, ORDER>::type::val_w2(r2, K, Wt);
     float2 lr = __fmul2_rn(I.l[0], rj[0]);
 #pragma unroll
     for (int d = 1; d < D; ++d) lr = __ffma2_rn(I.l[d], rj[d], lr);

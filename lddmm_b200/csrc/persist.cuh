@@ -8,25 +8,18 @@
 //
 //   * every CTA stays resident for the whole recursion; steps are separated by a
 //     grid barrier;
-//   * the work of a step is the list of row groups (kGroup = 16 rows of one pair)
-//     times their j ranges, laid end to end and cut into one contiguous share per CTA
-//     (host-side plan, snapped to 32-entry boundaries): every CTA gets the same number
-//     of pair interactions whatever the row-group count, so no SM idles at the barrier
-//     while another runs a second row group.  A CTA's share is a list of segments
-//     (row group, j range), taken two at a time ("rounds");
-//   * in a round the entries of its (one or two) segments, laid end to end, are cut
-//     into 8 equal contiguous warp shares (a share that straddles the two segments is
-//     processed as two pieces); lane l handles rows l % 8 and l % 8 + 8 against every
-//     4th point of each staged 32-point sub-tile (lane group l / 8), so each staged
-//     operand serves two pairs;
-//   * reductions: a shuffle butterfly over the 4 lane groups, then all 8 warps through
-//     shared memory in warp order (a warp without entries of the segment adds zero),
-//     in FP64 after the per-tile TwoSum.  A row
-//     group cut over several CTAs stores one FP64 partial per part; the CTA that
-//     completes the row group's arrival count (whichever it is) adds the parts in part
-//     order and finalises, so results are bit-reproducible for a given plan;
-//   * each segment of a round has its own 16-thread epilogue group (lanes 0-15 of warp
-//     0 or of warp 1): both run at once, with warp-level synchronisation only.
+//   * the work of a step is the list of 64-row tiles times their j ranges, cut into one
+//     share per CTA of equal cost (plan.h): no SM idles at the barrier while another runs a
+//     second tile.  A CTA's share is a list of segments (tile, j range);
+//   * each warp sums a contiguous part of the segment's j range for all 64 rows
+//     (persistent_sweep_kernel); the 8 warps' FP64 sums are added in warp order, and a tile
+//     cut over several CTAs stores one FP64 partial per part: the CTA that completes the
+//     tile's arrival count (whichever it is) adds the parts in part order and finalises, so
+//     results are bit-reproducible for a given plan.
+//
+// The cluster form (persistent_cluster_kernel) works on row groups of kGroup = 16 rows in
+// rounds of two segments (persist_round), the small form on whole pairs of a few hundred
+// points.
 //
 // Grid barrier: a monotonically increasing arrival count (fire-and-forget atomic
 // add) that the CTAs poll against (step + 1) x grid.  When a launch ends, each CTA
@@ -44,7 +37,7 @@
 
 namespace lddmm {
 
-constexpr int kGroup = 16;                // rows per persistent work unit
+constexpr int kGroup = 16;                // rows per work unit of the cluster form
 constexpr int kRowPairs = kGroup / 2;     // lanes sharing a j entry (2 rows each)
 constexpr int kLaneGroups = 32 / kRowPairs;  // j interleave inside a warp
 constexpr int kPersistWarps = 8;          // warps per persistent CTA
@@ -151,12 +144,12 @@ __device__ __forceinline__ void grid_depart(StepSync *sy) {
 
 // Work plan of the persistent sweeps (built on the host when the context is created).
 struct SweepPlan {
-  const int2 *units;      // (pair, row group) per unit
+  const int2 *units;      // (pair, 64-row tile) per unit
   const int4 *segs;       // (unit, j begin, j end, part) in CTA order
   const int *cta_seg;     // CTA k owns segs[cta_seg[k] .. cta_seg[k + 1])
   const int2 *unit_parts; // (parts, first partial slot) per unit
-  double *part;           // FP64 partials [slot][kGroup][kPartNA]
-  unsigned int *cnt;      // per-unit arrival count of split row groups (self-resetting)
+  double *part;           // FP64 partials [slot][kPartNA][kTile]
+  unsigned int *cnt;      // per-unit arrival count of split tiles (self-resetting)
 };
 
 constexpr int kPartNA = 6;  // accumulators per row in a partial slot (>= every Op::NA)
@@ -296,88 +289,176 @@ __device__ __forceinline__ void cluster_sync_all() {
 // write_group(p, k, v) (row-group partial of a kTileSum op).
 // dir = +1 runs t = 0..T-1, dir = -1 runs t = T-1..0.
 // Two CTAs per SM (<= 128 registers), 16 warps per SM.
+// Rows are taken 64 at a time (kTile), four per lane: lanes l and l + 16 hold the same rows
+// and take the even and the odd j points of a staged 32-point sub-tile, so that one staged
+// point serves four pairs per lane (with two, the 128 bytes per clock that shared memory
+// returns bound the loop, not the arithmetic).  A segment's j range is cut into 8 warp
+// shares; a warp keeps at most 32 plain FP32 terms per sum before it adds them to its FP64
+// sums in shared memory.  Bound at 2562 points by the chain around the pair loop (first loads,
+// combine of about 7 parts per tile, grid barrier: about half of the step), beyond by FP32
+// issue.  Us per step (3D Matern of order 1), 16-row groups cut over CTAs and 4 lane groups ->
+// this: 642 points shooting 4.7 -> 4.7, adjoint 6.6 -> 5.9; 2562 points 10.5 -> 8.6, 15.1 ->
+// 12.3; 5000 points 26.1 -> 21.2, 41.2 -> 32.8.
+struct SegDesc {
+  int4 seg;      // unit, j begin, j end, part
+  int row0, active;
+  int2 up;       // parts, first partial slot
+  PairDesc pd;
+};
+
 template <class Op>
 __global__ void __launch_bounds__(kPersistWarps * 32, 2)
     persistent_sweep_kernel(Op op, SweepPlan plan, int T, int dir, StepSync *sy) {
-  constexpr int JW = Op::JW;
-  constexpr int NA = Op::NA;
-  constexpr int NW = kPersistWarps;
-  static_assert(NA <= kPartNA, "partial slot too small");
+  constexpr int JW = Op::JW, NA = Op::NA;
+  constexpr int NW = kPersistWarps, NT = NW * 32, NS = NA * kTile;
+  static_assert(NA <= kPartNA && !Op::kTwoSets && kTile == 64 && NS <= 2 * NT, "shape");
   __shared__ float4 s_j[NW][JW][kSub];
-  __shared__ double s_red[2][NW][kGroup][NA];  // [segment of the round][warp][row]
-  __shared__ PairDesc s_pd[2];  // descriptors of the round's units
-  __shared__ int s_uinf[2][2];  // per round slot: pair | group << 16, active
-  __shared__ int4 s_seg[2];     // the round's segments
+  __shared__ double s_red[NW][NS];
+  __shared__ SegDesc s_d[2];
+  __shared__ int s_last;
   pdl_wait();
   stamp_entry(sy, dir > 0 ? 0 : 1);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int l16 = lane & 15, lg = lane >> 4;
   const int s0 = plan.cta_seg[blockIdx.x], s1 = plan.cta_seg[blockIdx.x + 1];
-  const bool one_round = s1 - s0 <= 2;  // descriptors loaded once for the whole launch
+  // descriptors of segment k: read once for the whole launch when the CTA has at most two
+  // (a grid barrier's acquire empties L1, and the reads depend on one another)
+  auto describe = [&](int k, SegDesc &d) {
+    const int4 sg = plan.segs[k];
+    const int2 un = plan.units[sg.x];
+    d.seg = sg;
+    d.row0 = un.y * kTile;
+    d.active = op.active(un.x);
+    d.up = plan.unit_parts[sg.x];
+    d.pd = op.pd[un.x];
+  };
+  const bool once = s1 - s0 <= 2;
+  if (once) {
+    if (tid < s1 - s0) describe(s0 + tid, s_d[tid]);
+    __syncthreads();
+  }
   for (int s = 0; s < T; ++s) {
-    const int t = dir > 0 ? s : T - 1 - s;
     Op o = op;
-    o.set_step(t);
-    for (int k = s0; k < s1; k += 2) {
-      const int nseg = min(2, s1 - k);
-      if (!one_round || s == 0)
-        persist_load_round(op, plan.segs, plan.units, k, nseg, s_seg, s_uinf, s_pd);
-      persist_round(o, nseg, s_seg, s_uinf, s_pd, s_j, s_red);
-      __syncthreads();
-      // epilogue: segment e on lanes 0-15 of warp e (both segments at once); the
-      // condition is uniform over those 16 lanes
-      const int e = warp;
-      if (e < nseg && lane < kGroup && s_uinf[e][1]) {
-        const int4 se = s_seg[e];
-        const int grp_e = s_uinf[e][0] >> 16;
-        Op &oe = o;
-        oe.pd = &s_pd[e];
-        typename Op::FData F;  // finalize operands, in flight during the combine
-        oe.fin_load(0, grp_e * kGroup + lane, F);
-        double v[NA];
+    o.set_step(dir > 0 ? s : T - 1 - s);
+    for (int k = s0; k < s1; ++k) {
+      if (k > s0) __syncthreads();  // the segment before is done with shared memory
+      if (!once) {
+        if (tid == 0) describe(k, s_d[0]);
+        __syncthreads();
+      }
+      const SegDesc &d = s_d[once ? k - s0 : 0];
+      if (!d.active) continue;  // uniform over the CTA
+      o.pd = &d.pd;             // the op reads descriptor 0 from shared memory
+      const int row0 = d.row0;
+      {
+        const int jb0 = d.seg.y, len = d.seg.z - jb0, chunk = (len + 2 * NW - 1) / (2 * NW) * 2;
+        const int jb = jb0 + min(len, chunk * warp), je = jb0 + min(len, chunk * (warp + 1));
+        float4 nxt[JW];
+        if (jb + lane < je) o.load_j(0, jb + lane, nxt);
+        typename Op::IData I[4];  // rows l16 + 16 r
 #pragma unroll
-        for (int a = 0; a < NA; ++a) {
-          // all NW warps in warp order (zeros from warps without entries here); the
-          // loads are independent of the running sum
-          double x = 0.0;
+        for (int r = 0; r < 4; ++r) o.load_i(0, row0 + 16 * r + l16, I[r]);
+        bool first = true;
+#pragma unroll 1
+        for (int c0 = jb; c0 < je || first; c0 += 2 * kSub) {
+          float acc[4][NA];
 #pragma unroll
-          for (int w = 0; w < NW; ++w) x += s_red[e][w][lane][a];
-          v[a] = x;
-        }
-        const int2 up = plan.unit_parts[se.x];
-        bool fin = true;
-        if (up.x > 1) {
-          // row group cut over several CTAs: publish this part; the CTA completing the
-          // count adds all parts in part order
-          double *slot = plan.part + ((size_t)(up.y + se.w) * kGroup + lane) * kPartNA;
+          for (int r = 0; r < 4; ++r)
 #pragma unroll
-          for (int a = 0; a < NA; ++a) slot[a] = v[a];
-          __syncwarp(0xffffu);  // the 16 lanes' part writes before lane 0's release
-          int last = 0;
-          if (lane == 0) {
-            // release: this part is visible with the count; acquire: the last arriver
-            // sees every other part
-            last = atom_add_acq_rel_gpu(&plan.cnt[se.x], 1u) == (unsigned int)up.x - 1u;
-            if (last) plan.cnt[se.x] = 0u;  // next step's arrivals come after the barrier
-          }
-          fin = __shfl_sync(0xffffu, last, 0) != 0;
-          __syncwarp(0xffffu);
-          if (fin) {
+            for (int a = 0; a < NA; ++a) acc[r][a] = 0.0f;
+          const int ce = min(je, c0 + 2 * kSub);
+#pragma unroll 1
+          for (int j0 = c0; j0 < ce; j0 += kSub) {
+            __syncwarp();
 #pragma unroll
-            for (int a = 0; a < NA; ++a) v[a] = 0.0;
-            for (int q = 0; q < up.x; ++q) {
-              const double *src = plan.part + ((size_t)(up.y + q) * kGroup + lane) * kPartNA;
+            for (int x = 0; x < JW; ++x) s_j[warp][x][lane] = nxt[x];
+            __syncwarp();
+            const int cnt = min(kSub, je - j0);
+            if (j0 + kSub + lane < je) o.load_j(0, j0 + kSub + lane, nxt);
+#pragma unroll Op::kUnroll
+            for (int jj = lg; jj < cnt; jj += 2) {
+              float4 w[JW];
 #pragma unroll
-              for (int a = 0; a < NA; ++a) v[a] += __ldcg(src + a);
+              for (int x = 0; x < JW; ++x) w[x] = s_j[warp][x][jj];
+#pragma unroll
+              for (int r = 0; r < 4; ++r) o.template pair<0>(I[r], w, acc[r]);
             }
           }
-        }
-        if (fin) {
-          double en = oe.finalize(0, grp_e * kGroup + lane, v, F);
-          if (Op::kTileSum) {
+          // the two lane halves: each keeps two of its rows and receives the other's sums
 #pragma unroll
-            for (int off = kGroup / 2; off > 0; off >>= 1)
-              en += __shfl_xor_sync(0xffffu, en, off);
-            if (lane == 0) oe.write_group(0, grp_e, en);
+          for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+              const float keep = lg ? acc[2 + r][a] : acc[r][a],
+                          give = lg ? acc[r][a] : acc[2 + r][a];
+              double x = (double)keep + (double)__shfl_xor_sync(0xffffffffu, give, 16);
+              double *y = &s_red[warp][a * kTile + 32 * lg + 16 * r + l16];
+              if (!first) x += *y;
+              *y = x;
+            }
+          first = false;
+        }
+      }
+      typename Op::FData F;  // finalize operands, in flight during the combine
+      if (tid < kTile) o.fin_load(0, row0 + tid, F);
+      __syncthreads();
+      // the 8 warps in warp order; thread i takes sums i and i + 256
+      const int parts = d.up.x;
+      double *part = plan.part + (size_t)d.up.y * kTile * kPartNA;
+      double x[2] = {0.0, 0.0};
+#pragma unroll
+      for (int w = 0; w < NW; ++w)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (tid + h * NT < NS) x[h] += s_red[w][tid + h * NT];
+      bool fin = true;
+      if (parts > 1) {
+        // tile cut over several CTAs: the CTA that completes the count adds all parts in
+        // part order
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (tid + h * NT < NS) part[(size_t)d.seg.w * kTile * kPartNA + tid + h * NT] = x[h];
+        __syncthreads();  // the parts are written before thread 0's release
+        if (tid == 0) {
+          unsigned int *cnt = &plan.cnt[d.seg.x];
+          s_last = atom_add_acq_rel_gpu(cnt, 1u) == (unsigned int)parts - 1u;
+          if (s_last) *cnt = 0u;  // next step's arrivals come after the barrier
+        }
+        __syncthreads();
+        fin = s_last != 0;
+        if (fin) {
+          x[0] = x[1] = 0.0;
+          for (int q0 = 0; q0 < parts; q0 += 8) {  // 8 parts' loads in flight at once
+            double y[2][8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+              for (int h = 0; h < 2; ++h)
+                y[h][q] = q0 + q < parts && tid + h * NT < NS
+                              ? __ldcg(part + (size_t)(q0 + q) * kTile * kPartNA + tid + h * NT)
+                              : 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) x[h] += y[h][q];
+          }
+        }
+      }
+      if (fin) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)  // (sum i of warp 0 was read by this thread alone)
+          if (tid + h * NT < NS) s_red[0][tid + h * NT] = x[h];
+        __syncthreads();
+        if (tid < kTile) {
+          double v[NA];
+#pragma unroll
+          for (int a = 0; a < NA; ++a) v[a] = s_red[0][a * kTile + tid];
+          double en = o.finalize(0, row0 + tid, v, F);
+          if (Op::kTileSum) {
+            // energy partials in the places of the tile's 16-row groups
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) en += __shfl_xor_sync(0xffffffffu, en, off);
+            if (lane < 2) o.write_group(0, row0 / kGroup + 2 * warp + lane, lane ? 0.0 : en);
           }
         }
       }

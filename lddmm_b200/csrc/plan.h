@@ -14,12 +14,11 @@ namespace lddmm {
 constexpr int kPlanSub = 32;          // j entries per staged sub-tile (kSub)
 constexpr int kPlanMaxJobParts = 8;   // parts of a row group in the cluster form (kMaxJobParts)
 
-// Work plan of the persistent sweeps: the step's work (row groups x their j ranges,
-// laid end to end in unit order) cut into G contiguous shares, one per CTA.  Cuts
-// inside a row group are rounded to the 32-entry sub-tile and moved to the row group's
-// edge when they would leave a part shorter than kMinPart entries.  With little work
-// per CTA (under kSplitMin entries) row groups are not cut at all: each CTA takes whole
-// row groups and G is at most the row-group count.
+// Work plan of the persistent sweeps: the units' (64-row tiles') j ranges laid end to end
+// and dealt to at most G CTAs, each up to the same cost, a segment costing its entries plus
+// kSegCost (a CTA's combine and finalise, in entries of pair time); the smallest such cost is
+// found by bisection.  Cuts fall on multiples of 16 entries and leave at least kMinSeg (fewer
+// per CTA cost more in parts than they save in pair time).
 struct HostPlan {
   std::vector<int4> segs;       // (unit, j begin, j end, part) in CTA order
   std::vector<int> cta_seg;     // G + 1 offsets into segs
@@ -27,61 +26,59 @@ struct HostPlan {
   int slots = 0;
 };
 
-constexpr long long kMinPart = 32;
-constexpr long long kSplitMin = 512;
+constexpr int kSegCost = 64;
+constexpr int kMinSeg = 64;
 
 inline HostPlan plan_sweeps(const std::vector<int2> &units, const std::vector<PairDesc> &hpd,
-                            int G_max) {
+                            int G) {
   const int nu = (int)units.size();
-  std::vector<long long> us(nu + 1, 0);
-  for (int u = 0; u < nu; ++u) us[u + 1] = us[u] + hpd[units[u].x].Npad;
-  const long long W = us[nu];
-  const bool cut = W / std::max(G_max, 1) >= kSplitMin;
-  const int G = cut ? G_max : std::max(1, std::min(G_max, nu));
-  std::vector<long long> b(G + 1, 0);
-  b[G] = W;
-  for (int k = 1; k < G; ++k) {
-    long long x;
-    if (cut) {
-      const long long w = W * k / G;
-      int u = (int)(std::upper_bound(us.begin(), us.end(), w) - us.begin()) - 1;
-      u = std::min(std::max(u, 0), nu - 1);
-      const long long J = us[u + 1] - us[u];
-      long long off = (w - us[u] + kPlanSub / 2) / kPlanSub * kPlanSub;
-      if (off < kMinPart) off = 0;
-      else if (J - off < kMinPart) off = J;
-      x = us[u] + off;
-    } else {
-      x = us[(long long)nu * k / G];
-    }
-    b[k] = std::max(b[k - 1], std::min(x, W));
-  }
   HostPlan h;
-  h.cta_seg.assign(G + 1, 0);
-  h.unit_parts.assign(nu, make_int2(0, 0));
-  std::vector<int> parts(nu, 0);
-  int u0 = 0;
-  for (int k = 0; k < G; ++k) {
-    h.cta_seg[k] = (int)h.segs.size();
-    while (u0 < nu && us[u0 + 1] <= b[k]) ++u0;
-    for (int v = u0; v < nu && us[v] < b[k + 1]; ++v) {
-      const long long lo = std::max(b[k], us[v]) - us[v];
-      const long long hi = std::min(b[k + 1], us[v + 1]) - us[v];
-      if (hi > lo) h.segs.push_back(make_int4(v, (int)lo, (int)hi, parts[v]++));
+  auto deal = [&](long long cap, bool emit) {
+    int ctas = 1;
+    long long left = cap;
+    for (int u = 0; u < nu; ++u) {
+      const int J = hpd[units[u].x].Npad;
+      int part = 0;
+      for (int x = 0; x < J;) {
+        int n = (int)std::min<long long>(J - x, std::max(left - kSegCost, 0LL) / 16 * 16);
+        if (n < J - x && J - x - n < kMinSeg) n = J - x - kMinSeg;
+        if (n < std::min(kMinSeg, J - x)) {  // no room here: the next CTA
+          ++ctas;
+          left = cap;
+          if (emit) h.cta_seg.push_back((int)h.segs.size());
+          continue;
+        }
+        if (emit) h.segs.push_back(make_int4(u, x, x + n, part));
+        ++part;
+        left -= n + kSegCost;
+        x += n;
+      }
+      if (emit) {
+        h.unit_parts.push_back(make_int2(part, h.slots));
+        if (part > 1) h.slots += part;
+      }
     }
+    return ctas;
+  };
+  long long lo = 2 * kMinSeg + kSegCost, hi = lo;
+  for (int u = 0; u < nu; ++u) hi += hpd[units[u].x].Npad + kSegCost;
+  while (lo < hi) {
+    const long long mid = (lo + hi) / 2;
+    if (deal(mid, false) <= std::max(G, 1)) hi = mid;
+    else lo = mid + 1;
   }
-  h.cta_seg[G] = (int)h.segs.size();
-  for (int v = 0; v < nu; ++v) {
-    h.unit_parts[v] = make_int2(parts[v], h.slots);
-    if (parts[v] > 1) h.slots += parts[v];
-  }
+  h.cta_seg.push_back(0);
+  deal(lo, true);
+  h.cta_seg.push_back((int)h.segs.size());
   return h;
 }
+
+constexpr long long kMinPart = 32;  // shortest part of a cut row group (cluster form)
 
 // Work plan of the cluster-form persistent sweeps: the row groups split into ncl
 // contiguous ranges of whole row groups, one per cluster, minimising the largest
 // range's work (binary search on the bound, greedy fill); each cluster's entries cut
-// into C CTA shares as in plan_sweeps.  Only a CTA's first and last segment can be part
+// into C equal CTA shares.  Only a CTA's first and last segment can be part
 // of a row group shared with other CTAs (slots 0 and 1); the CTA holding a shared row
 // group's first part finalises it (at most one per CTA: only a CTA's last segment can
 // be a first part).  CTA k * C + r is rank r of cluster k.  max_share: the largest CTA

@@ -85,3 +85,35 @@ def test_small_pairs_against_the_oracle(oracle, sizes, order, width):
         fo, go = oracle.objgrd(P, alp[k])
         assert abs(f[k] - fo) <= TOL * abs(fo)
         assert rel(g[k], go) < TOL
+
+
+@pytest.mark.parametrize("n", [64, 65, 1200, 2049, 3000])
+def test_row_tiles_against_the_oracle(oracle, n):
+    """The L2 form's 64-row tiles: one tile, a second of one row, tiles cut into more than 8
+    parts (1200), CTAs that take the end of one tile and the start of the next (3000)."""
+    from lddmm_b200 import api, problem, shapes
+
+    v, f = shapes.decimated_star(n, 6, 0.05, n)
+    tv, tf = shapes.icosphere(1)
+    P = problem.Problem(v, f, *shapes.varifold_of(tv, tf), knl_order=1, knl_width=0.4, time_num=4,
+                        time_stp=1 / 3, cen_width=0.3)
+    alp = np.random.default_rng(n).normal(size=P.var_num) * 0.02
+    f, g, _ = _objgrd(P, alp, 1)
+    fo, go = oracle.objgrd(P, alp)
+    assert abs(f - fo) <= TOL * abs(fo)
+    assert rel(g, go) < TOL
+
+
+def test_row_tiles_of_many_pairs(oracle):
+    """More tiles than twice the resident CTAs: shares of three and more whole tiles."""
+    from lddmm_b200 import api, problem
+
+    Ps = [problem.circle_to_square(200 + 5 * k, 40, time_num=4) for k in range(130)]
+    alp = [np.random.default_rng(k).normal(size=P.var_num) * 0.02 for k, P in enumerate(Ps)]
+    with api.Context(Ps, persistent=1) as ctx:
+        f, g = ctx.objgrd(np.concatenate(alp))
+    g = np.split(g, np.cumsum([P.var_num for P in Ps])[:-1])
+    for k in (0, 64, 129):
+        fo, go = oracle.objgrd(Ps[k], alp[k])
+        assert abs(f[k] - fo) <= TOL * abs(fo)
+        assert rel(g[k], go) < TOL
