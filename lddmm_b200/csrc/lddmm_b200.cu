@@ -1595,7 +1595,7 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     CU(dalloc(c.stream, &c.sync, 1));
     CU(cudaMemsetAsync(c.sync, 0, sizeof(StepSync), c.stream));
     if (c.persistent) {
-      const HostPlan h = plan_sweeps(pti, c.hpd, cap);
+      const HostPlan h = plan_sweeps(pti, c.hpd, cap, sms);
       c.pers_ctas = (int)h.cta_seg.size() - 1;
       c.n_segs = (int)h.segs.size();
       c.n_slots = h.slots;

@@ -297,8 +297,8 @@ __device__ __forceinline__ void cluster_sync_all() {
 // sums in shared memory.  Bound at 2562 points by the chain around the pair loop (first loads,
 // combine of about 7 parts per tile, grid barrier: about half of the step), beyond by FP32
 // issue.  Us per step (3D Matern of order 1), 16-row groups cut over CTAs and 4 lane groups ->
-// this: 642 points shooting 4.7 -> 4.7, adjoint 6.6 -> 5.9; 2562 points 10.5 -> 8.6, 15.1 ->
-// 12.3; 5000 points 26.1 -> 21.2, 41.2 -> 32.8.
+// this: 642 points shooting 4.7 -> 4.5, adjoint 6.6 -> 5.6; 1200 points 5.8 -> 5.1, 8.9 -> 6.5;
+// 2562 points 10.5 -> 8.6, 15.1 -> 12.3; 5000 points 26.1 -> 20.4, 41.2 -> 31.9.
 struct SegDesc {
   int4 seg;      // unit, j begin, j end, part
   int row0, active;
@@ -428,17 +428,17 @@ __global__ void __launch_bounds__(kPersistWarps * 32, 2)
         fin = s_last != 0;
         if (fin) {
           x[0] = x[1] = 0.0;
-          for (int q0 = 0; q0 < parts; q0 += 8) {  // 8 parts' loads in flight at once
-            double y[2][8];
+          for (int q0 = 0; q0 < parts; q0 += 10) {  // 10 parts' loads in flight at once
+            double y[2][10];
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
+            for (int q = 0; q < 10; ++q)
 #pragma unroll
               for (int h = 0; h < 2; ++h)
                 y[h][q] = q0 + q < parts && tid + h * NT < NS
                               ? __ldcg(part + (size_t)(q0 + q) * kTile * kPartNA + tid + h * NT)
                               : 0.0;
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
+            for (int q = 0; q < 10; ++q)
 #pragma unroll
               for (int h = 0; h < 2; ++h) x[h] += y[h][q];
           }

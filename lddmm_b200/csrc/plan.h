@@ -16,9 +16,14 @@ constexpr int kPlanMaxJobParts = 8;   // parts of a row group in the cluster for
 
 // Work plan of the persistent sweeps: the units' (64-row tiles') j ranges laid end to end
 // and dealt to at most G CTAs, each up to the same cost, a segment costing its entries plus
-// kSegCost (a CTA's combine and finalise, in entries of pair time); the smallest such cost is
-// found by bisection.  Cuts fall on multiples of 16 entries and leave at least kMinSeg (fewer
-// per CTA cost more in parts than they save in pair time).
+// kSegCost (a CTA's combine and finalise, in entries of pair time: with 64 instead of 256 a
+// step of 4000 points took 15.2 / 23.0 us shooting / adjoint instead of 14.6 / 22.2); the
+// smallest such cost is found by bisection.  Cuts fall on multiples of 16 entries and leave
+// at least kMinSeg.  A CTA takes no less than a tenth of the longest range: a tile's parts are
+// read ten at a time.  With sms given, G being twice that, one CTA per SM is preferred where
+// its shares are under 0.8 of what two CTAs of an SM take together: two hide each other's
+// latency, but a few SMs with two would be waited for (1200 points: 152 CTAs took 5.5 / 7.4 us
+// per step, 133 take 5.1 / 6.5).
 struct HostPlan {
   std::vector<int4> segs;       // (unit, j begin, j end, part) in CTA order
   std::vector<int> cta_seg;     // G + 1 offsets into segs
@@ -26,11 +31,11 @@ struct HostPlan {
   int slots = 0;
 };
 
-constexpr int kSegCost = 64;
-constexpr int kMinSeg = 64;
+constexpr int kSegCost = 256;
+constexpr int kMinSeg = 32;
 
 inline HostPlan plan_sweeps(const std::vector<int2> &units, const std::vector<PairDesc> &hpd,
-                            int G) {
+                            int G, int sms = 0) {
   const int nu = (int)units.size();
   HostPlan h;
   auto deal = [&](long long cap, bool emit) {
@@ -60,15 +65,29 @@ inline HostPlan plan_sweeps(const std::vector<int2> &units, const std::vector<Pa
     }
     return ctas;
   };
-  long long lo = 2 * kMinSeg + kSegCost, hi = lo;
-  for (int u = 0; u < nu; ++u) hi += hpd[units[u].x].Npad + kSegCost;
-  while (lo < hi) {
-    const long long mid = (lo + hi) / 2;
-    if (deal(mid, false) <= std::max(G, 1)) hi = mid;
-    else lo = mid + 1;
+  long long lo = 2 * kMinSeg, hi = kSegCost;
+  for (int u = 0; u < nu; ++u) {
+    const int J = hpd[units[u].x].Npad;
+    lo = std::max(lo, (J + 159LL) / 160 * 16);
+    hi += J + kSegCost;
+  }
+  lo += kSegCost;
+  auto smallest = [&](int ctas) {
+    long long l = lo, r = std::max(hi, lo);
+    while (l < r) {
+      const long long mid = (l + r) / 2;
+      if (deal(mid, false) <= ctas) r = mid;
+      else l = mid + 1;
+    }
+    return l;
+  };
+  long long cap = smallest(std::max(G, 1));
+  if (sms > 0 && deal(cap, false) > sms) {
+    const long long one = smallest(sms);
+    if (one - kSegCost < 0.8 * 2 * (cap - kSegCost)) cap = one;
   }
   h.cta_seg.push_back(0);
-  deal(lo, true);
+  deal(cap, true);
   h.cta_seg.push_back((int)h.segs.size());
   return h;
 }
