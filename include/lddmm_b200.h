@@ -310,7 +310,8 @@ int lddmm_fp32_peak(int device, double *tflops);
 int lddmm_pipe_peaks(int device, double *out);
 
 /* Storage order that lddmm_ctx_create gives the elements of a 3D surface (and the
- * target's): cen is n x 3 element centres; perm[k] receives the element stored in
+ * target's), except with Gaussian centres and Binet directions, whose sweep stores them
+ * in a k-d order: cen is n x 3 element centres; perm[k] receives the element stored in
  * slot k.  Returns 1 when the elements are reordered along a Morton curve of their
  * centres (because that makes the varifold sweep's 32-element blocks more compact),
  * 0 when the given order is kept (perm is then the identity).  Host only. */

@@ -323,161 +323,162 @@ __global__ void __launch_bounds__(W * 32, 4)
   pdl_trigger();
   int skip = -1;  // pair found to have nothing to do here
   for (int unit = blockIdx.x; unit < sp.items * sp.S; unit += gridDim.x) {
-  const int S = sp.S;
-  const int item = unit / S;
-  const int rank = unit - item * S;
-  const int2 it = items[item];
-  const int p = it.x, tile = it.y;
-  if (p == skip) continue;
-  GridDesc gd;
-  if (!op.active(p) || grid_active(ga, p, false, gd)) {
-    if (sp.one) return;
-    skip = p;
-    continue;
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const PairDesc &P = op.pd[p];
-  const int pt = P.pt_off, npad = P.Npad;
-  const int row0 = tile * kTile;
-  const bool two = row0 + kTile < npad;  // uniform over the cluster
-  const int blk0 = pt / kSub, nblk = npad / kSub;
-  // pairs with a grid come here when it cannot hold the step; their blocks have no
-  // statistics and every block is evaluated
-  const bool cull = !ga.slot || ga.slot[p] < 0;
-  float4 q[4];
-  bool live[4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int row = (r < 2 || two) ? row0 + 32 * r + lane : row0 + lane;
-    live[r] = row < P.N;
-    q[r] = __ldcg(&op.qs_t[pt + row]);
-  }
-  const GaussTile T = gauss_tile(q, live);
-  float S_I = 0.0f;
-  for (int b = 0; b < (two ? 4 : 2); ++b) S_I += __ldcg(&gs.wa[blk0 + row0 / kSub + b].x);
-  const float thr = T.diag2 - lg2_finite(S_I) + kCullBits + lg2f_approx((float)nblk);
-  float2 q2[4][3];  // compact: (2 x', 2 x'); else (x, x)
-  double b2[4];     // |x'|^2
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const float x = q[r].x - T.c[0], y = q[r].y - T.c[1], z = q[r].z - T.c[2];
-    b2[r] = (double)x * x + (double)y * y + (double)z * z;
-    const float f = T.compact ? 2.0f : 1.0f;
-    q2[r][0] = make_float2(f * x, f * x);
-    q2[r][1] = make_float2(f * y, f * y);
-    q2[r][2] = make_float2(f * z, f * z);
-  }
-  float hi[4][NA], lo[4][NA];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int a = 0; a < NA; ++a) hi[r][a] = lo[r][a] = 0.0f;
-
-  const int nw = S * W, gw = rank * W + warp;
-  int base = gw - 32 * nw;
-  unsigned mask = 0u;
-  auto next = [&]() {  // warp-uniform: the next block to evaluate, or nblk
-    while (mask == 0u) {
-      base += 32 * nw;
-      if (base >= nblk) return nblk;
-      const int sb = base + lane * nw;
-      bool keep = sb < nblk;
-      if (keep && cull) {
-        const float4 l = __ldcg(&gs.box[2 * (blk0 + sb)]), h = __ldcg(&gs.box[2 * (blk0 + sb) + 1]);
-        const float w = __ldcg(&gs.wa[blk0 + sb].x);
-        keep = !(gauss_gap2(T, l, h) >= lg2f_approx(w) + thr);
-      }
-      mask = __ballot_sync(0xffffffffu, keep);
+    const int S = sp.S;
+    const int item = unit / S;
+    const int rank = unit - item * S;
+    const int2 it = items[item];
+    const int p = it.x, tile = it.y;
+    if (p == skip) continue;
+    GridDesc gd;
+    if (!op.active(p) || grid_active(ga, p, false, gd)) {
+      if (sp.one) return;
+      skip = p;
+      continue;
     }
-    const int k = __ffs(mask) - 1;
-    mask &= mask - 1u;
-    return base + k * nw;
-  };
-  float4 nq, na;
-  auto fetch = [&](int s) {
-    nq = __ldcg(&op.qs_t[pt + s * kSub + lane]);
-    na = __ldcg(&op.as_t[pt + s * kSub + lane]);
-  };
-  float(*sj)[kSub] = s_j[warp];
-  int s = next();
-  if (s < nblk) fetch(s);
-  while (s < nblk) {
-    __syncwarp();
-    {
-      const float x = nq.x - T.c[0], y = nq.y - T.c[1], z = nq.z - T.c[2];
-      sj[0][lane] = x;
-      sj[1][lane] = y;
-      sj[2][lane] = z;
-      sj[3][lane] = -fmaf(z, z, fmaf(y, y, x * x));
-      sj[4][lane] = na.x;
-      sj[5][lane] = na.y;
-      sj[6][lane] = na.z;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const PairDesc &P = op.pd[p];
+    const int pt = P.pt_off, npad = P.Npad;
+    const int row0 = tile * kTile;
+    const bool two = row0 + kTile < npad;  // uniform over the cluster
+    const int blk0 = pt / kSub, nblk = npad / kSub;
+    // pairs with a grid come here when it cannot hold the step; their blocks have no
+    // statistics and every block is evaluated
+    const bool cull = !ga.slot || ga.slot[p] < 0;
+    float4 q[4];
+    bool live[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int row = (r < 2 || two) ? row0 + 32 * r + lane : row0 + lane;
+      live[r] = row < P.N;
+      q[r] = __ldcg(&op.qs_t[pt + row]);
     }
-    __syncwarp();
-    s = next();
-    if (s < nblk) fetch(s);
-    float2 acc[4][NA];
+    const GaussTile T = gauss_tile(q, live);
+    float S_I = 0.0f;
+    for (int b = 0; b < (two ? 4 : 2); ++b) S_I += __ldcg(&gs.wa[blk0 + row0 / kSub + b].x);
+    const float thr = T.diag2 - lg2_finite(S_I) + kCullBits + lg2f_approx((float)nblk);
+    float2 q2[4][3];  // compact: (2 x', 2 x'); else (x, x)
+    double b2[4];     // |x'|^2
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float x = q[r].x - T.c[0], y = q[r].y - T.c[1], z = q[r].z - T.c[2];
+      b2[r] = (double)x * x + (double)y * y + (double)z * z;
+      const float f = T.compact ? 2.0f : 1.0f;
+      q2[r][0] = make_float2(f * x, f * x);
+      q2[r][1] = make_float2(f * y, f * y);
+      q2[r][2] = make_float2(f * z, f * z);
+    }
+    float hi[4][NA], lo[4][NA];
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int a = 0; a < NA; ++a) acc[r][a] = make_float2(0.0f, 0.0f);
-    if (T.compact) {
+      for (int a = 0; a < NA; ++a) hi[r][a] = lo[r][a] = 0.0f;
+
+    const int nw = S * W, gw = rank * W + warp;
+    int base = gw - 32 * nw;
+    unsigned mask = 0u;
+    auto next = [&]() {  // warp-uniform: the next block to evaluate, or nblk
+      while (mask == 0u) {
+        base += 32 * nw;
+        if (base >= nblk) return nblk;
+        const int sb = base + lane * nw;
+        bool keep = sb < nblk;
+        if (keep && cull) {
+          const float4 l = __ldcg(&gs.box[2 * (blk0 + sb)]);
+          const float4 h = __ldcg(&gs.box[2 * (blk0 + sb) + 1]);
+          const float w = __ldcg(&gs.wa[blk0 + sb].x);
+          keep = !(gauss_gap2(T, l, h) >= lg2f_approx(w) + thr);
+        }
+        mask = __ballot_sync(0xffffffffu, keep);
+      }
+      const int k = __ffs(mask) - 1;
+      mask &= mask - 1u;
+      return base + k * nw;
+    };
+    float4 nq, na;
+    auto fetch = [&](int s) {
+      nq = __ldcg(&op.qs_t[pt + s * kSub + lane]);
+      na = __ldcg(&op.as_t[pt + s * kSub + lane]);
+    };
+    float(*sj)[kSub] = s_j[warp];
+    int s = next();
+    if (s < nblk) fetch(s);
+    while (s < nblk) {
+      __syncwarp();
+      {
+        const float x = nq.x - T.c[0], y = nq.y - T.c[1], z = nq.z - T.c[2];
+        sj[0][lane] = x;
+        sj[1][lane] = y;
+        sj[2][lane] = z;
+        sj[3][lane] = -fmaf(z, z, fmaf(y, y, x * x));
+        sj[4][lane] = na.x;
+        sj[5][lane] = na.y;
+        sj[6][lane] = na.z;
+      }
+      __syncwarp();
+      s = next();
+      if (s < nblk) fetch(s);
+      float2 acc[4][NA];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int a = 0; a < NA; ++a) acc[r][a] = make_float2(0.0f, 0.0f);
+      if (T.compact) {
 #pragma unroll 2
-      for (int jj = 0; jj < kSub; jj += 4) {
-        float4 v[7];
+        for (int jj = 0; jj < kSub; jj += 4) {
+          float4 v[7];
 #pragma unroll
-        for (int k = 0; k < 7; ++k) v[k] = *reinterpret_cast<const float4 *>(&sj[k][jj]);
+          for (int k = 0; k < 7; ++k) v[k] = *reinterpret_cast<const float4 *>(&sj[k][jj]);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+          for (int h = 0; h < 2; ++h) {
+            float2 w[7];
+#pragma unroll
+            for (int k = 0; k < 7; ++k)
+              w[k] = h ? make_float2(v[k].z, v[k].w) : make_float2(v[k].x, v[k].y);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              float2 e = __ffma2_rn(q2[r][0], w[0], w[3]);
+              e = __ffma2_rn(q2[r][1], w[1], e);
+              e = __ffma2_rn(q2[r][2], w[2], e);
+              const float2 K = make_float2(ex2f(e.x), ex2f(e.y));
+#pragma unroll
+              for (int a = 0; a < NA; ++a) acc[r][a] = __ffma2_rn(K, w[4 + a], acc[r][a]);
+            }
+          }
+        }
+      } else {
+#pragma unroll 2
+        for (int jj = 0; jj < kSub; jj += 2) {
           float2 w[7];
 #pragma unroll
-          for (int k = 0; k < 7; ++k)
-            w[k] = h ? make_float2(v[k].z, v[k].w) : make_float2(v[k].x, v[k].y);
+          for (int k = 0; k < 7; ++k) w[k] = *reinterpret_cast<const float2 *>(&sj[k][jj]);
+          const float2 m1 = make_float2(-1.0f, -1.0f);
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
-            float2 e = __ffma2_rn(q2[r][0], w[0], w[3]);
-            e = __ffma2_rn(q2[r][1], w[1], e);
-            e = __ffma2_rn(q2[r][2], w[2], e);
-            const float2 K = make_float2(ex2f(e.x), ex2f(e.y));
+            const float2 dx = __ffma2_rn(w[0], m1, q2[r][0]), dy = __ffma2_rn(w[1], m1, q2[r][1]),
+                         dz = __ffma2_rn(w[2], m1, q2[r][2]);
+            float2 r2 = __fmul2_rn(dx, dx);
+            r2 = __ffma2_rn(dy, dy, r2);
+            r2 = __ffma2_rn(dz, dz, r2);
+            const float2 K = make_float2(ex2f(-r2.x), ex2f(-r2.y));
 #pragma unroll
             for (int a = 0; a < NA; ++a) acc[r][a] = __ffma2_rn(K, w[4 + a], acc[r][a]);
           }
         }
       }
-    } else {
-#pragma unroll 2
-      for (int jj = 0; jj < kSub; jj += 2) {
-        float2 w[7];
 #pragma unroll
-        for (int k = 0; k < 7; ++k) w[k] = *reinterpret_cast<const float2 *>(&sj[k][jj]);
-        const float2 m1 = make_float2(-1.0f, -1.0f);
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const float2 dx = __ffma2_rn(w[0], m1, q2[r][0]), dy = __ffma2_rn(w[1], m1, q2[r][1]),
-                       dz = __ffma2_rn(w[2], m1, q2[r][2]);
-          float2 r2 = __fmul2_rn(dx, dx);
-          r2 = __ffma2_rn(dy, dy, r2);
-          r2 = __ffma2_rn(dz, dz, r2);
-          const float2 K = make_float2(ex2f(-r2.x), ex2f(-r2.y));
-#pragma unroll
-          for (int a = 0; a < NA; ++a) acc[r][a] = __ffma2_rn(K, w[4 + a], acc[r][a]);
-        }
-      }
+        for (int a = 0; a < NA; ++a) two_sum_acc(hi[r][a], lo[r][a], acc[r][a].x + acc[r][a].y);
     }
+    double v[4][NA];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 4; ++r) {
+      const double f = T.compact ? exp2(-b2[r]) : 1.0;
 #pragma unroll
-      for (int a = 0; a < NA; ++a) two_sum_acc(hi[r][a], lo[r][a], acc[r][a].x + acc[r][a].y);
-  }
-  double v[4][NA];
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const double f = T.compact ? exp2(-b2[r]) : 1.0;
-#pragma unroll
-    for (int a = 0; a < NA; ++a) v[r][a] = f * ((double)hi[r][a] + (double)lo[r][a]);
-  }
-  __syncthreads();  // the previous unit's reduction is done with the shared arrays
-  finish_split<ShootOp<3, -1>, W, 4>(op, p, tile, item, rank, sp, two, gs, v);
+      for (int a = 0; a < NA; ++a) v[r][a] = f * ((double)hi[r][a] + (double)lo[r][a]);
+    }
+    __syncthreads();  // the previous unit's reduction is done with the shared arrays
+    finish_split<ShootOp<3, -1>, W, 4>(op, p, tile, item, rank, sp, two, gs, v);
   }
 }
 
@@ -502,196 +503,197 @@ __global__ void __launch_bounds__(W * 32)
   pdl_trigger();
   int skip = -1;  // as in the shooting sweep
   for (int unit = blockIdx.x; unit < sp.items * sp.S; unit += gridDim.x) {
-  const int S = sp.S;
-  const int item = unit / S;
-  const int rank = unit - item * S;
-  const int2 it = items[item];
-  const int p = it.x, tile = it.y;
-  if (p == skip) continue;
-  GridDesc gd;
-  if (!op.active(p) || grid_active(ga, p, true, gd)) {
-    if (sp.one) return;
-    skip = p;
-    continue;
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const PairDesc &P = op.pd[p];
-  const int pt = P.pt_off, npad = P.Npad;
-  const int row0 = tile * kTile;
-  const bool two = row0 + kTile < npad;
-  const int nbt = two ? 4 : 2;
-  const int blk0 = pt / kSub, nblk = npad / kSub;
-  const bool cull = !ga.slot || ga.slot[p] < 0;  // as in the shooting sweep
-  float4 q[R];
-  bool live[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int row = (r < 2 || two) ? row0 + 32 * r + lane : row0 + lane;
-    live[r] = row < P.N;
-    q[r] = __ldcg(&op.qs_t[pt + row]);
-  }
-  const GaussTile T = gauss_tile(q, live);
-  // cut-offs: of K u against the tile's sum of |u|, and of s |x_i - x_j| against the same
-  // products of the tile's own points a quarter of its diagonal apart
-  float U_I = 0.0f, R_I = 0.0f, rm = 0.0f, um = 0.0f;
-  for (int b = 0; b < nbt; ++b) {
-    const float4 w = __ldcg(&gs.wu[blk0 + row0 / kSub + b]);
-    const float4 a = __ldcg(&gs.wa[blk0 + row0 / kSub + b]);
-    U_I += w.x;
-    um = fmaxf(um, w.y);
-    R_I += a.x;
-    rm = fmaxf(rm, a.y);
-  }
-  const float mm = um + rm;  // bounds |m| = |u - r|
-  const float bits = T.diag2 + kCullBits + lg2f_approx((float)nblk);
-  const float thr_u = bits - lg2_finite(U_I);
-  const float thr_s = bits + 2.0f - 0.5f * lg2f_approx(T.diag2) - lg2_finite(mm * R_I + rm * U_I);
-  float2 q2[R][3], mi[R][3], ri[R][3];
-  const float qf = T.compact ? 2.0f : 1.0f;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int row = pt + ((r < 2 || two) ? row0 + 32 * r + lane : row0 + lane);
-    const float4 u = __ldcg(&op.us_t[row]), a = __ldcg(&op.as_t[row]);
-    const float x[3] = {qf * (q[r].x - T.c[0]), qf * (q[r].y - T.c[1]), qf * (q[r].z - T.c[2])};
-    const float m[3] = {u.x - a.x, u.y - a.y, u.z - a.z}, rr[3] = {a.x, a.y, a.z};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      q2[r][d] = make_float2(x[d], x[d]);
-      mi[r][d] = make_float2(m[d], m[d]);
-      ri[r][d] = make_float2(rr[d], rr[d]);
+    const int S = sp.S;
+    const int item = unit / S;
+    const int rank = unit - item * S;
+    const int2 it = items[item];
+    const int p = it.x, tile = it.y;
+    if (p == skip) continue;
+    GridDesc gd;
+    if (!op.active(p) || grid_active(ga, p, true, gd)) {
+      if (sp.one) return;
+      skip = p;
+      continue;
     }
-  }
-  float hi[R][NS], lo[R][NS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const PairDesc &P = op.pd[p];
+    const int pt = P.pt_off, npad = P.Npad;
+    const int row0 = tile * kTile;
+    const bool two = row0 + kTile < npad;
+    const int nbt = two ? 4 : 2;
+    const int blk0 = pt / kSub, nblk = npad / kSub;
+    const bool cull = !ga.slot || ga.slot[p] < 0;  // as in the shooting sweep
+    float4 q[R];
+    bool live[R];
 #pragma unroll
-  for (int r = 0; r < R; ++r)
+    for (int r = 0; r < R; ++r) {
+      const int row = (r < 2 || two) ? row0 + 32 * r + lane : row0 + lane;
+      live[r] = row < P.N;
+      q[r] = __ldcg(&op.qs_t[pt + row]);
+    }
+    const GaussTile T = gauss_tile(q, live);
+    // cut-offs: of K u against the tile's sum of |u|, and of s |x_i - x_j| against the same
+    // products of the tile's own points a quarter of its diagonal apart
+    float U_I = 0.0f, R_I = 0.0f, rm = 0.0f, um = 0.0f;
+    for (int b = 0; b < nbt; ++b) {
+      const float4 w = __ldcg(&gs.wu[blk0 + row0 / kSub + b]);
+      const float4 a = __ldcg(&gs.wa[blk0 + row0 / kSub + b]);
+      U_I += w.x;
+      um = fmaxf(um, w.y);
+      R_I += a.x;
+      rm = fmaxf(rm, a.y);
+    }
+    const float mm = um + rm;  // bounds |m| = |u - r|
+    const float bits = T.diag2 + kCullBits + lg2f_approx((float)nblk);
+    const float thr_u = bits - lg2_finite(U_I);
+    const float thr_s = bits + 2.0f - 0.5f * lg2f_approx(T.diag2) - lg2_finite(mm * R_I + rm * U_I);
+    float2 q2[R][3], mi[R][3], ri[R][3];
+    const float qf = T.compact ? 2.0f : 1.0f;
 #pragma unroll
-    for (int a = 0; a < NS; ++a) hi[r][a] = lo[r][a] = 0.0f;
-  const int nw = S * W, gw = rank * W + warp;
-  int base = gw - 32 * nw;
-  unsigned mask = 0u;
-  auto next = [&]() {
-    while (mask == 0u) {
-      base += 32 * nw;
-      if (base >= nblk) return nblk;
-      const int sb = base + lane * nw;
-      bool keep = sb < nblk;
-      if (keep && cull) {
-        const int b = blk0 + sb;
-        const float4 l = __ldcg(&gs.box[2 * b]), h = __ldcg(&gs.box[2 * b + 1]);
-        const float4 w = __ldcg(&gs.wu[b]), a = __ldcg(&gs.wa[b]);
-        const float g2 = gauss_gap2(T, l, h);
-        keep = !(g2 >= 1.0f && g2 >= lg2f_approx(w.x) + thr_u &&
-                 g2 - 0.5f * lg2f_approx(g2) >= lg2f_approx(mm * a.x + rm * w.x) + thr_s);
+    for (int r = 0; r < R; ++r) {
+      const int row = pt + ((r < 2 || two) ? row0 + 32 * r + lane : row0 + lane);
+      const float4 u = __ldcg(&op.us_t[row]), a = __ldcg(&op.as_t[row]);
+      const float x[3] = {qf * (q[r].x - T.c[0]), qf * (q[r].y - T.c[1]), qf * (q[r].z - T.c[2])};
+      const float m[3] = {u.x - a.x, u.y - a.y, u.z - a.z}, rr[3] = {a.x, a.y, a.z};
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        q2[r][d] = make_float2(x[d], x[d]);
+        mi[r][d] = make_float2(m[d], m[d]);
+        ri[r][d] = make_float2(rr[d], rr[d]);
       }
-      mask = __ballot_sync(0xffffffffu, keep);
     }
-    const int k = __ffs(mask) - 1;
-    mask &= mask - 1u;
-    return base + k * nw;
-  };
-  float4 nq, nu, na;
-  auto fetch = [&](int s) {
-    nq = __ldcg(&op.qs_t[pt + s * kSub + lane]);
-    nu = __ldcg(&op.us_t[pt + s * kSub + lane]);
-    na = __ldcg(&op.as_t[pt + s * kSub + lane]);
-  };
-  float(*sj)[kSub] = s_j[warp];
-  int s = next();
-  if (s < nblk) fetch(s);
-  while (s < nblk) {
-    __syncwarp();
-    {
-      const float x = nq.x - T.c[0], y = nq.y - T.c[1], z = nq.z - T.c[2];
-      const float v[NJ] = {x, y, z, -fmaf(z, z, fmaf(y, y, x * x)), nu.x, nu.y, nu.z, na.x, na.y, na.z};
-#pragma unroll
-      for (int k = 0; k < NJ; ++k) sj[k][lane] = v[k];
-    }
-    __syncwarp();
-    s = next();
-    if (s < nblk) fetch(s);
-    float2 acc[R][NS];
+    float hi[R][NS], lo[R][NS];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int a = 0; a < NS; ++a) acc[r][a] = make_float2(0.0f, 0.0f);
-    auto rest = [&](int r, const float2 (&w)[NJ], const float2 &K, const float2 (&x)[3]) {
-      float2 lr = __fmul2_rn(mi[r][0], w[7]);
-#pragma unroll
-      for (int d = 1; d < 3; ++d) lr = __ffma2_rn(mi[r][d], w[7 + d], lr);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) lr = __ffma2_rn(ri[r][d], w[4 + d], lr);
-      lr = __fmul2_rn(lr, K);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        acc[r][d] = __ffma2_rn(K, w[4 + d], acc[r][d]);
-        acc[r][3 + d] = __ffma2_rn(lr, x[d], acc[r][3 + d]);
+      for (int a = 0; a < NS; ++a) hi[r][a] = lo[r][a] = 0.0f;
+    const int nw = S * W, gw = rank * W + warp;
+    int base = gw - 32 * nw;
+    unsigned mask = 0u;
+    auto next = [&]() {
+      while (mask == 0u) {
+        base += 32 * nw;
+        if (base >= nblk) return nblk;
+        const int sb = base + lane * nw;
+        bool keep = sb < nblk;
+        if (keep && cull) {
+          const int b = blk0 + sb;
+          const float4 l = __ldcg(&gs.box[2 * b]), h = __ldcg(&gs.box[2 * b + 1]);
+          const float4 w = __ldcg(&gs.wu[b]), a = __ldcg(&gs.wa[b]);
+          const float g2 = gauss_gap2(T, l, h);
+          keep = !(g2 >= 1.0f && g2 >= lg2f_approx(w.x) + thr_u &&
+                   g2 - 0.5f * lg2f_approx(g2) >= lg2f_approx(mm * a.x + rm * w.x) + thr_s);
+        }
+        mask = __ballot_sync(0xffffffffu, keep);
       }
-      acc[r][6] = __fadd2_rn(acc[r][6], lr);
+      const int k = __ffs(mask) - 1;
+      mask &= mask - 1u;
+      return base + k * nw;
     };
-    if (T.compact) {
+    float4 nq, nu, na;
+    auto fetch = [&](int s) {
+      nq = __ldcg(&op.qs_t[pt + s * kSub + lane]);
+      nu = __ldcg(&op.us_t[pt + s * kSub + lane]);
+      na = __ldcg(&op.as_t[pt + s * kSub + lane]);
+    };
+    float(*sj)[kSub] = s_j[warp];
+    int s = next();
+    if (s < nblk) fetch(s);
+    while (s < nblk) {
+      __syncwarp();
+      {
+        const float x = nq.x - T.c[0], y = nq.y - T.c[1], z = nq.z - T.c[2];
+        const float v[NJ] = {x,    y,    z,    -fmaf(z, z, fmaf(y, y, x * x)), nu.x, nu.y,
+                             nu.z, na.x, na.y, na.z};
+#pragma unroll
+        for (int k = 0; k < NJ; ++k) sj[k][lane] = v[k];
+      }
+      __syncwarp();
+      s = next();
+      if (s < nblk) fetch(s);
+      float2 acc[R][NS];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int a = 0; a < NS; ++a) acc[r][a] = make_float2(0.0f, 0.0f);
+      auto rest = [&](int r, const float2 (&w)[NJ], const float2 &K, const float2 (&x)[3]) {
+        float2 lr = __fmul2_rn(mi[r][0], w[7]);
+#pragma unroll
+        for (int d = 1; d < 3; ++d) lr = __ffma2_rn(mi[r][d], w[7 + d], lr);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) lr = __ffma2_rn(ri[r][d], w[4 + d], lr);
+        lr = __fmul2_rn(lr, K);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          acc[r][d] = __ffma2_rn(K, w[4 + d], acc[r][d]);
+          acc[r][3 + d] = __ffma2_rn(lr, x[d], acc[r][3 + d]);
+        }
+        acc[r][6] = __fadd2_rn(acc[r][6], lr);
+      };
+      if (T.compact) {
 #pragma unroll 2
-      for (int jj = 0; jj < kSub; jj += 4) {
-        float4 v[NJ];
+        for (int jj = 0; jj < kSub; jj += 4) {
+          float4 v[NJ];
 #pragma unroll
-        for (int k = 0; k < NJ; ++k) v[k] = *reinterpret_cast<const float4 *>(&sj[k][jj]);
+          for (int k = 0; k < NJ; ++k) v[k] = *reinterpret_cast<const float4 *>(&sj[k][jj]);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+          for (int h = 0; h < 2; ++h) {
+            float2 w[NJ];
+#pragma unroll
+            for (int k = 0; k < NJ; ++k)
+              w[k] = h ? make_float2(v[k].z, v[k].w) : make_float2(v[k].x, v[k].y);
+            const float2 x[3] = {w[0], w[1], w[2]};
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              float2 e = __ffma2_rn(q2[r][0], w[0], w[3]);
+              e = __ffma2_rn(q2[r][1], w[1], e);
+              e = __ffma2_rn(q2[r][2], w[2], e);
+              rest(r, w, make_float2(ex2f(e.x), ex2f(e.y)), x);
+            }
+          }
+        }
+      } else {
+#pragma unroll 2
+        for (int jj = 0; jj < kSub; jj += 2) {
           float2 w[NJ];
 #pragma unroll
-          for (int k = 0; k < NJ; ++k)
-            w[k] = h ? make_float2(v[k].z, v[k].w) : make_float2(v[k].x, v[k].y);
-          const float2 x[3] = {w[0], w[1], w[2]};
+          for (int k = 0; k < NJ; ++k) w[k] = *reinterpret_cast<const float2 *>(&sj[k][jj]);
+          const float2 m1 = make_float2(-1.0f, -1.0f);
 #pragma unroll
           for (int r = 0; r < R; ++r) {
-            float2 e = __ffma2_rn(q2[r][0], w[0], w[3]);
-            e = __ffma2_rn(q2[r][1], w[1], e);
-            e = __ffma2_rn(q2[r][2], w[2], e);
-            rest(r, w, make_float2(ex2f(e.x), ex2f(e.y)), x);
+            float2 x[3];  // x_j - x_i: the s x' sums are then the negated result
+#pragma unroll
+            for (int d = 0; d < 3; ++d) x[d] = __ffma2_rn(q2[r][d], m1, w[d]);
+            float2 r2 = __fmul2_rn(x[0], x[0]);
+            r2 = __ffma2_rn(x[1], x[1], r2);
+            r2 = __ffma2_rn(x[2], x[2], r2);
+            rest(r, w, make_float2(ex2f(-r2.x), ex2f(-r2.y)), x);
           }
         }
       }
-    } else {
-#pragma unroll 2
-      for (int jj = 0; jj < kSub; jj += 2) {
-        float2 w[NJ];
 #pragma unroll
-        for (int k = 0; k < NJ; ++k) w[k] = *reinterpret_cast<const float2 *>(&sj[k][jj]);
-        const float2 m1 = make_float2(-1.0f, -1.0f);
+      for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          float2 x[3];  // x_j - x_i: the s x' sums are then the negated result
+        for (int a = 0; a < NS; ++a) two_sum_acc(hi[r][a], lo[r][a], acc[r][a].x + acc[r][a].y);
+    }
+    double v[R][6];
 #pragma unroll
-          for (int d = 0; d < 3; ++d) x[d] = __ffma2_rn(q2[r][d], m1, w[d]);
-          float2 r2 = __fmul2_rn(x[0], x[0]);
-          r2 = __ffma2_rn(x[1], x[1], r2);
-          r2 = __ffma2_rn(x[2], x[2], r2);
-          rest(r, w, make_float2(ex2f(-r2.x), ex2f(-r2.y)), x);
-        }
+    for (int r = 0; r < R; ++r) {
+      double f = 1.0, x[3] = {0.0, 0.0, 0.0};
+      if (T.compact) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x[d] = 0.5 * (double)q2[r][d].x;
+        f = exp2(-(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]));
+      }
+      const double ss = (double)hi[r][6] + (double)lo[r][6];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        v[r][d] = f * ((double)hi[r][d] + (double)lo[r][d]);
+        v[r][3 + d] = f * (x[d] * ss - ((double)hi[r][3 + d] + (double)lo[r][3 + d]));
       }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int a = 0; a < NS; ++a) two_sum_acc(hi[r][a], lo[r][a], acc[r][a].x + acc[r][a].y);
-  }
-  double v[R][6];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    double f = 1.0, x[3] = {0.0, 0.0, 0.0};
-    if (T.compact) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) x[d] = 0.5 * (double)q2[r][d].x;
-      f = exp2(-(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]));
-    }
-    const double ss = (double)hi[r][6] + (double)lo[r][6];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      v[r][d] = f * ((double)hi[r][d] + (double)lo[r][d]);
-      v[r][3 + d] = f * (x[d] * ss - ((double)hi[r][3 + d] + (double)lo[r][3 + d]));
-    }
-  }
-  __syncthreads();
-  finish_split<Op, W, R>(op, p, tile, item, rank, sp, two, gs, v);
+    __syncthreads();
+    finish_split<Op, W, R>(op, p, tile, item, rank, sp, two, gs, v);
   }
 }
 

@@ -137,7 +137,8 @@ struct DefKernel {
 //           (k! (k+1)!), four polynomials by Horner's rule;
 //   x > 2   sqrt(x) e^x K_nu(x) as a polynomial of degree 8 in t = 2 / x on (0, 1]: Chebyshev
 //           interpolation of K0 and K1 in double precision, within 2.1e-9.
-// Relative error against double-precision K0 / K1 stays below 1e-6 over x in [1e-8, 90].
+// In FP32 the relative error against double-precision K0 / K1 is below 3e-7 rms (3e-6 at most,
+// K0 near x = 2) up to x = 10 and 7e-7 rms beyond, where the exponential's argument rounds.
 // Bound by FMA issue (18 and 28 per point); a trapezoid rule with 14 exponentials for 2 < x
 // <= 10 and an asymptotic series beyond took 7.55 instead of 6.73 us per shooting step of 500
 // points and 8.54 instead of 7.43 per adjoint step.

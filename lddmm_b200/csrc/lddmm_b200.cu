@@ -715,9 +715,10 @@ static cudaError_t varifold_impl(lddmm_ctx &c) {
     return launch(vfd_split_kernel<kWarps>, (unsigned)(c.n_el_items * c.S_vfd), kWarps * 32, 0,
                   c.stream, op, (const int2 *)c.el_items,
                   SplitPlan{c.S_vfd, c.n_el_items, c.P == 1, c.vpart, c.vcnt});
-  return launch(sweep_packed_kernel<VarifoldOp<D, CT, DT>, kWarps>,
-                (unsigned)(c.n_el_items * c.S_vfd), kWarps * 32, c.S_vfd, c.stream, op,
-                (const int2 *)c.el_items, c.S_vfd);
+  else
+    return launch(sweep_packed_kernel<VarifoldOp<D, CT, DT>, kWarps>,
+                  (unsigned)(c.n_el_items * c.S_vfd), kWarps * 32, c.S_vfd, c.stream, op,
+                  (const int2 *)c.el_items, c.S_vfd);
 }
 
 template <int D, char CT, char DT>
@@ -766,8 +767,14 @@ static int vfd_clusters_impl(int S) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int n = 0;
-  const cudaError_t e =
-      cudaOccupancyMaxActiveClusters(&n, sweep_packed_kernel<VarifoldOp<D, CT, DT>, kWarps>, &cfg);
+  cudaError_t e;
+  if constexpr (D == 3 && CT == 'G' && DT == 'B') {  // S independent CTAs
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vfd_split_kernel<kWarps>, kWarps * 32, 0);
+    n = n * 148 / S;
+  } else {
+    e = cudaOccupancyMaxActiveClusters(&n, sweep_packed_kernel<VarifoldOp<D, CT, DT>, kWarps>,
+                                       &cfg);
+  }
   cudaGetLastError();
   return e == cudaSuccess ? n : 0;
 }
