@@ -554,8 +554,7 @@ cudaError_t launch_gemm(GemmArgs a, int splits, cudaStream_t st) {
                                (int)gemm_resident_smem_bytes(256, kResK));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(gemm_bf16_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)std::max(gemm_ws_smem_bytes(256, kResK, true),
-                                             gemm_ws_smem_bytes(256, kResK, false)));
+                               (int)gemm_ws_smem_bytes(256, kResK));
     if (e != cudaSuccess) return e;
     attr_set[dev].store(true);
   }
@@ -572,8 +571,8 @@ cudaError_t launch_gemm(GemmArgs a, int splits, cudaStream_t st) {
       // a plain FP32 output leaves through TMA stores
       const bool tma_store = a.out && a.epi == kEpiNone && !a.pre_out && !a.out_bf &&
                              !a.out_bt && make_out_map(&mc, a.out, a.n_valid, a.M, a.ldo);
-      gemm_bf16_ws_kernel<<<grid, kWsThreads, gemm_ws_smem_bytes(a.N, a.K, tma_store), st>>>(
-          a, ma, mb, mc, tma_store ? 1 : 0, gemm_ws_stages(a.N, a.K, tma_store));
+      gemm_bf16_ws_kernel<<<grid, kWsThreads, gemm_ws_smem_bytes(a.N, a.K), st>>>(
+          a, ma, mb, mc, tma_store ? 1 : 0, gemm_ws_stages(a.N, a.K));
     } else
       gemm_bf16_resident_kernel<<<grid, kGemmThreads, gemm_resident_smem_bytes(a.N, a.K), st>>>(a);
   } else {
