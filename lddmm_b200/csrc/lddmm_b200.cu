@@ -1668,8 +1668,9 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
       }
       if (cf.persistent == 0) {
         // the small form: one cluster per pair of at most 512 points, beyond which a CTA's
-        // rows no longer fit its threads (at 500 points it ties with the L2 form, at 200 it
-        // takes three quarters of the time); no more CTAs than the smallest pair has 16-row
+        // rows no longer fit its threads (at 200 points a step takes three quarters of the
+        // L2 form's; costly 2D Matern pairs at 500 are faster there, section "small form"
+        // of persist.cuh); no more CTAs than the smallest pair has 16-row
         // groups (a CTA's energy partial takes one's place).  Autotuning times all forms
         int np = 0, ng = kSmallCtas;
         for (const PairDesc &d : c.hpd) {

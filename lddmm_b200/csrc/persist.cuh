@@ -665,9 +665,10 @@ __global__ void __launch_bounds__(kPersistWarps * 32, 2)
 // by definition and every CTA of it reaches every barrier.
 // Bound by the step's own latency (a chain of shared loads, exponential, shuffles, FP64
 // finalise and cluster barrier); 16 lanes per row is the most that a block of 512 threads
-// gives 512 points in 16 CTAs.  Us per step, L2 form -> this form: 200 points (2D, Gaussian)
-// shooting 3.30 -> 2.42, adjoint 3.66 -> 2.76; 500 points (2D, Matern of order 3) 6.73 ->
-// 6.70 and 7.43 -> 7.47: the two meet at its largest pairs.
+// gives 512 points in 16 CTAs.  200 points (2D, Gaussian), us per step against 16-row groups
+// combined through L2: shooting 3.30 -> 2.42, adjoint 3.66 -> 2.76.  500 points (2D, Matern of
+// order 3) are bound by the Bessel functions instead: an evaluation takes 350 us with this
+// form and 303 on the 64-row tiles, which autotuning then picks.
 
 constexpr int kSmallMax = 512;      // padded points of a pair; threads per CTA
 constexpr int kSmallCtas = 16;      // CTAs per cluster
