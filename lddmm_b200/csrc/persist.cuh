@@ -660,8 +660,9 @@ __global__ void __launch_bounds__(kPersistWarps * 32, 2)
 // finalised row's new operands go straight into every CTA's buffer of the next step
 // (distributed shared memory), and the hardware cluster barrier ends the step: no operand
 // of the recursion passes through L2 between steps, and there is no atomic to poll.
-// Operands that do not depend on the step before (a; q and r in the adjoint) are loaded
-// during the sums.  The cluster barrier waits without a bound, but a cluster is co-resident
+// The row's FP64 state stays in registers, a step's global results are stored after its
+// barrier (whose release would wait for them), and operands that do not depend on the step
+// before (a; q and r in the adjoint) are loaded two steps ahead.  The cluster barrier waits without a bound, but a cluster is co-resident
 // by definition and every CTA of it reaches every barrier.
 // Bound by the step's own latency (a chain of shared loads, exponential, shuffles, FP64
 // finalise and cluster barrier); 16 lanes per row is the most that a block of 512 threads
