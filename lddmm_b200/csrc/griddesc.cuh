@@ -74,10 +74,10 @@ __device__ __forceinline__ bool grid_active(const GridArgs &a, int p, bool adj, 
   return g.ok;
 }
 
-// 2^k with N m 2^k <= 2^61.
+// 2^k with N m 2^k <= 2^61.  In FP64: N m may exceed the largest float.
 __device__ __forceinline__ int grid_scale_exp(int N, unsigned mbits) {
-  const float b = (float)N * __uint_as_float(mbits);
-  return b > 0.0f ? 60 - ilogbf(b) : 0;
+  const double b = (double)N * __uint_as_float(mbits);
+  return b > 0.0 ? 60 - ilogb(b) : 0;
 }
 
 }  // namespace lddmm

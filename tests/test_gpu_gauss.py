@@ -105,6 +105,22 @@ def test_gridded_sums_against_fp64(n):
             assert np.max(np.abs(P.time_stp * dq - step)) < 1e-7 * np.max(np.abs(pst[t]))
 
 
+def test_gridded_sums_of_huge_momenta():
+    """Finite momenta whose largest value times N exceeds the largest float: the first step
+    still runs on the grid (later ones outgrow it).  Tolerance as above."""
+    from lddmm_b200 import api
+
+    P = _grid_problem(40000, 0.3, 5)
+    a = np.random.default_rng(3).normal(size=(P.T, 40000, 3)) * 1e34
+    assert a.max() < 3e38 < 40000 * a.max()
+    with api.Context(P) as ctx:
+        (q, v), = ctx.shoot(a.reshape(-1))
+    rows = np.random.default_rng(4).integers(0, 40000, 40)
+    d2 = ((q[0][rows][:, None] - q[0][None]) ** 2).sum(-1)
+    vo = np.exp(-d2 / P.knl_width ** 2) @ a[0]
+    assert np.max(np.abs(v[0][rows] - vo)) < 1e-7 * np.max(np.abs(vo))
+
+
 @pytest.mark.parametrize("n,cw", [(40, 0.1), (66, 0.5), (1500, 1.0), (1500, 0.3), (1500, 0.1),
                                   (1500, 0.02)])
 def test_split_varifold_sweep_against_the_oracle(oracle, n, cw):
