@@ -284,7 +284,8 @@ inline void def_kernel_scales(int order, int dim, double width, float *kscale,
 //        dk/dc_i = -2 k / sigma^2 dc  ->  gradient weight k
 //   'C'  k = 1 / (1 + |dc|^2/sigma^2),         cscale = 1/sigma,
 //        dk/dc_i = -2 k^2 / sigma^2 dc  ->  gradient weight k^2
-// Both share dc_fac = -2 / (sigma^2 cscale) on the host.
+// Both share dc_fac = -2 / (sigma^2 cscale) on the host.  cscale is rounded to FP32 except
+// with `exact` (vfd.cuh, where that rounding would be the largest systematic error).
 template <char CT>
 struct CenKernel {
   static __device__ __forceinline__ void val_w(float nr2, float &k, float &kw) {
@@ -298,10 +299,11 @@ struct CenKernel {
   }
 };
 
-inline void cen_kernel_scales(char type, double width, float *cscale, double *dc_fac) {
+inline void cen_kernel_scales(char type, double width, bool exact, double *cscale,
+                              double *dc_fac) {
   const double log2e = 1.4426950408889634;
   const double s = (type == 'G') ? std::sqrt(log2e) / width : 1.0 / width;
-  *cscale = (float)s;
+  *cscale = exact ? s : (double)(float)s;
   *dc_fac = -2.0 / (width * width * s);
 }
 

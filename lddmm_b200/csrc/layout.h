@@ -35,12 +35,12 @@ struct PairDesc {
   long long var_off;  // first FP64 variable
   long long var_num;  // D * N * T
   float kscale;       // coordinate scale of the deformation kernel (ex2 argument)
-  float cscale;       // centre scale of the varifold centre kernel
   double dt;          // time step
   double dis_wgt;     // varifold weight
   double pd_fac;      // dq factor: pdot = pd_fac * sum(lr * W * dq_scaled)
   double dc_fac;      // varifold dc factor (without the 2 a_i): -2 / (sigma_W^2 * cscale)
   double tt;          // target self-term, FP64, computed once
+  double cscale;      // centre scale of the varifold centre kernel
   double kscale64;    // coordinate scale of the Gaussian deformation kernel in FP64 (grid.cuh)
 };
 

@@ -1255,7 +1255,9 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
     P.dis_wgt = a.dis_wgt;
     def_kernel_scales(a.knl_order, a.dim, a.knl_width, &P.kscale, &P.pd_fac);
     P.kscale64 = a.knl_order == -1 ? std::sqrt(1.4426950408889634) / a.knl_width : P.kscale;
-    if (c.has_vfd) cen_kernel_scales(a.cen_knl_type, a.cen_knl_width, &P.cscale, &P.dc_fac);
+    if (c.has_vfd)
+      cen_kernel_scales(a.cen_knl_type, a.cen_knl_width, c.D == 3 && c.ct == 'G' && c.dt == 'B',
+                        &P.cscale, &P.dc_fac);
     pt += P.Npad;
     el += P.Edpad;
     tg += P.Etpad;

@@ -4,7 +4,7 @@
 // distance test, items split over independent CTAs.
 //
 // With x' a scaled centre minus the tile's centre, k = 2^-|x_i - x_j|^2 =
-// 2^(2 x_i'.x_j' - |x_j'|^2) 2^-|x_i'|^2, and the sums of VarifoldOp (ops.cuh) are
+// 2^(2 x_i'.x_j' - |x_j'|^2 - 1) 2^(1 - |x_i'|^2), and the sums of VarifoldOp (ops.cuh) are
 //   S = sum k w ang^2,  A = sum k w ang n_j,
 //   C = sum k w ang^2 (x_i - x_j) = x_i' (S_DD + S_DT) - sum k w ang^2 x_j':
 // 16 packed instructions per two pairs instead of 25, 8 staged values per column instead
@@ -16,6 +16,16 @@
 // wider than kVfdCompactR2 are evaluated from differences of x' (19 instructions), those
 // wider than kVfdNearR2 (elements in no spatial order) from the double-single differences
 // (25).
+//
+// Systematic errors.  The value V = DD - 2 DT + TT keeps a common relative error of DD and
+// DT whole, since TT is formed in FP64, and near convergence V is small against TT.  ex2.approx
+// is low by 5.0e-8 on average over [-1, 0) and high by 3.3e-8 over [0, 1) (measured on 2^20
+// arguments, the same in every unit interval; exact at 0).  The compact tiles' arguments are
+// therefore kept negative by a factor 2^-1 that the row undoes, and the FP64 sums are raised by
+// the error that is left, the mean of ex2's over the kernel's pairs on a surface: 4.6e-8 there,
+// 3.7e-8 for arguments -r^2 (the error is smaller near r = 0).  The centre scale is not rounded
+// to FP32: its 2.5e-8 widened the kernel and had hidden part of this.  |V - V64| / TT of 20,000 landmarks, centre width 0.2: 1.4e-8 with
+// neither (0.9e-8 with double-single differences throughout), 0.12e-8 now.
 //
 // A block is skipped when 2^-gap^2 times its area is at most 2^-32 / nblk of 2^-diag^2
 // times the tile's own area (all skipped blocks: 2^-32 of what the tile's own elements
@@ -30,6 +40,8 @@ namespace lddmm {
 constexpr float kVfdCompactR2 = 1.0f;  // squared half diagonal of a compact row tile
 constexpr float kVfdNearR2 = 16.0f;    // of one evaluated from centred differences
 constexpr float kVfdCullBits = 32.0f;
+constexpr double kEx2Low = 4.6e-8;     // ex2's mean error, compact tiles (see above)
+constexpr double kEx2LowR2 = 3.7e-8;   // the others
 
 template <int W>
 __global__ void __launch_bounds__(W * 32, 4)
@@ -37,7 +49,7 @@ __global__ void __launch_bounds__(W * 32, 4)
                      const SplitPlan sp) {
   using Op = VarifoldOp<3, 'G', 'B'>;
   constexpr int R = 2, NS = 8;  // S_DD, S_DT, A, sum tb x'
-  constexpr int NJ = 11;        // x', -|x'|^2, n, w; wide tiles: centre hi, lo
+  constexpr int NJ = 11;        // x', -|x'|^2 - 1, n, w; wide tiles: centre hi, lo
   __shared__ __align__(16) float s_j[W][NJ][kSub];
   const int S = sp.S;
   const int item = blockIdx.x / S;
@@ -130,7 +142,7 @@ __global__ void __launch_bounds__(W * 32, 4)
     __syncwarp();
     {
       const float x = (nc.x - c[0]) + nl.x, y = (nc.y - c[1]) + nl.y, z = (nc.z - c[2]) + nl.z;
-      sj[3][lane] = -fmaf(z, z, fmaf(y, y, x * x));
+      sj[3][lane] = -1.0f - fmaf(z, z, fmaf(y, y, x * x));
       sj[4][lane] = nn.x;
       sj[5][lane] = nn.y;
       sj[6][lane] = nn.z;
@@ -238,10 +250,11 @@ __global__ void __launch_bounds__(W * 32, 4)
   double v[R][NS];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const double f = compact ? exp2(-(xi[r][0] * xi[r][0] + xi[r][1] * xi[r][1] +
-                                      xi[r][2] * xi[r][2])) : 1.0;
+    const double f = compact ? exp2(1.0 - (xi[r][0] * xi[r][0] + xi[r][1] * xi[r][1] +
+                                           xi[r][2] * xi[r][2])) : 1.0;
+    const double low = compact ? kEx2Low : kEx2LowR2;
 #pragma unroll
-    for (int a = 0; a < NS; ++a) v[r][a] = f * ((double)hi[r][a] + (double)lo[r][a]);
+    for (int a = 0; a < NS; ++a) v[r][a] = (1.0 + low) * f * ((double)hi[r][a] + (double)lo[r][a]);
     const double t = compact ? v[r][0] + v[r][1] : 0.0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) v[r][5 + d] = xi[r][d] * t - v[r][5 + d];
@@ -251,7 +264,7 @@ __global__ void __launch_bounds__(W * 32, 4)
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int d = 0; d < 3; ++d)  // xi may be infinite or meaningless here
-        v[r][5 + d] = -((double)hi[r][5 + d] + (double)lo[r][5 + d]);
+        v[r][5 + d] = -(1.0 + kEx2LowR2) * ((double)hi[r][5 + d] + (double)lo[r][5 + d]);
   }
   finish_split<Op, W, R>(op, p, tile, item, rank, sp, false, GaussStats{}, v);
 }

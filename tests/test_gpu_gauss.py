@@ -135,3 +135,32 @@ def test_split_varifold_sweep_against_the_oracle(oracle, n, cw):
     vo, go = oracle.varifold(P, P.ini_nde)
     assert abs(v - vo) <= TOL * abs(vo)
     assert rel(dq, go) < TOL
+
+
+@pytest.mark.parametrize("cw", [0.4, 0.15, 0.05])
+def test_split_varifold_value_near_convergence(cw):
+    """Compact, near and wide element tiles: V between two meshes of one surface, small
+    against TT, so that its error is the systematic one of DD and DT.  Of the exponential's
+    mean error (3.7e-8 and 4.6e-8 over a kernel's pairs, removed) its variation with the
+    distribution of the arguments remains, some 0.5e-8; rounding errors average out over
+    3.6e7 pairs.  8e-9 of TT."""
+    import torch
+
+    from lddmm_b200 import api, problem, shapes
+
+    v, f = shapes.decimated_star(3000, 6, 0.05, 23)
+    tv, tf = shapes.decimated_star(3100, 6, 0.05, 23)
+    P = problem.Problem(v, f, *shapes.varifold_of(tv, tf), knl_order=-1, knl_width=0.3,
+                        time_num=2, time_stp=1.0, cen_width=cw)
+    V, _ = api.varifold(P, P.ini_nde)
+    S, T = ([torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in y]
+            for y in (shapes.varifold_of(v, f), shapes.varifold_of(tv, tf)))
+
+    def dot(x, y):
+        d2 = sum((x[0][:, None, k] - y[0][None, :, k]) ** 2 for k in range(3))
+        return float(x[2] @ (torch.exp(-d2 / cw ** 2) * (x[1] @ y[1].T) ** 2) @ y[2])
+
+    tt = dot(T, T)
+    v64 = dot(S, S) - 2 * dot(S, T) + tt
+    assert v64 < 0.2 * tt
+    assert abs(V - v64) < 8e-9 * tt, (V - v64) / tt
