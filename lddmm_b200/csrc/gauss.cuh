@@ -10,7 +10,7 @@
 // coordinates as long as |x_i'| is about 1; a tile whose points lie further apart
 // (kCompactR2) is evaluated from coordinate differences instead.
 //
-// Distance test.  A 32-column block B is skipped for a row tile I when its whole
+// Distance test (shooting; the adjoint's: cull.h).  A 32-column block B is skipped for a row tile I when its whole
 // contribution is bounded by
 //   2^-gap(I, B)^2 S_B  <=  2^-26 / nblk * 2^-diag(I)^2 S_I,
 // S the sum of the momenta's absolute values over a block's (the tile's) points, gap the
@@ -23,6 +23,7 @@
 // of all of space and S_B = inf: it is never skipped.
 #pragma once
 
+#include "cull.h"
 #include "griddesc.cuh"
 #include "kernels.cuh"
 #include "layout.h"
@@ -34,13 +35,12 @@ namespace lddmm {
 
 constexpr int kGaussRows = 128;         // rows per work item (two 64-row tiles)
 constexpr float kCompactR2 = 3.0f;      // squared half diagonal of a compact row tile
-constexpr float kCullBits = 26.0f;      // see the distance test above
 
 // Block statistics of one time step (32-point blocks of the concatenated points).
 struct GaussStats {
   const float4 *box;  // per block: (lo, -), (hi, -) of the scaled positions
-  const float4 *wa;   // per block: (sum |a|, max |a|, -, -) of alpha_t
-  const float4 *wu;   // adjoint, per block: (sum |u|, max |u|, -, -)
+  const float4 *wa;   // per block: (sum |a|, -, -, -) of alpha_t
+  const float4 *wu;   // adjoint, per block: (sum |u|, -, -, -)
   float4 *box_n;      // shooting: boxes of the next step's positions (written)
   float4 *wu_n;       // adjoint: weights of the next backward step's u (written; or null)
   // contexts with a grid (grid.cuh): the next positions' box keys [pair][6], max |u| of the
@@ -152,10 +152,6 @@ __device__ __forceinline__ float abs_sum(const float4 &a) {
 __device__ __forceinline__ float abs_max(const float4 &a) {
   return fmaxf(fabsf(a.x), fmaxf(fabsf(a.y), fabsf(a.z)));
 }
-// log2 of a tile's weight; -inf (nothing is skipped) when it is not finite.
-__device__ __forceinline__ float lg2_finite(float s) {
-  return lg2f_approx(s < INFINITY ? s : 0.0f);
-}
 // A NaN or infinity anywhere in the block gives S = inf (fmaxf drops NaNs, sums keep them).
 __device__ __forceinline__ float or_inf(float s) { return s < INFINITY ? s : INFINITY; }
 
@@ -172,7 +168,7 @@ __global__ void gauss_alpha_kernel(const float4 *as, long long nblk_tot, int nbl
     const float4 a = __ldcg(&as[b * 32 + lane]);
     const float s = or_inf(warp_sum_f(abs_sum(a))), m = warp_max_f(abs_max(a));
     if (lane == 0) {
-      wa[b] = make_float4(s, m, 0.0f, 0.0f);
+      wa[b] = make_float4(s, 0.0f, 0.0f, 0.0f);
       const int t = (int)(b / nblk), p = pt_pair[(b - (long long)t * nblk) * 32];
       if (mx && p >= 0) atomicMax(&mx[t * P + p], __float_as_uint(s < INFINITY ? m : s));
     }
@@ -211,7 +207,7 @@ __device__ __forceinline__ void gauss_next_stats(const AdjointOp<D, ORDER> &op,
   const float4 u = live ? op.us_n[g] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const float s = or_inf(warp_sum_f(abs_sum(u))), m = warp_max_f(abs_max(u));
   if ((threadIdx.x & 31) == 0) {
-    if (blk >= 0) gs.wu_n[blk] = make_float4(s, m, 0.0f, 0.0f);
+    if (blk >= 0) gs.wu_n[blk] = make_float4(s, 0.0f, 0.0f, 0.0f);
     if (gs.umax_n) atomicMax(&gs.umax_n[p], __float_as_uint(s < INFINITY ? m : s));
   }
 }
@@ -532,21 +528,12 @@ __global__ void __launch_bounds__(W * 32)
       q[r] = __ldcg(&op.qs_t[pt + row]);
     }
     const GaussTile T = gauss_tile(q, live);
-    // cut-offs: of K u against the tile's sum of |u|, and of s |x_i - x_j| against the same
-    // products of the tile's own points a quarter of its diagonal apart
-    float U_I = 0.0f, R_I = 0.0f, rm = 0.0f, um = 0.0f;
+    float U_I = 0.0f, R_I = 0.0f;
     for (int b = 0; b < nbt; ++b) {
-      const float4 w = __ldcg(&gs.wu[blk0 + row0 / kSub + b]);
-      const float4 a = __ldcg(&gs.wa[blk0 + row0 / kSub + b]);
-      U_I += w.x;
-      um = fmaxf(um, w.y);
-      R_I += a.x;
-      rm = fmaxf(rm, a.y);
+      U_I += __ldcg(&gs.wu[blk0 + row0 / kSub + b].x);
+      R_I += __ldcg(&gs.wa[blk0 + row0 / kSub + b].x);
     }
-    const float mm = um + rm;  // bounds |m| = |u - r|
-    const float bits = T.diag2 + kCullBits + lg2f_approx((float)nblk);
-    const float thr_u = bits - lg2_finite(U_I);
-    const float thr_s = bits + 2.0f - 0.5f * lg2f_approx(T.diag2) - lg2_finite(mm * R_I + rm * U_I);
+    const AdjointCut cut = adjoint_cut(T.diag2, nblk, U_I, R_I);
     float2 q2[R][3], mi[R][3], ri[R][3];
     const float qf = T.compact ? 2.0f : 1.0f;
 #pragma unroll
@@ -579,10 +566,8 @@ __global__ void __launch_bounds__(W * 32)
         if (keep && cull) {
           const int b = blk0 + sb;
           const float4 l = __ldcg(&gs.box[2 * b]), h = __ldcg(&gs.box[2 * b + 1]);
-          const float4 w = __ldcg(&gs.wu[b]), a = __ldcg(&gs.wa[b]);
-          const float g2 = gauss_gap2(T, l, h);
-          keep = !(g2 >= 1.0f && g2 >= lg2f_approx(w.x) + thr_u &&
-                   g2 - 0.5f * lg2f_approx(g2) >= lg2f_approx(mm * a.x + rm * w.x) + thr_s);
+          keep = !adjoint_skips(cut, gauss_gap2(T, l, h), __ldcg(&gs.wu[b].x),
+                                __ldcg(&gs.wa[b].x));
         }
         mask = __ballot_sync(0xffffffffu, keep);
       }

@@ -24,8 +24,9 @@
 // therefore kept negative by a factor 2^-1 that the row undoes, and the FP64 sums are raised by
 // the error that is left, the mean of ex2's over the kernel's pairs on a surface: 4.6e-8 there,
 // 3.7e-8 for arguments -r^2 (the error is smaller near r = 0).  The centre scale is not rounded
-// to FP32: its 2.5e-8 widened the kernel and had hidden part of this.  |V - V64| / TT of 20,000 landmarks, centre width 0.2: 1.4e-8 with
-// neither (0.9e-8 with double-single differences throughout), 0.12e-8 now.
+// to FP32: its 2.5e-8 widened the kernel and had hidden part of this.  |V - V64| / TT of 20,000
+// landmarks, centre width 0.2: 1.4e-8 with neither (0.9e-8 with double-single differences
+// throughout), 0.12e-8 now.
 //
 // A block is skipped when 2^-gap^2 times its area is at most 2^-32 / nblk of 2^-diag^2
 // times the tile's own area (all skipped blocks: 2^-32 of what the tile's own elements
