@@ -41,6 +41,7 @@ struct GaussStats {
   const float4 *box;  // per block: (lo, -), (hi, -) of the scaled positions
   const float4 *wa;   // per block: (sum |a|, -, -, -) of alpha_t
   const float4 *wu;   // adjoint, per block: (sum |u|, -, -, -)
+  // (pairs with a grid have them only in the steps that it cannot hold: grid_conv_yz_kernel)
   float4 *box_n;      // shooting: boxes of the next step's positions (written)
   float4 *wu_n;       // adjoint: weights of the next backward step's u (written; or null)
   // contexts with a grid (grid.cuh): the next positions' box keys [pair][6], max |u| of the
@@ -337,9 +338,6 @@ __global__ void __launch_bounds__(W * 32, 4)
     const int row0 = tile * kTile;
     const bool two = row0 + kTile < npad;  // uniform over the cluster
     const int blk0 = pt / kSub, nblk = npad / kSub;
-    // pairs with a grid come here when it cannot hold the step; their blocks have no
-    // statistics and every block is evaluated
-    const bool cull = !ga.slot || ga.slot[p] < 0;
     float4 q[4];
     bool live[4];
 #pragma unroll
@@ -378,7 +376,7 @@ __global__ void __launch_bounds__(W * 32, 4)
         if (base >= nblk) return nblk;
         const int sb = base + lane * nw;
         bool keep = sb < nblk;
-        if (keep && cull) {
+        if (keep) {
           const float4 l = __ldcg(&gs.box[2 * (blk0 + sb)]);
           const float4 h = __ldcg(&gs.box[2 * (blk0 + sb) + 1]);
           const float w = __ldcg(&gs.wa[blk0 + sb].x);
@@ -518,7 +516,6 @@ __global__ void __launch_bounds__(W * 32)
     const bool two = row0 + kTile < npad;
     const int nbt = two ? 4 : 2;
     const int blk0 = pt / kSub, nblk = npad / kSub;
-    const bool cull = !ga.slot || ga.slot[p] < 0;  // as in the shooting sweep
     float4 q[R];
     bool live[R];
 #pragma unroll
@@ -563,7 +560,7 @@ __global__ void __launch_bounds__(W * 32)
         if (base >= nblk) return nblk;
         const int sb = base + lane * nw;
         bool keep = sb < nblk;
-        if (keep && cull) {
+        if (keep) {
           const int b = blk0 + sb;
           const float4 l = __ldcg(&gs.box[2 * b]), h = __ldcg(&gs.box[2 * b + 1]);
           keep = !adjoint_skips(cut, gauss_gap2(T, l, h), __ldcg(&gs.wu[b].x),

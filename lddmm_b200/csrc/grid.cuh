@@ -24,7 +24,8 @@
 // addition is associative, so the sums do not depend on the order of arrival and results
 // are reproducible bit for bit.  A pair whose box outgrows its grid or whose operands are
 // not finite is evaluated by the pair sums (gauss.cuh) in that step; both sides read the
-// same descriptor.
+// same descriptor, and the first convolution's CTAs, which have nothing else to do then,
+// write the statistics of the pair's blocks that the pair sums' distance test reads.
 #pragma once
 
 #include "gauss.cuh"
@@ -247,9 +248,22 @@ __device__ __forceinline__ void load_ker(const GridTables *tab, double *T) {
   }
 }
 
+// Statistics of one block in the points' own order, one point per lane (u or null).
+__device__ __forceinline__ void block_stats(int pt, bool live, const float4 *qs, const float4 *us,
+                                            float4 *box, float4 *wu) {
+  const float4 x = __ldcg(&qs[pt]);
+  gauss_block_box(box, pt / kSub, live, x.x, x.y, x.z, nullptr);
+  if (!us) return;
+  const float s = or_inf(warp_sum_f(abs_sum(__ldcg(&us[pt]))));
+  if ((threadIdx.x & 31) == 0) wu[pt / kSub] = make_float4(s, 0.0f, 0.0f, 0.0f);
+}
+
 // The plane x = blockIdx.x of component blockIdx.y of grid blockIdx.z: integers to
-// doubles (the integers are cleared for the next step), z axis, y axis.
-__global__ void __launch_bounds__(kConvThreads) grid_conv_yz_kernel(const GridArgs A, int adj) {
+// doubles (the integers are cleared for the next step), z axis, y axis.  Pairs that the step does not fit: the
+// statistics of their blocks (in the spread kernel this branch cost a step of 40,962 landmarks
+// that does not take it 0.8 to 2.5 %).
+__global__ void __launch_bounds__(kConvThreads) grid_conv_yz_kernel(
+    const GridArgs A, int adj, const float4 *qs, const float4 *us, float4 *box, float4 *wu) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *T = reinterpret_cast<double *>(smem_raw);
   pdl_wait();
@@ -257,7 +271,16 @@ __global__ void __launch_bounds__(kConvThreads) grid_conv_yz_kernel(const GridAr
   const int p = A.pairs[blockIdx.z], c = blockIdx.y;
   if (!A.act[p]) return;
   GridDesc g;
-  if (!grid_active(A, p, adj != 0, g) || (int)blockIdx.x >= g.n[0]) return;
+  if (!grid_active(A, p, adj != 0, g)) {
+    const int lane = threadIdx.x & 31, nw = gridDim.x * gridDim.y * (kConvThreads / 32);
+    const PairDesc &P = A.pd[p];
+    for (int b = (blockIdx.y * gridDim.x + blockIdx.x) * (kConvThreads / 32) + threadIdx.x / 32;
+         b < P.Npad / kSub; b += nw)
+      block_stats(P.pt_off + b * kSub + lane, b * kSub + lane < P.N, qs, adj ? us : nullptr, box,
+                  wu);
+    return;
+  }
+  if ((int)blockIdx.x >= g.n[0]) return;
   const int ny = g.n[1], nz = g.n[2];
   const int zs = nz + 1;  // odd row stride in shared memory
   double *b0 = T + 2 * kGridMaxDim + 2, *b1 = b0 + ny * zs;

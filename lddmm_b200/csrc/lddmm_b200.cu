@@ -396,11 +396,10 @@ static cudaError_t grid_attributes() {
   return cudaSuccess;
 }
 
-// Spread and convolve step t's sources: a (and u) -> fields of 3 (6) components.
-static cudaError_t grid_fields(lddmm_ctx &c, int t, const float4 *a, const float4 *u) {
+// Spread step t's sources: a (and u), 3 (6) components.
+static cudaError_t grid_spread(lddmm_ctx &c, int t, const float4 *a, const float4 *u) {
   const GridArgs A = grid_args(c, t);
   const double *q = c.q64 + (size_t)t * c.NPtot * 3;
-  const int adj = u ? 1 : 0;
   for (int k = 0; k < 2; ++k) {
     if (!c.n_gtile[k]) continue;
     GridArgs B = A;
@@ -408,10 +407,21 @@ static cudaError_t grid_fields(lddmm_ctx &c, int t, const float4 *a, const float
     CUE(launch_smem(k ? grid_spread_kernel<128> : grid_spread_kernel<32>,
                     dim3((unsigned)c.n_gtile[k]), kGridThreads, 0,
                     k ? sizeof(GridSpreadSmem<128>) : sizeof(GridSpreadSmem<32>), c.stream, B, a, u,
-                    q, adj));
+                    q, u ? 1 : 0));
   }
+  return cudaSuccess;
+}
+
+// Convolve them: fields of 3 (6) components.  For pairs that the step does not fit: the block
+// statistics of the step's pair sweep.
+static cudaError_t grid_convolve(lddmm_ctx &c, int t, int adj) {
+  const size_t nb = (size_t)c.NPtot / kSub;
+  const GridArgs A = grid_args(c, t);
   const dim3 gr((unsigned)c.grid_dmax, adj ? 6u : 3u, (unsigned)c.n_grid);
-  CUE(launch_smem(grid_conv_yz_kernel, gr, kConvThreads, 0, conv_smem(c), c.stream, A, adj));
+  CUE(launch_smem(grid_conv_yz_kernel, gr, kConvThreads, 0, conv_smem(c), c.stream, A, adj,
+                  (const float4 *)(c.qs + (size_t)t * c.NPtot),
+                  (const float4 *)(c.us + (size_t)(t & 1) * c.NPtot), c.gbox + 2 * nb * t,
+                  c.gwu + nb * (t & 1)));
   return launch_smem(grid_conv_x_kernel, gr, kConvThreads, 0, conv_smem(c), c.stream, A, adj);
 }
 
@@ -450,16 +460,18 @@ static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
       if (c.grid) {
         op.by_group = 1;
         op.tile_part = c.reg_part + (size_t)t * c.ngrp_tot;
+        CUE(grid_spread(c, t, op.as_t, nullptr));
+        CUE(grid_convolve(c, t, 0));
+        CUE(launch_smem(grid_interp_kernel<false, ShootOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
+                        kInterpWarps * 32, 0, sizeof(GridInterpSmem<false>), c.stream, op,
+                        grid_args(c, t), op.q64_t, gs));
       }
-      // pairs without a grid, and those whose grid cannot hold this step
-      CUE(launch(gauss_shoot_kernel<kWarps>, gauss_ctas(c, c.n_pt_items2 * c.S_shoot), kWarps * 32,
-                 0, c.stream, op, gs, (const int2 *)c.pt_items2,
-                 SplitPlan{c.S_shoot, c.n_pt_items2, c.P == 1, c.gpart, c.gcnt}, grid_args(c, t)));
-      if (!c.grid) return cudaSuccess;
-      CUE(grid_fields(c, t, op.as_t, nullptr));
-      return launch_smem(grid_interp_kernel<false, ShootOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
-                         kInterpWarps * 32, 0, sizeof(GridInterpSmem<false>), c.stream, op,
-                         grid_args(c, t), op.q64_t, gs);
+      // pairs without a grid, and those whose grid cannot hold this step (last: between the
+      // spread and the convolutions it delayed each step of a gridded pair by 5 us)
+      return launch(gauss_shoot_kernel<kWarps>, gauss_ctas(c, c.n_pt_items2 * c.S_shoot),
+                    kWarps * 32, 0, c.stream, op, gs, (const int2 *)c.pt_items2,
+                    SplitPlan{c.S_shoot, c.n_pt_items2, c.P == 1, c.gpart, c.gcnt},
+                    grid_args(c, t));
     }
   }
   // packed FP32x2 form of the same sweep (bitwise the same sums), on one- or two-tile
@@ -498,14 +510,16 @@ static cudaError_t adjoint_impl(lddmm_ctx &c, int t, double *g, double *pdot) {
   if constexpr (D == 3 && ORDER == -1) {
     if (c.gauss) {
       const GaussStats gs = gauss_stats(c, t);
-      CUE(launch(gauss_adjoint_kernel<kWarps>, gauss_ctas(c, c.n_pt_items2 * c.S_adj), kWarps * 32,
-                 0, c.stream, op, gs, (const int2 *)c.pt_items2,
-                 SplitPlan{c.S_adj, c.n_pt_items2, c.P == 1, c.gpart, c.gcnt}, grid_args(c, t)));
-      if (!c.grid) return cudaSuccess;
-      CUE(grid_fields(c, t, op.as_t, op.us_t));
-      return launch_smem(grid_interp_kernel<true, AdjointOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
-                         kInterpWarps * 32, 0, sizeof(GridInterpSmem<true>), c.stream, op,
-                         grid_args(c, t), (const double *)(c.q64 + (size_t)t * c.NPtot * D), gs);
+      if (c.grid) {
+        CUE(grid_spread(c, t, op.as_t, op.us_t));
+        CUE(grid_convolve(c, t, 1));
+        CUE(launch_smem(grid_interp_kernel<true, AdjointOp<D, ORDER>>, dim3((unsigned)c.n_gblk),
+                        kInterpWarps * 32, 0, sizeof(GridInterpSmem<true>), c.stream, op,
+                        grid_args(c, t), (const double *)(c.q64 + (size_t)t * c.NPtot * D), gs));
+      }
+      return launch(gauss_adjoint_kernel<kWarps>, gauss_ctas(c, c.n_pt_items2 * c.S_adj),
+                    kWarps * 32, 0, c.stream, op, gs, (const int2 *)c.pt_items2,
+                    SplitPlan{c.S_adj, c.n_pt_items2, c.P == 1, c.gpart, c.gcnt}, grid_args(c, t));
     }
   }
   // packed FP32x2 form of the same sweep (bitwise the same sums), one- or two-tile
@@ -1095,9 +1109,14 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf);
 // dependent launches per sweep (22 M: 80 us of 148 SMs) and the convolutions, 9 fields x
 // 3 axes x about 53 taps per node at 64 per clock (20,011 landmarks: 0.28 ms against 0.46,
 // 40,962: 0.42, 163,842: 1.27 against 32).  The grid must win by a tenth: from about
-// 15,000 landmarks on for a unit shape at kernel width 0.3.  The grids of a context are
-// bounded to 4 GB, largest pairs first; each is 1.7 times the nodes of the initial box
-// (extents up to 1.35 times).
+// 15,000 landmarks on for a unit shape at kernel width 0.3.
+//
+// Room: a registration ends near its target, so an axis may hold 1.35 times the source's
+// extent or 1.1 times that of source and target together (a target 1.5 times as large: 7.7
+// instead of 38.4 ms for an evaluation of 163,842 landmarks whose momenta carry the source
+// there, which left the grid when its room came from the source alone).  The grids of a
+// context are bounded to 4 GB, largest pairs first; where the room does not fit, 1.7 times
+// the nodes of the initial box.
 static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
   constexpr long long kGridBytes = 4ll << 30;
   std::vector<int> order(c.P), pairs, slot(c.P, -1);
@@ -1109,31 +1128,45 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
   for (int p : order) {
     const PairDesc &P = c.hpd[p];
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    bool fin = true;
-    for (int i = 0; i < P.N; ++i)
-      for (int d = 0; d < 3; ++d) {
-        const double x = probs[p].ini_nde[(size_t)i * 3 + d] * P.kscale64;
-        fin &= std::isfinite(x);
-        lo[d] = std::min(lo[d], x);
-        hi[d] = std::max(hi[d], x);
-      }
-    double nodes = 1.0, nmax = 0.0;
+    auto extend = [&](const double *x, int n) {
+      bool fin = true;
+      for (int i = 0; i < n; ++i)
+        for (int d = 0; d < 3; ++d) {
+          const double y = x[(size_t)i * 3 + d] * P.kscale64;
+          fin &= std::isfinite(y);
+          lo[d] = std::min(lo[d], y);
+          hi[d] = std::max(hi[d], y);
+        }
+      return fin;
+    };
+    double ext[3], room[3], nodes = 1.0, roomy = 1.0, nmax = 0.0, rmax = 0.0;
+    const bool fin = extend(probs[p].ini_nde, P.N);
     for (int d = 0; d < 3; ++d) {
-      const double n = std::floor((hi[d] - lo[d]) / kGridH) + kWin + 2;
-      nodes *= n;
-      nmax = std::max(nmax, n);
+      ext[d] = std::floor((hi[d] - lo[d]) / kGridH) + kWin + 2;
+      nodes *= ext[d];
+      nmax = std::max(nmax, ext[d]);
+    }
+    extend(probs[p].tgt_cen_pos, P.Et);
+    for (int d = 0; d < 3; ++d) {
+      const double both = 1.1 * (std::floor((hi[d] - lo[d]) / kGridH) + kWin + 2);
+      // (a target that is not finite: the first branch)
+      room[d] = std::ceil(both > 1.35 * ext[d] && both < 2.0 * kGridMaxDim ? both : 1.35 * ext[d]);
+      room[d] = std::min(room[d], (double)kGridMaxDim);
+      roomy *= room[d];
+      rmax = std::max(rmax, room[d]);
     }
     if (!fin || !(nmax <= 0.9 * kGridMaxDim)) continue;
     const double pair = 0.32 * P.N * (double)P.N;
     const double grid = 22e6 + 2500.0 * P.N + 9.0 * 3.0 * std::min(nmax, 53.0) / 64.0 * nodes;
-    const long long cp = (long long)(1.7 * nodes);
+    long long cp = (long long)roomy;
+    if ((total + cp) * 6 * 16 > kGridBytes) cp = (long long)(1.7 * nodes);
     if (pair < 1.1 * grid || (total + cp) * 6 * 16 > kGridBytes) continue;
     slot[p] = (int)pairs.size();
     pairs.push_back(p);
     off.push_back(total);
     cap.push_back(cp);
     total += cp;
-    c.grid_dmax = std::max(c.grid_dmax, std::min(kGridMaxDim, (int)std::ceil(1.35 * nmax)));
+    c.grid_dmax = std::max(c.grid_dmax, (int)rmax);
   }
   c.n_grid = (int)pairs.size();
   if (!c.n_grid) return 0;

@@ -164,3 +164,120 @@ def test_split_varifold_value_near_convergence(cw):
     v64 = dot(S, S) - 2 * dot(S, T) + tt
     assert v64 < 0.2 * tt
     assert abs(V - v64) < 8e-9 * tt, (V - v64) / tt
+
+
+def _radial(P, growth):
+    """Momenta whose velocities carry the unit sphere's neighbourhood outwards by `growth` in
+    each of the T steps: the kernel's mass on a sphere of radius R is N w^2 / (4 R^2)."""
+    a, R = np.empty((P.T, P.nde_num, 3)), 1.0
+    for t in range(P.T):
+        a[t] = P.ini_nde * (growth / P.time_stp * 4 * R * R / (P.nde_num * P.knl_width ** 2))
+        R *= 1 + growth
+    return a.reshape(-1)
+
+
+def _shoot_ms(P, a, reps=3):
+    from lddmm_b200 import api
+
+    with api.Context(P) as ctx:
+        ctx.objgrd(a)
+        return min(ctx.time_sweeps(reps)["shoot"] for _ in range(3))
+
+
+def test_a_larger_target_leaves_the_grid_its_room():
+    """163,842 landmarks on the way to a target 1.5 times as large stay on the grid, at twice
+    the time of a source that does not move at most (the pair sums take 15 times as long)."""
+    from lddmm_b200 import problem, shapes
+
+    P = problem.star_pair()
+    tv, tf = shapes.icosphere(4)
+    P = problem.Problem(P.ini_nde, P.elm_vtx, *shapes.varifold_of(1.5 * tv, tf), knl_order=-1,
+                        knl_width=0.3, time_num=4, time_stp=1 / 3, cen_width=0.1)
+    assert _shoot_ms(P, _radial(P, 0.3)) < 2.0 * _shoot_ms(P, np.zeros(P.var_num))
+
+
+def test_steps_off_the_grid_skip_blocks():
+    """Steps that outgrow their grid take the time of pair sums that never had one (a landmark
+    far away, without momentum), whose distance test skips most blocks at this width."""
+    from lddmm_b200 import problem
+
+    P = problem.star_pair()
+    P.time_num, P.time_stp, P.knl_width = 4, 1 / 3, 0.15
+    a = _radial(P, 0.7)  # steps 1 and 2 are off the grid
+    off = _shoot_ms(P, a)
+    P.ini_nde = P.ini_nde.copy()
+    P.ini_nde[0] *= 100.0
+    a.reshape(P.T, -1, 3)[:, 0] = 0.0
+    assert off < 1.2 * _shoot_ms(P, a)
+
+
+def test_from_grid_to_pairs_against_fp64():
+    """Step 0 on the grid, steps 1 and 2 beyond it, alone and in a batch with a pair too small
+    for a grid: velocities, gradients and costate steps of a row sample against FP64 sums.
+    FP32 sums are accurate against the sum of their terms' absolute values (the costate step's
+    terms cancel): 1e-6 of each row's."""
+    import ctypes as C
+
+    import torch
+
+    from lddmm_b200 import _lib, api
+
+    P, small = _grid_problem(40000, 0.3, 5), _grid_problem(3000, 0.3, 6)
+    P.dis_wgt = small.dis_wgt = 1e-3
+    noise = np.random.default_rng(2).normal(size=(P.T, P.nde_num, 3))
+    a = _radial(P, 0.7).reshape(P.T, -1, 3)
+    a *= 1 + 0.3 * noise
+    b = _radial(small, 0.2)
+    rows = np.random.default_rng(1).integers(0, P.nde_num, 40)
+    ab = lambda x: np.abs(x).sum(1)  # noqa: E731
+    for batch in ([P], [P, small]):
+        x = np.concatenate([a.reshape(-1), b][:len(batch)])
+        with api.Context(batch) as ctx:
+            q, v = ctx.shoot(x)[0]
+            d = torch.from_numpy(x).cuda()
+            f, g = torch.empty(len(batch), dtype=torch.float64, device="cuda"), d.clone()
+            pst = d.clone()
+            _lib.check(_lib.lib.lddmm_objgrd_costate(
+                ctx.handle, *[C.c_void_p(z.data_ptr()) for z in (d, f, g, pst)]))
+            f = f.cpu().numpy()
+            g, pst = (z.cpu().numpy()[:P.var_num].reshape(a.shape) for z in (g, pst))
+        w2 = P.knl_width ** 2
+        energy = 0.0
+        for t in range(P.T):
+            dx = q[t][rows][:, None] - q[t][None]
+            K = np.exp(-(dx ** 2).sum(-1) / w2)
+            u, l = a[t] - pst[t], 0.5 * a[t] - pst[t]
+            assert np.all(ab(K @ a[t] - v[t][rows]) < 1e-6 * ab(K @ np.abs(a[t])))
+            assert np.all(ab(K @ u - g[t][rows] / P.time_stp) < 1e-6 * ab(K @ np.abs(u)))
+            energy += 0.5 * P.time_stp * np.sum(a[t] * v[t])
+            if t:
+                lr = l[rows] @ a[t].T + a[t][rows] @ l.T
+                dq = -2 / w2 * ((K * lr)[..., None] * dx).sum(1)
+                step = (pst[t][rows] - pst[t - 1][rows]) / P.time_stp
+                al, ar = np.abs(l), np.abs(a[t])
+                tot = 2 / w2 * (K * (al[rows] @ ar.T + ar[rows] @ al.T)
+                                * np.sqrt((dx ** 2).sum(-1))).sum(1)
+                assert np.all(ab(dq - step) < 1e-6 * tot)
+        value, _ = api.varifold(P, q[-1])
+        assert abs(f[0] - energy - P.dis_wgt * value) < 1e-6 * abs(f[0])
+
+
+def test_momenta_on_a_part_of_a_gridded_shape():
+    """Momenta on a cap only.  The grid's kernel is wrong by an absolute 3.6e-11 where it is
+    near 1, less further out (1e-6 of itself at 4.2 scaled units, 3.5 widths), and the node
+    sums are multiples of N max|a| 2^-61: every row, however far from the momenta, is within
+    1e-6 of its own sum of absolute values (the FP32 coordinates of pair sums leave as much
+    there), or within 1e-12 of the largest."""
+    from lddmm_b200 import api
+
+    P = _grid_problem(40000, 0.3, 5)
+    rng = np.random.default_rng(8)
+    a = (rng.normal(size=(P.T, 40000, 3)) * 0.01).astype(np.float32).astype(np.float64)
+    a[:, P.ini_nde[:, 2] < 0.6] = 0.0
+    with api.Context(P) as ctx:
+        (q, v), = ctx.shoot(a.reshape(-1))
+    rows = rng.integers(0, 40000, 400)
+    for t in range(P.T):
+        K = np.exp(-((q[t][rows][:, None] - q[t][None]) ** 2).sum(-1) / P.knl_width ** 2)
+        own, err = (K @ np.abs(a[t])).sum(1), np.abs(K @ a[t] - v[t][rows]).sum(1)
+        assert np.all(err < 1e-6 * own + 1e-12 * own.max())
