@@ -11,6 +11,8 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/lddmm_b200.h"
@@ -133,7 +135,15 @@ int pad_to(int n, int k) { return (n + k - 1) / k * k; }
 
 // ============================================================== the context
 
+// What a context is created for.  The single-call helpers evaluate one sum and do without what
+// pays off over a registration's evaluations only: the grids with their k-d order (kMultiply),
+// all of the time loops and their tuning but the general adjoint sweep (kDq) or all of them
+// (kVarifold).  Host times with all of it -> now: multiplyKernel of 20,000 / 163,842 3D Gaussian
+// points 3.8 -> 1.3 / 39.0 -> 18.2 ms, dqKernel 4.0 -> 1.3 / 57.0 -> 26.6, varifold 140 -> 89.
+enum class Use { kRegistration, kMultiply, kDq, kVarifold };
+
 struct lddmm_ctx {
+  Use use = Use::kRegistration;
   int D = 3, order = -1, T = 0, time_num = 0, P = 0;
   char ct = 'G', dt = 'B';
   bool has_vfd = true;
@@ -466,8 +476,8 @@ static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
                         kInterpWarps * 32, 0, sizeof(GridInterpSmem<false>), c.stream, op,
                         grid_args(c, t), op.q64_t, gs));
       }
-      // pairs without a grid, and those whose grid cannot hold this step (last: between the
-      // spread and the convolutions it delayed each step of a gridded pair by 5 us)
+      // pairs without a grid, and those whose grid cannot hold this step (their block
+      // statistics come from the convolution)
       return launch(gauss_shoot_kernel<kWarps>, gauss_ctas(c, c.n_pt_items2 * c.S_shoot),
                     kWarps * 32, 0, c.stream, op, gs, (const int2 *)c.pt_items2,
                     SplitPlan{c.S_shoot, c.n_pt_items2, c.P == 1, c.gpart, c.gcnt},
@@ -476,11 +486,11 @@ static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
   }
   // packed FP32x2 form of the same sweep (bitwise the same sums), on one- or two-tile
   // work items (c.tpw_shoot; the default rule and the autotuner pick it).  Two tiles
-  // per item serve four rows per lane from each staged column: the Gaussian sweep,
-  // held first by the shared-memory reads, gains (163,842 landmarks: 11.13 -> 10.58
-  // ms); the Matern kernels, with a square root per pair and fewer CTAs per SM at the
-  // larger register count, were faster on single tiles (40,962: 1.02 vs 1.10 ms).
-  if (c.tpw_shoot == 2)
+  // per item serve four rows per lane from each staged column; the Matern kernels, with a
+  // square root per pair and fewer CTAs per SM at the larger register count, were faster
+  // on single tiles (40,962: 1.02 vs 1.10 ms).  3D Gaussian shooting never comes here.
+  if constexpr (D == 3 && ORDER == -1) return cudaErrorNotSupported;
+  else if (c.tpw_shoot == 2)
     return launch(sweep_packed_kernel<ShootOp<D, ORDER>, kWarps, 2>,
                   (unsigned)(c.n_pt_items2 * c.S_shoot), kWarps * 32, c.S_shoot, c.stream, op,
                   (const int2 *)c.pt_items2, c.S_shoot);
@@ -984,29 +994,58 @@ static int default_cluster(int n_items, int sms = 148) {
 
 // Points in k-d order: split at the median of the longest axis, at multiples of 128 and
 // then of 32 points, so that consecutive tiles of that size are compact whatever the order
-// of the mesh's vertices or elements.
-static void kd_order(const double *x, int *idx, int lo, int hi) {
-  while (hi - lo > 32) {
-    const int unit = hi - lo > 128 ? 128 : 32;
-    const int mid = lo + std::max(unit, ((hi - lo) / 2 + unit / 2) / unit * unit);
+// of the mesh's vertices or elements.  The points are sorted with their coordinates, halves
+// of more than 1,024 points in threads of their own (at most 16; where none can be had, in
+// this one).  Creating a context of 20,000 landmarks: 14.3 ms, 20.6 with a sort through an
+// index in one thread.
+struct KdPoint {
+  double x[3];
+  int i;
+};
+
+static void kd_split(KdPoint *p, int n, int threads) {
+  while (n > 32) {
+    const int unit = n > 128 ? 128 : 32;
+    const int mid = std::max(unit, (n / 2 + unit / 2) / unit * unit);
+    if (mid >= n) return;
     double l[3], h[3];
-    for (int d = 0; d < 3; ++d) l[d] = h[d] = x[(size_t)idx[lo] * 3 + d];
-    for (int k = lo + 1; k < hi; ++k)
+    for (int d = 0; d < 3; ++d) l[d] = h[d] = p[0].x[d];
+    for (int k = 1; k < n; ++k)
       for (int d = 0; d < 3; ++d) {
-        l[d] = std::min(l[d], x[(size_t)idx[k] * 3 + d]);
-        h[d] = std::max(h[d], x[(size_t)idx[k] * 3 + d]);
+        l[d] = std::min(l[d], p[k].x[d]);
+        h[d] = std::max(h[d], p[k].x[d]);
       }
     int ax = 0;
     for (int d = 1; d < 3; ++d)
       if (h[d] - l[d] > h[ax] - l[ax]) ax = d;
-    if (mid >= hi) return;
-    std::nth_element(idx + lo, idx + mid, idx + hi, [&](int a, int b) {
-      const double u = x[(size_t)a * 3 + ax], v = x[(size_t)b * 3 + ax];
-      return u < v || (u == v && a < b);
+    std::nth_element(p, p + mid, p + n, [ax](const KdPoint &a, const KdPoint &b) {
+      return a.x[ax] < b.x[ax] || (a.x[ax] == b.x[ax] && a.i < b.i);
     });
-    kd_order(x, idx, lo, mid);
-    lo = mid;
+    std::thread half;
+    if (threads > 1 && mid > 1024) {
+      try {
+        half = std::thread(kd_split, p, mid, threads / 2);
+      } catch (const std::system_error &) {
+      }
+    }
+    if (half.joinable()) {
+      kd_split(p + mid, n - mid, threads - threads / 2);
+      half.join();
+      return;
+    }
+    kd_split(p, mid, 1);
+    p += mid;
+    n -= mid;
   }
+}
+
+static std::vector<int> kd_order(const double *x, int n) {
+  std::vector<KdPoint> p(n);
+  for (int k = 0; k < n; ++k) p[k] = {{x[3 * (size_t)k], x[3 * (size_t)k + 1], x[3 * (size_t)k + 2]}, k};
+  kd_split(p.data(), n, (int)std::min(std::max(std::thread::hardware_concurrency(), 1u), 16u));
+  std::vector<int> idx(n);
+  for (int k = 0; k < n; ++k) idx[k] = p[k].i;
+  return idx;
 }
 
 // Summed extent of the bounding boxes of consecutive 32-element blocks.
@@ -1072,9 +1111,7 @@ static std::vector<int> kd_spatial_order(const std::vector<double> &cen, int n) 
   if (n < 64) return {};
   for (double x : cen)
     if (!std::isfinite(x)) return {};
-  std::vector<int> perm(n);
-  for (int e = 0; e < n; ++e) perm[e] = e;
-  kd_order(cen.data(), perm.data(), 0, n);
+  const std::vector<int> perm = kd_order(cen.data(), n);
   if (block_extent(cen, n, &perm) < 0.9 * block_extent(cen, n, nullptr)) return perm;
   return {};
 }
@@ -1180,9 +1217,8 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
   c.n_gblk = (int)blk.size();
   std::vector<int> ord(c.NPtot, 0);
   for (int p : pairs) {
-    int *o = &ord[c.hpd[p].pt_off];
-    for (int i = 0; i < c.hpd[p].N; ++i) o[i] = i;
-    kd_order(probs[p].ini_nde, o, 0, c.hpd[p].N);
+    const std::vector<int> o = kd_order(probs[p].ini_nde, c.hpd[p].N);
+    std::copy(o.begin(), o.end(), ord.begin() + c.hpd[p].pt_off);
   }
   auto put = [&](auto **d, const auto &h) -> cudaError_t {
     CUE(dalloc(c.stream, d, h.size()));
@@ -1211,8 +1247,8 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
   return 0;
 }
 
-extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm_config *cfg,
-                                lddmm_ctx **out) {
+static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *cfg, Use use,
+                      lddmm_ctx **out) {
   if (!out || !probs || num <= 0) {
     set_err("lddmm_ctx_create: bad arguments");
     return LDDMM_ERR_ARG;
@@ -1234,6 +1270,7 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
   if (cfg) cf = *cfg;
   std::unique_ptr<lddmm_ctx> cp(new lddmm_ctx());
   lddmm_ctx &c = *cp;
+  c.use = use;
   const lddmm_problem &p0 = probs[0];
   c.D = p0.dim;
   c.order = p0.knl_order;
@@ -1736,7 +1773,7 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
       c.cycle_grid_lm = bc * sms;
     }
   }
-  if (c.D == 3 && c.order == -1 && cf.persistent <= 0) {
+  if (c.D == 3 && c.order == -1 && (use == Use::kRegistration || use == Use::kMultiply)) {
     // 3D Gaussian per-step sweeps: S independent CTAs per 128-row item (default 8: at
     // 9,001 / 40,962 / 163,842 landmarks 8 is within 3 % of the best of 1..32; fewer
     // leave SMs idle at the end of a sweep, 1: 119 / 859 / 7065 us per shooting step
@@ -1751,8 +1788,10 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
                                       kGaussRows * AdjointOp<3, -1>::NA));
     CU(dalloc(c.stream, &c.gcnt, c.n_pt_items2));
     c.gauss = true;
-    const int rc = setup_grid(c, probs);
-    if (rc) return rc;
+    if (use == Use::kRegistration && cf.persistent <= 0) {
+      const int rc = setup_grid(c, probs);
+      if (rc) return rc;
+    }
     CU(launch(gauss_box_kernel, (unsigned)((nb + 3) / 4), 128, 0, c.stream, (const float4 *)c.qs,
               (const int *)c.pt_pair, (int)nb, c.gbox, c.gkeys));
   }
@@ -1763,6 +1802,11 @@ extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm
   if (c.persistent) c.gauss = c.grid = false;
   *out = cp.release();
   return 0;
+}
+
+extern "C" int lddmm_ctx_create(const lddmm_problem *probs, int num, const lddmm_config *cfg,
+                                lddmm_ctx **out) {
+  return create_ctx(probs, num, cfg, Use::kRegistration, out);
 }
 
 // Clears the persistent kernels' barrier / error words and the split row groups'
@@ -2490,7 +2534,7 @@ static std::string tune_key(const lddmm_ctx &c, const lddmm_config &cf) {
   auto add = [&](long long v) { k += std::to_string(v) + ","; };
   add(c.device); add(c.D); add(c.order); add(c.ct); add(c.dt); add(c.T); add(c.has_vfd);
   add(c.persistent); add(cf.cluster_shoot); add(cf.cluster_adjoint); add(cf.cluster_varifold);
-  add(cf.persistent);
+  add(cf.persistent); add((int)c.use);
   for (const PairDesc &d : c.hpd) {
     add(d.Npad); add(d.Edpad); add(d.Etpad);
   }
@@ -2569,8 +2613,8 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
   if (c.gauss) {
     CU(gauss_begin(c));
     CU(cudaMemsetAsync(c.gwu, 0, sizeof(float4) * 2 * c.NPtot / kSub, c.stream));
-  } else {
-    tune_step(0, &c.S_shoot, &c.tpw_shoot, cf.cluster_shoot > 0);
+  } else if (c.use != Use::kVarifold) {
+    if (c.use != Use::kDq) tune_step(0, &c.S_shoot, &c.tpw_shoot, cf.cluster_shoot > 0);
     tune_step(1, &c.S_adj, &c.tpw_adj, cf.cluster_adjoint > 0);
   }
   if (err == cudaSuccess && c.has_vfd && cf.cluster_varifold <= 0) {
@@ -2666,7 +2710,7 @@ extern "C" int lddmm_multiply_kernel(int dim, int n, const double *q, const doub
   lddmm_ctx *ctx = nullptr;
   lddmm_config cfg = {};
   cfg.use_graph = -1;
-  int rc = lddmm_ctx_create(&p, 1, &cfg, &ctx);
+  int rc = create_ctx(&p, 1, &cfg, Use::kMultiply, &ctx);
   if (rc) return rc;
   std::unique_ptr<lddmm_ctx, void (*)(lddmm_ctx *)> guard(ctx, lddmm_ctx_destroy);
   std::vector<double> vs((size_t)2 * n * dim), qs;
@@ -2686,7 +2730,8 @@ extern "C" int lddmm_dq_kernel(int dim, int n, const double *q, const double *l,
   lddmm_ctx *ctx = nullptr;
   lddmm_config cfg = {};
   cfg.use_graph = -1;
-  int rc = lddmm_ctx_create(&p, 1, &cfg, &ctx);
+  cfg.persistent = -1;
+  int rc = create_ctx(&p, 1, &cfg, Use::kDq, &ctx);
   if (rc) return rc;
   std::unique_ptr<lddmm_ctx, void (*)(lddmm_ctx *)> guard(ctx, lddmm_ctx_destroy);
   lddmm_ctx &c = *ctx;
@@ -2709,7 +2754,7 @@ extern "C" int lddmm_dq_kernel(int dim, int n, const double *q, const double *l,
   CU(cudaMemcpyAsync(c.ls, hl.data(), sizeof(float4) * c.NPtot, cudaMemcpyHostToDevice, c.stream));
   CU(cudaMemcpyAsync(c.as, hr.data(), sizeof(float4) * c.NPtot, cudaMemcpyHostToDevice, c.stream));
   CU(launch_set_active(c, 1));
-  c.gauss = c.grid = false;  // l and r are not a step's operands (u = l + r / 2): the general sweep
+  // (l and r are not a step's operands, u = l + r / 2: the general sweep)
   CU(c.adjoint(c, 0, nullptr, pd));
   std::vector<double> h((size_t)c.NPtot * dim);
   CU(cudaMemcpyAsync(h.data(), pd, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c.stream));
@@ -2966,7 +3011,8 @@ extern "C" int lddmm_varifold(const lddmm_problem *prob, const double *nde, doub
   lddmm_ctx *ctx = nullptr;
   lddmm_config cfg = {};
   cfg.use_graph = -1;
-  int rc = lddmm_ctx_create(&p, 1, &cfg, &ctx);
+  cfg.persistent = -1;
+  int rc = create_ctx(&p, 1, &cfg, Use::kVarifold, &ctx);
   if (rc) return rc;
   std::unique_ptr<lddmm_ctx, void (*)(lddmm_ctx *)> guard(ctx, lddmm_ctx_destroy);
   lddmm_ctx &c = *ctx;

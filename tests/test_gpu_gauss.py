@@ -281,3 +281,27 @@ def test_momenta_on_a_part_of_a_gridded_shape():
         K = np.exp(-((q[t][rows][:, None] - q[t][None]) ** 2).sum(-1) / P.knl_width ** 2)
         own, err = (K @ np.abs(a[t])).sum(1), np.abs(K @ a[t] - v[t][rows]).sum(1)
         assert np.all(err < 1e-6 * own + 1e-12 * own.max())
+
+
+@pytest.mark.parametrize("kind", ["multiply", "dq"])
+def test_single_sums_prepare_no_grid(kind):
+    """One kernel sum of 60,000 3D Gaussian points on host arrays costs about what the Matern
+    sum of the same size does (whose kernel takes longer): no k-d order, no grids."""
+    import time
+
+    from lddmm_b200 import api
+
+    rng = np.random.default_rng(4)
+    q, a = rng.normal(size=(2, 60000, 3))
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+
+    def ms(order):
+        t = []
+        for _ in range(6):  # the first one tunes
+            t0 = time.perf_counter()
+            api.multiplyKernel(q, a, order, 0.3) if kind == "multiply" else \
+                api.dqKernel(q, a, a, order, 0.3)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    assert ms(-1) < 1.5 * ms(1)
