@@ -233,7 +233,8 @@ struct lddmm_ctx {
   OptParams loop_opt{};
   int *cyc = nullptr;  // cycles run by the device loop
   long long last_cycles = 0, last_launches = 0, last_evals = 0;
-  int last_mem = 0;  // L-BFGS memory (ring slots) of the last lddmm_lbfgs call
+  // kernels per cycle: of the last lddmm_lbfgs call, of the two graphs
+  long long last_kernels = 0, graph_kernels = 0, loop_kernels = 0;
   int lbfgs_calls = 0;  // graphs are captured from the second L-BFGS call on
   bool use_graph = true;
   cudaGraphExec_t cycle_exec = nullptr;
@@ -295,6 +296,16 @@ lddmm_ctx::~lddmm_ctx() {
 
 // ============================================================ kernel launch
 
+// This thread's launches, counted where they are made: kernels per optimiser cycle.
+static thread_local long long t_launches = 0;
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_ex(const cudaLaunchConfig_t *cfg, void (*kern)(KArgs...),
+                             Args &&...args) {
+  ++t_launches;
+  return cudaLaunchKernelEx(cfg, kern, std::forward<Args>(args)...);
+}
+
 // Every kernel of the objective sweep and the L-BFGS cycle goes through launch():
 // programmatic stream serialisation (the kernel calls pdl_wait() before touching its
 // predecessor's output) and, for the sweeps, the thread-block cluster size.
@@ -320,7 +331,7 @@ static cudaError_t launch_smem(void (*kern)(KArgs...), dim3 grid, unsigned block
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+  return launch_ex(&cfg, kern, std::forward<Args>(args)...);
 }
 
 template <typename... KArgs, typename... Args>
@@ -570,7 +581,7 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, persistent_cluster_kernel<Op>, op, cp, T, dir, c.sync);
+    return launch_ex(&cfg, persistent_cluster_kernel<Op>, op, cp, T, dir, c.sync);
   }
   if (c.pers_kind == 2)  // one cluster per pair: stream serialisation like the other sweeps
     return launch_smem(small_sweep_kernel<Op>, dim3((unsigned)(c.P * c.small_C)),
@@ -592,7 +603,7 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, persistent_sweep_kernel<Op>, op, plan, T, dir, c.sync);
+  return launch_ex(&cfg, persistent_sweep_kernel<Op>, op, plan, T, dir, c.sync);
 }
 
 // Whether clusters of C CTAs of the small form can run both persistent sweeps.
@@ -2094,9 +2105,8 @@ static cudaError_t launch_cycle(lddmm_ctx &c, const OptParams &o,
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, lbfgs_cycle_kernel, A, o, c.rec, c.act,
-                              c.P, c.nchunk_tot, c.sync, h, max_cycles > 0 ? c.cyc : nullptr,
-                              max_cycles);
+    return launch_ex(&cfg, lbfgs_cycle_kernel, A, o, c.rec, c.act, c.P, c.nchunk_tot, c.sync, h,
+                     max_cycles > 0 ? c.cyc : nullptr, max_cycles);
   }
   auto pass = [&](int mode) -> cudaError_t {
     return launch(vec_pass_kernel, nb, kVecThreads, 0, c.stream, A, mode);
@@ -2126,16 +2136,6 @@ static cudaError_t launch_cycle(lddmm_ctx &c, const OptParams &o,
   return cudaSuccess;
 }
 
-static long long kernels_per_cycle(const lddmm_ctx &c, int m) {
-  // objective: T shooting + [geometry + varifold] + gather + objective + T adjoint
-  // (2 launches when the time loops are persistent); optimiser: POST, DECIDE, ACCEPT,
-  // SOLVE, FIN, LSINIT, or POST, DECIDE, the 7 long-memory phases, LSINIT (1 launch
-  // when fused)
-  const long long sweeps = c.persistent ? 2 : 2LL * c.T;
-  const long long opt = c.cycle_grid > 0 ? 1 : (m > kMaxMem ? 10 : 6);
-  return sweeps + 2 + (c.has_vfd ? 2 : 0) + opt;
-}
-
 static bool same_opt(const OptParams &a, const OptParams &b) {
   return std::memcmp(&a, &b, sizeof(OptParams)) == 0;
 }
@@ -2148,7 +2148,9 @@ static int build_graph(lddmm_ctx &c, const OptParams &o) {
   }
   cudaGraph_t g = nullptr;
   CU(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
+  const long long n0 = t_launches;
   cudaError_t e = launch_cycle(c, o);
+  c.graph_kernels = t_launches - n0;
   cudaError_t e2 = cudaStreamEndCapture(c.stream, &g);
   if (e != cudaSuccess || e2 != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
@@ -2189,7 +2191,9 @@ static bool build_loop_graph(lddmm_ctx &c, const OptParams &o, int max_cycles) {
       cudaGraph_t body = np.conditional.phGraph_out[0];
       if (cudaStreamBeginCaptureToGraph(c.stream, body, nullptr, nullptr, 0,
                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+        const long long n0 = t_launches;
         const cudaError_t e = launch_cycle(c, o, h, max_cycles);
+        c.loop_kernels = t_launches - n0;
         cudaGraph_t captured = nullptr;
         const cudaError_t e2 = cudaStreamEndCapture(c.stream, &captured);
         ok = (e == cudaSuccess && e2 == cudaSuccess);
@@ -2300,12 +2304,16 @@ static int lbfgs_run(lddmm_ctx &c, const lddmm_opt *opt, const double *alp, bool
     const int rc = build_graph(c, o);
     if (rc) return rc;
   }
+  long long per_cycle = host_loop ? c.graph_kernels : c.loop_kernels;
   while (host_loop) {
     for (int k = 0; k < check_every; ++k) {
-      if (graphs)
+      if (graphs) {
         CU(cudaGraphLaunch(c.cycle_exec, c.stream));
-      else
+      } else {
+        const long long n0 = t_launches;
         CU(launch_cycle(c, o));
+        per_cycle = t_launches - n0;
+      }
     }
     cycles += check_every;
     CU(cudaMemcpyAsync(hact.data(), c.act, sizeof(int) * c.P, cudaMemcpyDeviceToHost, c.stream));
@@ -2323,8 +2331,8 @@ static int lbfgs_run(lddmm_ctx &c, const lddmm_opt *opt, const double *alp, bool
     }
   }
   c.last_cycles = cycles;
-  c.last_launches = cycles * kernels_per_cycle(c, o.mem_num) + 2;
-  c.last_mem = o.mem_num;
+  c.last_kernels = per_cycle;
+  c.last_launches = cycles * per_cycle + 1;  // and the one that begins the call
   CU(cudaMemcpyAsync(hs.data(), c.st, sizeof(PairState) * c.P, cudaMemcpyDeviceToHost, c.stream));
   CU(cudaMemcpyAsync(alp_out, c.X, sizeof(double) * c.nvar,
                      host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, c.stream));
@@ -2423,11 +2431,10 @@ extern "C" int lddmm_ctx_timeline(const lddmm_ctx *ctx, double *us6) {
 
 extern "C" int lddmm_ctx_counters(const lddmm_ctx *ctx, long long *out, int n) {
   if (!ctx || !out || n < 0) return LDDMM_ERR_ARG;
-  const long long v[4] = {ctx->last_cycles, ctx->last_cycles ? ctx->last_launches / ctx->last_cycles : 0,
-                          ctx->last_launches, ctx->last_evals};
+  const long long v[4] = {ctx->last_cycles, ctx->last_kernels, ctx->last_launches,
+                          ctx->last_evals};
   const int k = std::min(n, 4);
   for (int i = 0; i < k; ++i) out[i] = v[i];
-  if (k >= 2 && ctx->last_cycles) out[1] = kernels_per_cycle(*ctx, ctx->last_mem);
   return k;
 }
 

@@ -243,3 +243,30 @@ def test_uneven_3d_batch_objgrd_equals_individual(api, persistent):
         else:  # the persistent work plan cuts the batch's rows differently
             assert abs(fb[k] - f1[0]) <= 1e-6 * abs(f1[0])
             assert np.max(np.abs(gbs[k] - g1)) <= 1e-5 * np.max(np.abs(g1))
+
+
+@pytest.mark.parametrize("form,n,persistent,kernels", [
+    # 2 time loops, geometry, varifold, gather, objective, 1 fused update
+    ("loops", 642, 0, 7),
+    # weights of a and u, 3 + 3 steps, the 4 above, 6 kernels of the update (and one that
+    # controls the device loop, which the fused update does itself)
+    ("steps", 642, -1, 18),
+    # reset, weights of a and u, 3 + 3 steps of spread, 2 convolutions, interpolation and the
+    # pair sweep, the 4 above, 1 fused update
+    ("grid", 40962, 0, 38)])
+def test_kernel_launches_are_counted(form, n, persistent, kernels):
+    """lddmm_ctx_counters counts the launches of each form of the evaluation, from the host and
+    (the second call) from the device loop's graph; one more begins a call."""
+    from lddmm_b200 import api, problem, shapes
+
+    v, f = shapes.icosphere({642: 3, 40962: 6}[n])
+    tv, tf = shapes.icosphere(2)
+    P = problem.Problem(v, f, *shapes.varifold_of(tv * 1.1, tf), knl_order=-1, knl_width=0.3,
+                        time_num=4, time_stp=1 / 3, cen_width=0.3)
+    with api.Context(P, persistent=persistent, autotune=False) as ctx:
+        for call in range(2):
+            ctx.lbfgs(np.zeros(P.var_num), itr_max=2)
+            c = ctx.counters()
+            want = kernels + (call if form == "steps" else 0)
+            assert c["kernels_per_cycle"] == want
+            assert c["launches"] == c["cycles"] * want + 1
