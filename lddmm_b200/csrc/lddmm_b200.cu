@@ -2544,6 +2544,12 @@ static std::string tune_key(const lddmm_ctx &c, const lddmm_config &cf) {
   add(cf.persistent); add((int)c.use);
   for (const PairDesc &d : c.hpd) {
     add(d.Npad); add(d.Edpad); add(d.Etpad);
+    // the kernel widths: they decide what the sweeps with a distance test skip
+    for (double w : {d.pd_fac, d.dc_fac}) {
+      long long b;
+      std::memcpy(&b, &w, sizeof(b));
+      add(b);
+    }
   }
   return k;
 }
@@ -2567,13 +2573,42 @@ static cudaError_t time_median(lddmm_ctx &c, cudaEvent_t e0, cudaEvent_t e1, int
   return cudaSuccess;
 }
 
+// Operands of the trial sweeps: a, u and l of every landmark of one magnitude, too small to
+// move the shape (kTuneMomentum); zero afterwards.
+constexpr double kTuneMomentum = 1e-9;
+__global__ void tune_fill_kernel(const int *pt_pair, int NPtot, double *xt, long long nvar,
+                                 float4 *us, float4 *ls, double m) {
+  const long long nthr = (long long)gridDim.x * blockDim.x;
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nvar; k += nthr)
+    xt[k] = m;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < 2 * NPtot; k += (int)nthr)
+    if (pt_pair[k % NPtot] >= 0) {
+      const float a = (float)m, b = (float)(0.5 * m);
+      us[k] = make_float4(a, a, a, 0.0f);
+      ls[k] = make_float4(b, b, b, 0.0f);
+    }
+}
+
+static cudaError_t tune_operands(lddmm_ctx &c, double m) {
+  tune_fill_kernel<<<256, 256, 0, c.stream>>>(c.pt_pair, c.NPtot, c.XT, c.nvar, c.us, c.ls, m);
+  CUE(cudaGetLastError());
+  CUE(begin_trial(c, c.XT, false));
+  if (!c.gauss) return cudaSuccess;
+  CUE(gauss_begin(c));
+  const int nblk = c.NPtot / kSub;
+  return launch(gauss_alpha_kernel, (unsigned)((nblk + 3) / 4), 128, 0, c.stream,
+                (const float4 *)c.us, 2LL * nblk, nblk, c.gwu, (const int *)c.pt_pair,
+                (unsigned *)nullptr, c.P);
+}
+
 static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
-  // The launch shape of each sweep, chosen by timing the candidates on this batch
-  // (zero momenta; the cost does not depend on the values): per-step shooting and
-  // adjoint sweeps over one or two 64-row tiles per work item and a cluster split S of
-  // 1, 2, 4 or 8 CTAs per item; the varifold sweep over S = 1..8; and, for a batch on
-  // the persistent time-loop sweeps, those against T per-step launches of the tuned
-  // shape.  Sizes given in the configuration are kept.  Every candidate gives the same
+  // The launch shape of each sweep, chosen by timing the candidates on this batch, with
+  // momenta of one magnitude (zeros would switch the Gaussian sweeps' distance test off):
+  // per-step shooting and adjoint sweeps over one or two 64-row tiles per work item and a
+  // cluster split S of 1, 2, 4 or 8 CTAs per item (the 3D Gaussian ones keep theirs); the
+  // varifold sweep over S = 1..8; and, for a batch on the persistent time-loop sweeps, their
+  // L2 and small forms (the cluster form where it is asked for) against T per-step launches
+  // of the tuned shape.  Sizes given in the configuration are kept.  Every candidate gives the same
   // sums up to the order in which a cluster's partial sums are added (two-tile items
   // are bitwise one-tile items), so the choice affects time only.
   const std::string key = tune_key(c, cf);
@@ -2588,7 +2623,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
       return 0;
     }
   }
-  CU(launch_set_active(c, c.P));
+  CU(tune_operands(c, kTuneMomentum));
   if (c.has_vfd) CU(launch_geometry(c, c.q64));  // element boxes of the initial surface
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
@@ -2617,10 +2652,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
     *S = bS;
     *tpw = bT;
   };
-  if (c.gauss) {
-    CU(gauss_begin(c));
-    CU(cudaMemsetAsync(c.gwu, 0, sizeof(float4) * 2 * c.NPtot / kSub, c.stream));
-  } else if (c.use != Use::kVarifold) {
+  if (!c.gauss && c.use != Use::kVarifold) {
     if (c.use != Use::kDq) tune_step(0, &c.S_shoot, &c.tpw_shoot, cf.cluster_shoot > 0);
     tune_step(1, &c.S_adj, &c.tpw_adj, cf.cluster_adjoint > 0);
   }
@@ -2639,8 +2671,6 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
     c.S_vfd = bS;
   }
   if (err == cudaSuccess && c.persistent) {
-    // whole time loops: the persistent forms (L2 combine; cluster combine when the
-    // runtime accepted it) against T per-step launches of the tuned shape
     auto time_loops = [&](float *ms) {
       return time_median(c, e0, e1, reps, [&]() {
         cudaError_t e = c.shoot_all(c, nullptr);
@@ -2679,7 +2709,8 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   CU(err);
-  // the trial sweeps wrote the step-1 positions and adjoint state; reset them
+  // the trial sweeps wrote the later positions and the adjoint state; reset them
+  CU(tune_operands(c, 0.0));
   CU(cudaMemsetAsync(c.p64, 0, sizeof(double) * c.NPtot * c.D, c.stream));
   CU(cudaStreamSynchronize(c.stream));
   std::lock_guard<std::mutex> lk(g_tune_mu);

@@ -59,3 +59,51 @@ def test_autotuned_shape_is_never_slower_than_the_rule(which):
         ms_tuned = _eval_ms(tuned, reps)
     print(f"{which}: rule {shape_rule} {ms_rule:.3f} ms, tuned {shape_tuned} {ms_tuned:.3f} ms")
     assert ms_tuned <= 1.02 * ms_rule, (shape_rule, ms_rule, shape_tuned, ms_tuned)
+
+
+def _surface_pair(n, width=0.3):
+    from lddmm_b200 import problem, shapes
+
+    v, f = shapes.decimated_star(n, 8, 0.05, n)
+    tv, tf = shapes.decimated_star(n, 8, 0.05, n + 1)
+    return problem.Problem(v, f, *shapes.varifold_of(tv, tf), knl_order=-1, knl_width=width,
+                           time_num=11, time_stp=0.1, cen_width=0.1)
+
+
+@pytest.mark.parametrize("n,width", [(3000, 0.3), (5000, 0.1), (9001, 0.3), (9001, 0.1)])
+def test_tuned_time_loops_with_momenta(n, width):
+    """The Gaussian per-step sweeps skip blocks according to the momenta and the width: the
+    form that the tuner picks (on momenta of one magnitude) is at most 5 % slower, with random
+    momenta, than the faster of the two that it chose from."""
+    from lddmm_b200 import api
+
+    P = _surface_pair(n, width)
+    x = np.random.default_rng(n).normal(size=P.var_num) * 1e-4
+    ms = {}
+    for form in (0, 1, -1):
+        with api.Context(P, persistent=form) as ctx:
+            ctx.objgrd(x)
+            ms[form] = _eval_ms(ctx, 20)
+            shape = ctx.launch_shape()["persistent"] if form == 0 else shape
+    print(n, width, shape, ms)
+    assert ms[0] <= 1.05 * min(ms[1], ms[-1]), (shape, ms)
+
+
+def test_contexts_of_other_widths_are_tuned_again():
+    """A context of the same sizes takes over the shapes (no trial sweeps), one of another
+    kernel width does not: what its sweeps skip differs."""
+    import time
+
+    from lddmm_b200 import api
+
+    def seconds(P):
+        t0 = time.perf_counter()
+        with api.Context(P):
+            pass
+        return time.perf_counter() - t0
+
+    P, other = _surface_pair(8999, 0.3), _surface_pair(8999, 0.2)
+    seconds(P)
+    again = min(seconds(P) for _ in range(3))
+    assert seconds(other) > 1.5 * again
+    assert seconds(other) < 1.5 * again
