@@ -148,7 +148,7 @@ struct lddmm_ctx {
   char ct = 'G', dt = 'B';
   bool has_vfd = true;
   float ow2 = 0.0f;
-  int device = 0;
+  int device = 0, sms = 0;  // and its SMs
   std::vector<PairDesc> hpd;
   int NPtot = 0, EDtot = 0, ETtot = 0, ntile_tot = 0, ngrp_tot = 0, netile_tot = 0,
       nchunk_tot = 0;
@@ -252,7 +252,7 @@ struct lddmm_ctx {
   int (*pers_clusters)(int C, int grid) = nullptr;
   cudaError_t (*probe_cluster)(lddmm_ctx &) = nullptr;  // a cluster-form launch, no steps
   cudaError_t (*varifold)(lddmm_ctx &) = nullptr;
-  int (*vfd_clusters)(int S) = nullptr;  // co-resident clusters of S varifold CTAs
+  int (*vfd_clusters)(int S, int sms) = nullptr;  // co-resident clusters of S varifold CTAs
   cudaError_t (*tt)(lddmm_ctx &, int p, double *part, dim3 grid, double cw, double dw) = nullptr;
 
   ~lddmm_ctx();
@@ -387,7 +387,7 @@ static GridArgs grid_args(const lddmm_ctx &c, int t) {
 // CTAs of the pair sweeps: one per unit, or, where every pair has a grid and the sweep
 // usually finds nothing to do, four per SM that walk the units.
 static unsigned gauss_ctas(const lddmm_ctx &c, int units) {
-  return (unsigned)(c.n_grid == c.P && c.grid ? std::min(units, 4 * 148) : units);
+  return (unsigned)(c.n_grid == c.P && c.grid ? std::min(units, 4 * c.sms) : units);
 }
 
 static size_t conv_smem(const lddmm_ctx &c) {
@@ -790,9 +790,9 @@ static bool pick_def(int order, lddmm_ctx &c) {
 }
 
 template <int D, char CT, char DT>
-static int vfd_clusters_impl(int S) {
+static int vfd_clusters_impl(int S, int sms) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(S * 148));
+  cfg.gridDim = dim3((unsigned)(S * sms));
   cfg.blockDim = dim3(kWarps * 32);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -805,7 +805,7 @@ static int vfd_clusters_impl(int S) {
   cudaError_t e;
   if constexpr (D == 3 && CT == 'G' && DT == 'B') {  // S independent CTAs
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, vfd_split_kernel<kWarps>, kWarps * 32, 0);
-    n = n * 148 / S;
+    n = n * sms / S;
   } else {
     e = cudaOccupancyMaxActiveClusters(&n, sweep_packed_kernel<VarifoldOp<D, CT, DT>, kWarps>,
                                        &cfg);
@@ -1644,7 +1644,7 @@ static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *c
   }
   CU(cudaMemcpyAsync(c.pd, c.hpd.data(), sizeof(PairDesc) * num, cudaMemcpyHostToDevice, c.stream));
 
-  const int dev_sms = device_sms(c.device);
+  const int dev_sms = c.sms = device_sms(c.device);
   c.S_shoot = cf.cluster_shoot > 0 ? cf.cluster_shoot : default_cluster(c.n_pt_items, dev_sms);
   c.S_adj = cf.cluster_adjoint > 0 ? cf.cluster_adjoint : default_cluster(c.n_pt_items, dev_sms);
   c.S_vfd =
@@ -1656,7 +1656,7 @@ static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *c
     // S = 5 vs 134-150 us at 6-8 for 80 element tiles)
     int S = 0;
     for (int s = 8; s >= 1 && !S; --s)
-      if (c.n_el_items <= c.vfd_clusters(s)) S = s;
+      if (c.n_el_items <= c.vfd_clusters(s, dev_sms)) S = s;
     if (S) c.S_vfd = S;
   }
   if (c.D == 3 && c.ct == 'G' && c.dt == 'B' && c.has_vfd) {
@@ -1754,7 +1754,8 @@ static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *c
         // rows no longer fit its threads (at 200 points a step takes three quarters of the
         // L2 form's; costly 2D Matern pairs at 500 are faster there, section "small form"
         // of persist.cuh); no more CTAs than the smallest pair has 16-row
-        // groups (a CTA's energy partial takes one's place).  Autotuning times all forms
+        // groups (a CTA's energy partial takes one's place), if the largest pair's rows then
+        // fit a CTA.  Autotuning times all forms
         int np = 0, ng = kSmallCtas;
         for (const PairDesc &d : c.hpd) {
           np = std::max(np, d.Npad);
@@ -1870,10 +1871,11 @@ extern "C" int lddmm_ctx_launch_config(const lddmm_ctx *c, int *o) {
 
 extern "C" int lddmm_ctx_launch_shape(const lddmm_ctx *c, int *o, int n) {
   if (!c || !o || n < 0) return LDDMM_ERR_ARG;
-  const long long v[11] = {c->S_shoot, c->S_adj, c->S_vfd, c->tpw_shoot, c->tpw_adj,
+  const long long v[12] = {c->S_shoot, c->S_adj, c->S_vfd, c->tpw_shoot, c->tpw_adj,
                            c->persistent ? (c->pers_kind == 1 ? 2 : 1) : 0, c->pers_C, c->pers_cl_ctas,
-                           c->pers_ctas, c->pers_cl_share, c->pers_l2_share};
-  const int k = std::min(n, 11);
+                           c->pers_ctas, c->pers_cl_share, c->pers_l2_share,
+                           c->persistent && c->pers_kind == 2 ? c->small_C : 0};
+  const int k = std::min(n, 12);
   for (int i = 0; i < k; ++i) o[i] = (int)v[i];
   return k;
 }

@@ -117,3 +117,17 @@ def test_row_tiles_of_many_pairs(oracle):
         fo, go = oracle.objgrd(Ps[k], alp[k])
         assert abs(f[k] - fo) <= TOL * abs(fo)
         assert rel(g[k], go) < TOL
+
+
+@pytest.mark.parametrize("sizes,ctas", [((5,), 4), ((64,), 4), ((65, 250), 8),
+                                        ((65, 300), 0), ((128,), 8), ((257,), 16), ((512,), 16),
+                                        ((513,), 0)])
+def test_the_small_form_runs_where_it_should(sizes, ctas):
+    """The rule without tuning: pairs of at most 512 points, as many CTAs as the smallest pair
+    has 16-row groups of 64-row padding, at most 16, if the largest pair's rows then fit a CTA
+    (32, of 16 threads each)."""
+    from lddmm_b200 import api, problem
+
+    with api.Context([problem.circle_to_square(n, 40, 0.5) for n in sizes], autotune=False) as ctx:
+        shape = ctx.launch_shape()
+    assert shape["persistent"] == 1 and shape["small_ctas"] == ctas
