@@ -1216,8 +1216,21 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
     total += cp;
     c.grid_dmax = std::max(c.grid_dmax, (int)rmax);
   }
+  if (pairs.empty()) return 0;
+  {
+    cudaError_t e = dalloc(c.stream, &c.graw, (size_t)total * 6);
+    if (e == cudaSuccess) e = dalloc(c.stream, &c.gfld, (size_t)total * 6);
+    if (e == cudaErrorMemoryAllocation) {  // the pair sums need none of it
+      cudaGetLastError();
+      dfree(c.graw, c.stream);
+      dfree(c.gfld, c.stream);
+      c.graw = nullptr;
+      c.gfld = nullptr;
+      return 0;
+    }
+    CU(e);
+  }
   c.n_grid = (int)pairs.size();
-  if (!c.n_grid) return 0;
   std::vector<int2> blk, tile[2];
   for (int p : pairs) {
     const int nb = c.hpd[p].Npad / 32;
@@ -1251,8 +1264,6 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
   CU(dalloc(c.stream, &c.gkeys, (size_t)(c.T + 1) * c.P * 6));
   CU(cudaMemsetAsync(c.gkeys, 0xff, sizeof(unsigned) * (size_t)(c.T + 1) * c.P * 6, c.stream));
   CU(dalloc(c.stream, &c.gmax, (size_t)2 * c.T * c.P));
-  CU(dalloc(c.stream, &c.graw, (size_t)total * 6));
-  CU(dalloc(c.stream, &c.gfld, (size_t)total * 6));
   CU(cudaStreamSynchronize(c.stream));  // the host arrays go out of scope
   c.grid = true;
   return 0;
