@@ -38,6 +38,7 @@ namespace lddmm {
 constexpr int kGridMaxDim = 112;  // nodes per axis: a plane of doubles fits shared memory
 constexpr int kGridKZ = 16;       // z nodes handled at once in registers
 constexpr int kGridThreads = 128;
+constexpr int kSpreadPts = 32;    // points of a spread tile
 constexpr int kConvThreads = 256;
 constexpr int kInterpWarps = 4;
 
@@ -88,29 +89,30 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 
 // ------------------------------------------------------------------------ spread
 //
-// A CTA takes a tile of 32 or 128 points that are close in space (k-d order of the initial
+// A CTA takes a tile of 32 points that are close in space (k-d order of the initial
 // positions).  For a plane m of x nodes and 8 rows n of y nodes,
 //   S_c(n, k) = sum_p [psi_m psi_n a_c](p) psi_k(p)
 // is an (8 x points) x (points x 16 z nodes) product for each of the 3 momenta
 // components, on the FP64 tensor cores: the left operand is formed in registers, the
-// right one holds the points' z windows.  A node receives one atomic per tile.
+// right one holds the points' z windows.  A node receives one atomic per tile.  (128 points per
+// tile take fewer atomics but scan four times the points for each of their nodes: shooting
+// steps of 40,962 / 163,842 / 655,362 landmarks 234 / 428 / 1186 us, with 32 points 162 / 334 /
+// 1120.)
 
-template <int TPTS>
 struct GridSpreadSmem {
-  double w[2][kWin][TPTS];        // x and y windows
-  double z[kWin][TPTS];
-  double zw[TPTS][kGridKZ + 4];   // z windows over the current nodes, zero outside
-  float a[6][TPTS];
-  int o[3][TPTS];
+  double w[2][kWin][kSpreadPts];       // x and y windows
+  double z[kWin][kSpreadPts];
+  double zw[kSpreadPts][kGridKZ + 4];   // z windows over the current nodes, zero outside
+  float a[6][kSpreadPts];
+  int o[3][kSpreadPts];
   int lo[3], hi[3];
 };
 
-template <int TPTS>
 __global__ void __launch_bounds__(kGridThreads)
     grid_spread_kernel(const GridArgs A, const float4 *s0, const float4 *s1,
                        const double *__restrict__ q64, int adj) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  GridSpreadSmem<TPTS> &sm = *reinterpret_cast<GridSpreadSmem<TPTS> *>(smem_raw);
+  GridSpreadSmem &sm = *reinterpret_cast<GridSpreadSmem *>(smem_raw);
   const int2 it = A.blocks[blockIdx.x];
   pdl_wait();
   pdl_trigger();
@@ -120,14 +122,14 @@ __global__ void __launch_bounds__(kGridThreads)
   if (!grid_active(A, p, adj != 0, g)) return;
   const PairDesc &P = A.pd[p];
   const int row0 = it.y * 32;
-  const int npt = min(TPTS, P.N - row0);
+  const int npt = min(kSpreadPts, P.N - row0);
   if (npt <= 0) return;
   if (tid < 3) {
     sm.lo[tid] = 1 << 20;
     sm.hi[tid] = -1;
   }
   const int *ord = A.ord + P.pt_off + row0;
-  for (int i = tid; i < TPTS; i += kGridThreads) {
+  for (int i = tid; i < kSpreadPts; i += kGridThreads) {
     const int g0 = i < npt ? P.pt_off + ord[i] : 0;
     float4 a = make_float4(0, 0, 0, 0), b = a;
     if (i < npt) {
@@ -138,11 +140,11 @@ __global__ void __launch_bounds__(kGridThreads)
     sm.a[3][i] = b.x; sm.a[4][i] = b.y; sm.a[5][i] = b.z;
   }
   __syncthreads();
-  for (int i = tid; i < 3 * TPTS; i += kGridThreads) {
-    const int axis = i / TPTS, pt = i - axis * TPTS;
+  for (int i = tid; i < 3 * kSpreadPts; i += kGridThreads) {
+    const int axis = i / kSpreadPts, pt = i - axis * kSpreadPts;
     const int src = min(pt, npt - 1);  // padding repeats the last point, with a = 0
     const double x = __ldcg(&q64[(size_t)(P.pt_off + ord[src]) * 3 + axis]) * P.kscale64;
-    grid_windows<false>(A.tab, x, pt, TPTS, g.f[axis], g.n[axis],
+    grid_windows<false>(A.tab, x, pt, kSpreadPts, g.f[axis], g.n[axis],
                         axis == 2 ? &sm.z[0][0] : &sm.w[axis][0][0], nullptr, sm.o[axis]);
     const int o = sm.o[axis][pt];
     atomicMin(&sm.lo[axis], o);
@@ -156,7 +158,7 @@ __global__ void __launch_bounds__(kGridThreads)
   const double sca = scalbn(1.0, grid_scale_exp(P.N, __ldcg(&A.amax[p])));
   const double scu = s1 ? scalbn(1.0, grid_scale_exp(P.N, __ldcg(&A.umax[p]))) : 0.0;
   for (int z0 = sm.lo[2]; z0 < hz; z0 += kGridKZ) {
-    for (int i = tid; i < TPTS * kGridKZ; i += kGridThreads) {
+    for (int i = tid; i < kSpreadPts * kGridKZ; i += kGridThreads) {
       const int pt = i / kGridKZ, k = i - pt * kGridKZ;
       const int q = z0 + k - sm.o[2][pt];
       sm.zw[pt][k] = (q >= 0 && q < kWin) ? sm.z[q][pt] : 0.0;

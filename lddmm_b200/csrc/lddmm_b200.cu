@@ -196,8 +196,8 @@ struct lddmm_ctx {
   // gridded kernel sums of large pairs (grid.cuh)
   bool grid = false;
   int n_grid = 0, grid_dmax = 0;        // pairs with a grid, largest extent per axis
-  int n_gblk = 0, n_gtile[2] = {0, 0};  // 32-point blocks; spread tiles of 32 / 128 points
-  int2 *gblk = nullptr, *gtile[2] = {nullptr, nullptr};
+  int n_gblk = 0;  // 32-point tiles
+  int2 *gblk = nullptr;
   int *gpairs = nullptr, *gslot = nullptr, *gord = nullptr;
   long long *goff = nullptr, *gcap = nullptr;
   unsigned *gkeys = nullptr, *gmax = nullptr;  // box keys [T + 1][P][6]; max |a|, |u| [2][T][P]
@@ -288,7 +288,7 @@ lddmm_ctx::~lddmm_ctx() {
   dfree(dbb, stream); dfree(tbb, stream);
   dfree(gbox, stream); dfree(gwa, stream); dfree(gwu, stream); dfree(gpart, stream);
   dfree(gcnt, stream); dfree(vpart, stream); dfree(vcnt, stream);
-  dfree(gblk, stream); dfree(gtile[0], stream); dfree(gtile[1], stream); dfree(gpairs, stream);
+  dfree(gblk, stream); dfree(gpairs, stream);
   dfree(gslot, stream); dfree(gord, stream); dfree(goff, stream); dfree(gcap, stream); dfree(gkeys, stream);
   dfree(gmax, stream); dfree(graw, stream); dfree(gfld, stream); dfree(gtab, stream);
   if (own_stream && stream) cudaStreamDestroy(stream);
@@ -403,10 +403,8 @@ static cudaError_t grid_attributes() {
   const int cs = (int)(sizeof(double) * (2 * kGridMaxDim + 2 + 2 * kGridMaxDim * (kGridMaxDim + 1)));
   CUE(cudaFuncSetAttribute(grid_conv_yz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
   CUE(cudaFuncSetAttribute(grid_conv_x_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cs));
-  CUE(cudaFuncSetAttribute(grid_spread_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(GridSpreadSmem<128>)));
-  CUE(cudaFuncSetAttribute(grid_spread_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(GridSpreadSmem<32>)));
+  CUE(cudaFuncSetAttribute(grid_spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(GridSpreadSmem)));
   CUE(cudaFuncSetAttribute(grid_interp_kernel<false, ShootOp<3, -1>>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)sizeof(GridInterpSmem<false>)));
@@ -421,16 +419,8 @@ static cudaError_t grid_attributes() {
 static cudaError_t grid_spread(lddmm_ctx &c, int t, const float4 *a, const float4 *u) {
   const GridArgs A = grid_args(c, t);
   const double *q = c.q64 + (size_t)t * c.NPtot * 3;
-  for (int k = 0; k < 2; ++k) {
-    if (!c.n_gtile[k]) continue;
-    GridArgs B = A;
-    B.blocks = c.gtile[k];
-    CUE(launch_smem(k ? grid_spread_kernel<128> : grid_spread_kernel<32>,
-                    dim3((unsigned)c.n_gtile[k]), kGridThreads, 0,
-                    k ? sizeof(GridSpreadSmem<128>) : sizeof(GridSpreadSmem<32>), c.stream, B, a, u,
-                    q, u ? 1 : 0));
-  }
-  return cudaSuccess;
+  return launch_smem(grid_spread_kernel, dim3((unsigned)c.n_gblk), kGridThreads, 0,
+                     sizeof(GridSpreadSmem), c.stream, A, a, u, q, u ? 1 : 0);
 }
 
 // Convolve them: fields of 3 (6) components.  For pairs that the step does not fit: the block
@@ -1231,12 +1221,10 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
     CU(e);
   }
   c.n_grid = (int)pairs.size();
-  std::vector<int2> blk, tile[2];
+  std::vector<int2> blk;
   for (int p : pairs) {
     const int nb = c.hpd[p].Npad / 32;
     for (int k = 0; k < nb; ++k) blk.push_back(make_int2(p, k));
-    const int big = c.hpd[p].N >= 100000 ? 1 : 0;  // 128-point spread tiles
-    for (int k = 0; k < nb; k += big ? 4 : 1) tile[big].push_back(make_int2(p, k));
   }
   c.n_gblk = (int)blk.size();
   std::vector<int> ord(c.NPtot, 0);
@@ -1251,10 +1239,6 @@ static int setup_grid(lddmm_ctx &c, const lddmm_problem *probs) {
   };
   CU(grid_attributes());
   CU(put(&c.gblk, blk));
-  for (int k = 0; k < 2; ++k) {
-    c.n_gtile[k] = (int)tile[k].size();
-    CU(put(&c.gtile[k], tile[k]));
-  }
   CU(put(&c.gpairs, pairs));
   CU(put(&c.gslot, slot));
   CU(put(&c.gord, ord));
