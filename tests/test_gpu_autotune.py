@@ -106,4 +106,4 @@ def test_contexts_of_other_widths_are_tuned_again():
     seconds(P)
     again = min(seconds(P) for _ in range(3))
     assert seconds(other) > 1.5 * again
-    assert seconds(other) < 1.5 * again
+    assert min(seconds(other) for _ in range(3)) < 1.5 * again

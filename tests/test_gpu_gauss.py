@@ -105,6 +105,32 @@ def test_gridded_sums_against_fp64(n):
             assert np.max(np.abs(P.time_stp * dq - step)) < 1e-7 * np.max(np.abs(pst[t]))
 
 
+def test_gridded_sums_of_the_large_pair():
+    """163,842 landmarks, all steps on the grid: velocities and gradients of a row sample
+    against FP64 sums.  Tolerance as above."""
+    import ctypes as C
+
+    import torch
+
+    from lddmm_b200 import _lib, api, problem
+
+    P = problem.star_pair(time_num=4)
+    a = np.random.default_rng(1).normal(size=(P.T, P.nde_num, 3)) * 2e-4 + 1e-4 * P.ini_nde
+    with api.Context(P) as ctx:
+        (q, v), = ctx.shoot(a.reshape(-1))
+        d = torch.from_numpy(a.reshape(-1)).cuda()
+        f, g, pst = torch.empty(1, dtype=torch.float64, device="cuda"), d.clone(), d.clone()
+        _lib.check(_lib.lib.lddmm_objgrd_costate(
+            ctx.handle, *[C.c_void_p(x.data_ptr()) for x in (d, f, g, pst)]))
+    g, pst = (x.cpu().numpy().reshape(a.shape) for x in (g, pst))
+    rows = np.random.default_rng(2).integers(0, P.nde_num, 40)
+    for t in range(P.T):
+        K = np.exp(-((q[t][rows][:, None] - q[t][None]) ** 2).sum(-1) / P.knl_width ** 2)
+        u = a[t] - pst[t]
+        assert np.max(np.abs(K @ a[t] - v[t][rows])) < 1e-7 * np.max(np.abs(v[t]))
+        assert np.max(np.abs(P.time_stp * K @ u - g[t][rows])) < 1e-7 * np.max(np.abs(g[t]))
+
+
 def test_gridded_sums_of_huge_momenta():
     """Finite momenta whose largest value times N exceeds the largest float: the first step
     still runs on the grid (later ones outgrow it).  Tolerance as above."""
