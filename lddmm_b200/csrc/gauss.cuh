@@ -399,11 +399,14 @@ __global__ void __launch_bounds__(W * 32, 4)
     while (s < nblk) {
       __syncwarp();
       {
-        const float x = nq.x - T.c[0], y = nq.y - T.c[1], z = nq.z - T.c[2];
+        float x = nq.x - T.c[0], y = nq.y - T.c[1], z = nq.z - T.c[2];
+        const float r2 = fmaf(z, z, fmaf(y, y, x * x));
+        // a point at infinity: K = 2^-inf in the expanded exponent too, not inf - inf
+        if (T.compact && r2 == INFINITY) x = y = z = 0.0f;
         sj[0][lane] = x;
         sj[1][lane] = y;
         sj[2][lane] = z;
-        sj[3][lane] = -fmaf(z, z, fmaf(y, y, x * x));
+        sj[3][lane] = -r2;
         sj[4][lane] = na.x;
         sj[5][lane] = na.y;
         sj[6][lane] = na.z;

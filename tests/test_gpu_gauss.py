@@ -331,3 +331,18 @@ def test_single_sums_prepare_no_grid(kind):
         return min(t)
 
     assert ms(-1) < 1.5 * ms(1)
+
+
+@pytest.mark.parametrize("far", [np.inf, -np.inf, 1e30])
+def test_a_point_at_infinity_adds_nothing(far):
+    """Beyond the persistent forms' sizes: K of a point at infinity is 0, for every other row."""
+    from lddmm_b200 import api
+
+    rng = np.random.default_rng(6)
+    q, a = rng.normal(size=(2, 10500, 3))
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    q = q[np.argsort(q[:, 2])]  # compact tiles
+    v0 = api.multiplyKernel(np.delete(q, 7000, 0), np.delete(a, 7000, 0), -1, 1.0)
+    q[7000, 1] = far
+    v = np.delete(api.multiplyKernel(q, a, -1, 1.0), 7000, 0)
+    assert rel(v, v0) < 1e-6
