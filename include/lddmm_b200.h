@@ -40,8 +40,7 @@
  * independent.  Process-wide state, all of it guarded or per thread: the error
  * message (per host thread), one stream-ordered device memory pool per device from
  * which contexts take their memory (guarded by a mutex), and the fixed device array of
- * lddmm_multiply_kernel_noalloc with its cached per-device address.  Creating a context
- * sorts large meshes in up to 16 host threads that end before it returns.
+ * lddmm_multiply_kernel_noalloc with its cached per-device address.
  */
 #ifndef LDDMM_B200_H
 #define LDDMM_B200_H
