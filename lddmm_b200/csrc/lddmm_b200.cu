@@ -1154,7 +1154,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf);
 // sweeps (40,962 landmarks: 1.92 ms); on the grid 2,500 per landmark, the latency of four
 // dependent launches per sweep (22 M: 80 us of 148 SMs) and the convolutions, 9 fields x
 // 3 axes x about 53 taps per node at 64 per clock (20,011 landmarks: 0.28 ms against 0.46,
-// 40,962: 0.42, 163,842: 1.27 against 32).  The grid must win by a tenth: from about
+// 40,962: 0.46 against 1.92, 163,842: 1.09 against 32).  The grid must win by a tenth: from about
 // 15,000 landmarks on for a unit shape at kernel width 0.3.
 //
 // Room: a registration ends near its target, so an axis may hold 1.35 times the source's
