@@ -61,8 +61,12 @@ void set_err(const char *fmt, ...) {
   } while (0)
 
 constexpr int kWarps = 4;  // warps per sweep CTA
-// persistent sweeps are chosen automatically up to this many row groups per resident CTA
-constexpr int kPersistAutoUnits = 2;
+// persistent sweeps are the rule up to kPersistAutoUnits row groups of 16 rows per resident CTA
+// and, tuned, a candidate up to twice as many.  Evaluations, persistent / per-step launches: 30 pairs
+// of 620 landmarks (3D Gaussian) 0.50 / 0.93 ms, 8 pairs of 2,562 1.06 / 1.47 (Matern 1.22 /
+// 1.45), one of 13,500 2.73 / 3.07, Matern pairs of 20,000 6.88 / 7.02 and 30,000 15.1 / 14.7,
+// 16 Gaussian pairs of 2,562 2.05 / 2.35
+constexpr int kPersistAutoUnits = 5;
 // polls of the wait self-test's barrier before it gives up (about a second)
 constexpr unsigned int kSelftestSpin = 1u << 20;
 
@@ -487,9 +491,9 @@ static cudaError_t shoot_impl(lddmm_ctx &c, int t, double *vlc) {
   // work items (c.tpw_shoot; the default rule and the autotuner pick it).  Two tiles
   // per item serve four rows per lane from each staged column; the Matern kernels, with a
   // square root per pair and fewer CTAs per SM at the larger register count, were faster
-  // on single tiles (40,962: 1.02 vs 1.10 ms).  3D Gaussian shooting never comes here.
-  if constexpr (D == 3 && ORDER == -1) return cudaErrorNotSupported;
-  else if (c.tpw_shoot == 2)
+  // on single tiles (40,962: 1.02 vs 1.10 ms).  3D Gaussian pairs come here where tuning
+  // finds it faster than gauss.cuh (many small meshes in no spatial order).
+  if (c.tpw_shoot == 2)
     return launch(sweep_packed_kernel<ShootOp<D, ORDER>, kWarps, 2>,
                   (unsigned)(c.n_pt_items2 * c.S_shoot), kWarps * 32, c.S_shoot, c.stream, op,
                   (const int2 *)c.pt_items2, c.S_shoot);
@@ -1682,9 +1686,10 @@ static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *c
     const int cap = std::min(b0, b1) * sms;
     // automatic: up to a few row groups per resident CTA the persistent sweep wins (a
     // step is a few microseconds and the plan balances any row-group count); bigger
-    // batches keep per-step launches, whose 64-row tiles are cheaper per pair
+    // batches keep per-step launches, which also skip finished pairs' work
     c.persistent = cap > 0 && (cf.persistent > 0 ||
-                               (cf.persistent == 0 && c.n_units <= kPersistAutoUnits * cap));
+                               (cf.persistent == 0 &&
+                                c.n_units <= kPersistAutoUnits * cap * (cf.autotune < 0 ? 1 : 2)));
     CU(dalloc(c.stream, &c.sync, 1));
     CU(cudaMemsetAsync(c.sync, 0, sizeof(StepSync), c.stream));
     if (c.persistent) {
@@ -1789,23 +1794,29 @@ static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *c
     }
   }
   if (c.D == 3 && c.order == -1 && (use == Use::kRegistration || use == Use::kMultiply)) {
-    // 3D Gaussian per-step sweeps: S independent CTAs per 128-row item (default 8: at
-    // 9,001 / 40,962 / 163,842 landmarks 8 is within 3 % of the best of 1..32; fewer
-    // leave SMs idle at the end of a sweep, 1: 119 / 859 / 7065 us per shooting step
-    // against 47 / 510 / 6096)
+    // 3D Gaussian per-step sweeps: S independent CTAs per 128-row item.  8 from 4,096 points
+    // in the largest pair on (at 9,001 / 40,962 / 163,842 landmarks within 3 % of the best of
+    // 1..32; fewer leave SMs idle at the end of a sweep, 1: 119 / 859 / 7065 us per shooting
+    // step against 47 / 510 / 6096); of smaller pairs the 32 warps of such a split have less
+    // than a few blocks each (30 pairs of 620 landmarks, S = 2 / 8: 23 / 27 us shooting, 33 /
+    // 45 adjoint)
     const size_t nb = (size_t)c.NPtot / kSub;
-    if (cf.cluster_shoot <= 0) c.S_shoot = 8;
-    if (cf.cluster_adjoint <= 0) c.S_adj = 8;
+    int np = 0;
+    for (const PairDesc &d : c.hpd) np = std::max(np, d.Npad);
+    const int split = np < 2048 ? 2 : np < 4096 ? 4 : 8;
+    if (cf.cluster_shoot <= 0) c.S_shoot = split;
+    if (cf.cluster_adjoint <= 0) c.S_adj = split;
     CU(dalloc(c.stream, &c.gbox, 2 * nb * (c.T + 1)));
     CU(dalloc(c.stream, &c.gwa, nb * c.T));
     CU(dalloc(c.stream, &c.gwu, 2 * nb));
-    CU(dalloc(c.stream, &c.gpart, (size_t)c.n_pt_items2 * std::max(c.S_shoot, c.S_adj) *
-                                      kGaussRows * AdjointOp<3, -1>::NA));
+    CU(dalloc(c.stream, &c.gpart,
+              (size_t)c.n_pt_items2 * 8 * kGaussRows * AdjointOp<3, -1>::NA));
     CU(dalloc(c.stream, &c.gcnt, c.n_pt_items2));
     c.gauss = true;
     if (use == Use::kRegistration && cf.persistent <= 0) {
       const int rc = setup_grid(c, probs);
       if (rc) return rc;
+      if (c.grid && cf.autotune < 0) c.persistent = false;  // (tuned: by their times)
     }
     CU(launch(gauss_box_kernel, (unsigned)((nb + 3) / 4), 128, 0, c.stream, (const float4 *)c.qs,
               (const int *)c.pt_pair, (int)nb, c.gbox, c.gkeys));
@@ -2536,7 +2547,7 @@ extern "C" int lddmm_ctx_time_sweeps(lddmm_ctx *ctx, int reps, double *ms4) {
 // Choices of the autotuner, cached per launch signature for the life of the process
 // (a later context of the same shapes starts with them, without timing anything).
 struct TuneChoice {
-  int S_shoot, S_adj, S_vfd, tpw_shoot, tpw_adj, persistent, pers_kind;
+  int S_shoot, S_adj, S_vfd, tpw_shoot, tpw_adj, persistent, pers_kind, gauss;
 };
 static std::mutex g_tune_mu;
 static std::map<std::string, TuneChoice> g_tune_cache;
@@ -2610,8 +2621,8 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
   // The launch shape of each sweep, chosen by timing the candidates on this batch, with
   // momenta of one magnitude (zeros would switch the Gaussian sweeps' distance test off):
   // per-step shooting and adjoint sweeps over one or two 64-row tiles per work item and a
-  // cluster split S of 1, 2, 4 or 8 CTAs per item (the 3D Gaussian ones keep theirs); the
-  // varifold sweep over S = 1..8; and, for a batch on the persistent time-loop sweeps, their
+  // cluster split S of 1, 2, 4 or 8 CTAs per item (3D Gaussian: gauss.cuh's and the general
+  // ones); the varifold sweep over S = 1..8; and, for a batch on the persistent time-loop sweeps, their
   // L2 and small forms (the cluster form where it is asked for) against T per-step launches
   // of the tuned shape.  Sizes given in the configuration are kept.  Every candidate gives the same
   // sums up to the order in which a cluster's partial sums are added (two-tile items
@@ -2625,6 +2636,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
       c.S_shoot = t.S_shoot; c.S_adj = t.S_adj; c.S_vfd = t.S_vfd;
       c.tpw_shoot = t.tpw_shoot; c.tpw_adj = t.tpw_adj; c.persistent = t.persistent != 0;
       c.pers_kind = t.pers_kind;
+      c.gauss = c.gauss && t.gauss != 0;
       return 0;
     }
   }
@@ -2635,10 +2647,10 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
   CU(cudaEventCreate(&e1));
   const int reps = 3;
   cudaError_t err = cudaSuccess;
-  auto tune_step = [&](int which, int *S, int *tpw, bool fixS) {
+  auto tune_step = [&](int which, int *S, int *tpw, bool fixS) {  // the best time, ms
     float best = 1e30f;
     int bS = *S, bT = *tpw;
-    for (int T2 = 1; T2 <= 2 && err == cudaSuccess; ++T2)
+    for (int T2 = c.gauss ? 2 : 1; T2 <= 2 && err == cudaSuccess; ++T2)
       for (int Sc : {1, 2, 4, 8}) {
         if (fixS && Sc != bS) continue;
         *S = Sc;
@@ -2656,10 +2668,32 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
       }
     *S = bS;
     *tpw = bT;
+    return best;
   };
-  if (!c.gauss && c.use != Use::kVarifold) {
-    if (c.use != Use::kDq) tune_step(0, &c.S_shoot, &c.tpw_shoot, cf.cluster_shoot > 0);
-    tune_step(1, &c.S_adj, &c.tpw_adj, cf.cluster_adjoint > 0);
+  // (splits of the 3D Gaussian sweeps: of pairs up to 16,384 points, not beside a grid)
+  int np = 0;
+  for (const PairDesc &d : c.hpd) np = std::max(np, d.Npad);
+  if (c.use != Use::kVarifold && !(c.gauss && (c.grid || np > 16384 || cf.persistent > 0))) {
+    auto both = [&]() {
+      const float s = c.use != Use::kDq
+                          ? tune_step(0, &c.S_shoot, &c.tpw_shoot, cf.cluster_shoot > 0) : 0.0f;
+      return s + tune_step(1, &c.S_adj, &c.tpw_adj, cf.cluster_adjoint > 0);
+    };
+    const float ms = both();
+    if (c.gauss) {
+      // against the general packed sweeps: tiles of meshes in no spatial order are not compact,
+      // and 120 pairs of 620 such landmarks take 64 / 132 us per shooting / adjoint step with
+      // gauss.cuh, 60 / 113 with these (one of 10,000 in spatial order: 66 / 121 and 64 / 127)
+      const int keep[4] = {c.S_shoot, c.S_adj, c.tpw_shoot, c.tpw_adj};
+      c.gauss = false;
+      if (both() > 0.97f * ms || err != cudaSuccess) {
+        c.gauss = true;
+        c.S_shoot = keep[0];
+        c.S_adj = keep[1];
+        c.tpw_shoot = keep[2];
+        c.tpw_adj = keep[3];
+      }
+    }
   }
   if (err == cudaSuccess && c.has_vfd && cf.cluster_varifold <= 0) {
     float best = 1e30f;
@@ -2720,7 +2754,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
   CU(cudaStreamSynchronize(c.stream));
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune_cache[key] = TuneChoice{c.S_shoot, c.S_adj, c.S_vfd, c.tpw_shoot, c.tpw_adj,
-                                 c.persistent ? 1 : 0, c.pers_kind};
+                                 c.persistent ? 1 : 0, c.pers_kind, c.gauss ? 1 : 0};
   return 0;
 }
 
