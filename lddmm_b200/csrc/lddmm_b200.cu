@@ -248,7 +248,7 @@ struct lddmm_ctx {
   cudaError_t (*adjoint)(lddmm_ctx &, int t, double *g, double *pdot) = nullptr;
   cudaError_t (*shoot_all)(lddmm_ctx &, double *vlc) = nullptr;
   cudaError_t (*adjoint_all)(lddmm_ctx &, double *g) = nullptr;
-  bool (*small_ok)(int C, int threads, int np) = nullptr;
+  int (*small_clusters)(int C, int threads, int np) = nullptr;
   int (*pers_blocks)(int which) = nullptr;  // resident CTAs per SM of the persistent kernels
   // co-resident clusters of C CTAs of the cluster-form persistent kernels (min of both)
   int (*pers_clusters)(int C, int grid) = nullptr;
@@ -598,9 +598,9 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
   return launch_ex(&cfg, persistent_sweep_kernel<Op>, op, plan, T, dir, c.sync);
 }
 
-// Whether clusters of C CTAs of the small form can run both persistent sweeps.
+// Co-resident clusters of C CTAs of the small form's two sweeps (0: not available).
 template <int D, int ORDER>
-static bool small_ok_impl(int C, int threads, int np) {
+static int small_clusters_impl(int C, int threads, int np) {
   const auto ks = small_sweep_kernel<ShootOp<D, ORDER>>;
   const auto ka = small_sweep_kernel<AdjointOp<D, ORDER>>;
   cudaLaunchConfig_t cfg = {};
@@ -627,7 +627,7 @@ static bool small_ok_impl(int C, int threads, int np) {
   cfg.dynamicSmemBytes = small_smem<AdjointOp<D, ORDER>>(np);
   ok = ok && cudaOccupancyMaxActiveClusters(&b, ka, &cfg) == cudaSuccess;
   if (!ok) cudaGetLastError();
-  return ok && a > 0 && b > 0;
+  return ok ? std::min(a, b) : 0;
 }
 
 template <int D, int ORDER>
@@ -763,7 +763,7 @@ static void set_def(lddmm_ctx &c) {
   c.shoot_all = shoot_all_impl<D, ORDER>;
   c.adjoint_all = adjoint_all_impl<D, ORDER>;
   c.pers_blocks = pers_blocks_impl<D, ORDER>;
-  c.small_ok = small_ok_impl<D, ORDER>;
+  c.small_clusters = small_clusters_impl<D, ORDER>;
   c.pers_clusters = pers_clusters_impl<D, ORDER>;
   c.probe_cluster = probe_cluster_impl<D, ORDER>;
 }
@@ -1771,12 +1771,15 @@ static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *c
         }
         const int C = ng >= 16 ? 16 : ng >= 8 ? 8 : 4;
         const int threads = pad_to((np + C - 1) / C * kSmallLanes, 32);
-        if (np <= kSmallMax && threads <= kSmallMax && 2 * threads >= np &&
-            c.small_ok(C, threads, np)) {
+        const int n = np <= kSmallMax && threads <= kSmallMax && 2 * threads >= np
+                          ? c.small_clusters(C, threads, np) : 0;
+        if (n > 0) {
           c.small_C = C;
           c.small_threads = threads;
           c.small_np = np;
-          c.pers_kind = 2;
+          // untuned, only where all pairs' clusters run at once: 16 pairs of 500 points (two
+          // waves) take 0.70 ms an evaluation this way, 0.29 on the 64-row tiles
+          if (c.P <= n) c.pers_kind = 2;
         }
       }
       if (cf.persistent == 2 && c.pers_C == 0) {

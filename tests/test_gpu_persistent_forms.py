@@ -131,3 +131,13 @@ def test_the_small_form_runs_where_it_should(sizes, ctas):
     with api.Context([problem.circle_to_square(n, 40, 0.5) for n in sizes], autotune=False) as ctx:
         shape = ctx.launch_shape()
     assert shape["persistent"] == 1 and shape["small_ctas"] == ctas
+
+
+def test_the_small_form_is_not_the_rule_beyond_one_wave():
+    """Without tuning, 16 clusters of 16 CTAs would take turns: 16 pairs of 500 points run on
+    the 64-row tiles."""
+    from lddmm_b200 import api, problem
+
+    with api.Context([problem.circle_to_square(500, 40, 0.5)] * 16, autotune=False) as ctx:
+        shape = ctx.launch_shape()
+    assert shape["persistent"] == 1 and shape["small_ctas"] == 0
