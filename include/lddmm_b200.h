@@ -156,11 +156,11 @@ int lddmm_ctx_launch_config(const lddmm_ctx *ctx, int *out3);
 /* Launch shape in use: out[0..2] cluster sizes (shoot, adjoint, varifold), out[3..4]
  * 64-row tiles per work item of the shooting / adjoint sweeps, out[5] the form of
  * the time loops (0 per-step launches, 1 persistent: 64-row tiles whose parts meet in L2,
- * or a cluster per small pair, 2 persistent cluster form); the persistent plans: out[6]
+ * a cluster per small pair or whole 16-row groups, 2 persistent cluster form); the persistent plans: out[6]
  * cluster size and out[7] CTAs of the cluster form (0: unavailable), out[8] CTAs of the
  * L2 form, out[9] / out[10] the largest CTA share (j entries of 16 rows) of the cluster
  * / L2 plan; out[11] CTAs per pair where the time loops run a cluster per small pair, else
- * 0.  Writes at most n values; returns the number written. */
+ * 0; out[12] 1 where they run one whole 16-row group per CTA, else 0.  Writes at most n values; returns the number written. */
 int lddmm_ctx_launch_shape(const lddmm_ctx *ctx, int *out, int n);
 
 /* Objective and gradient of every pair at alp (concatenated, host memory);

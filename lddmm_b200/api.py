@@ -90,13 +90,13 @@ class Context:
         """dict(cluster=(shoot, adjoint, varifold), tiles=(shoot, adjoint),
         persistent=0 | 1 | 2, plans=...): the launch shape the context runs (after
         autotuning); persistent 0: per-step launches, 1: persistent time loops
-        (64-row tiles whose parts meet in L2, or a cluster of small_ctas CTAs per small
-        pair), 2: the cluster form.  plans: the cluster form's cluster size and CTAs, the
+        (64-row tiles whose parts meet in L2; small_ctas not 0: a cluster of so many CTAs
+        per small pair; groups: whole 16-row groups), 2: the cluster form.  plans: the cluster form's cluster size and CTAs, the
         L2 form's CTAs, and each plan's largest CTA share."""
-        o = np.zeros(12, dtype=np.int32)
-        check(lib.lddmm_ctx_launch_shape(self._h, iptr(o), 12))
+        o = np.zeros(13, dtype=np.int32)
+        check(lib.lddmm_ctx_launch_shape(self._h, iptr(o), 13))
         return dict(cluster=tuple(int(x) for x in o[:3]), tiles=(int(o[3]), int(o[4])),
-                    persistent=int(o[5]), small_ctas=int(o[11]),
+                    persistent=int(o[5]), small_ctas=int(o[11]), groups=bool(o[12]),
                     plans=dict(cluster_size=int(o[6]), cluster_ctas=int(o[7]),
                                l2_ctas=int(o[8]), cluster_share=int(o[9]),
                                l2_share=int(o[10])))

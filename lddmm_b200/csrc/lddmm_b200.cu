@@ -162,6 +162,8 @@ struct lddmm_ctx {
   // persistent multi-step sweeps (one cooperative launch per direction)
   bool persistent = false;
   int pers_ctas = 0;          // CTAs of the persistent kernels (one share of work each)
+  // group form (pers_kind 3): one 16-row group per CTA, a candidate of the tuner
+  bool group_ok = false;
   // small form (pers_kind 2): CTAs per pair, threads, points of the largest pair
   int small_C = 0, small_threads = 0, small_np = 0;
   // cluster form of the persistent sweeps (persist.cuh persistent_cluster_kernel):
@@ -249,6 +251,7 @@ struct lddmm_ctx {
   cudaError_t (*shoot_all)(lddmm_ctx &, double *vlc) = nullptr;
   cudaError_t (*adjoint_all)(lddmm_ctx &, double *g) = nullptr;
   int (*small_clusters)(int C, int threads, int np) = nullptr;
+  int (*group_blocks)() = nullptr;
   int (*pers_blocks)(int which) = nullptr;  // resident CTAs per SM of the persistent kernels
   // co-resident clusters of C CTAs of the cluster-form persistent kernels (min of both)
   int (*pers_clusters)(int C, int grid) = nullptr;
@@ -579,6 +582,20 @@ static cudaError_t launch_persistent(lddmm_ctx &c, const Op &op, int dir, int T 
     return launch_smem(small_sweep_kernel<Op>, dim3((unsigned)(c.P * c.small_C)),
                        (unsigned)c.small_threads, c.small_C, small_smem<Op>(c.small_np), c.stream,
                        op, c.small_C, c.small_np, T, dir, c.sync);
+  if constexpr (Op::kGroupForm)
+    if (c.pers_kind == 3) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)c.n_units);
+      cfg.blockDim = dim3(kPersistWarps * 32);
+      cfg.stream = c.stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeCooperative;
+      attr[0].val.cooperative = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      return launch_ex(&cfg, persistent_group_kernel<Op>, op, (const int2 *)c.units, T, dir,
+                       c.sync);
+    }
   SweepPlan plan;
   plan.units = c.pt_items;
   plan.segs = c.segs;
@@ -721,6 +738,20 @@ static int pers_blocks_impl(int which) {
   return e == cudaSuccess ? n : 0;
 }
 
+// The same of the group form (0: this kernel has none).
+template <int D, int ORDER>
+static int group_blocks_impl() {
+  if constexpr (ShootOp<D, ORDER>::kGroupForm) {
+    int a = 0, b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &a, persistent_group_kernel<ShootOp<D, ORDER>>, kPersistWarps * 32, 0) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &b, persistent_group_kernel<AdjointOp<D, ORDER>>, kPersistWarps * 32, 0) == cudaSuccess)
+      return std::min(a, b);
+  }
+  return 0;
+}
+
 template <int D, char CT, char DT>
 static cudaError_t varifold_impl(lddmm_ctx &c) {
   VarifoldOp<D, CT, DT> op;
@@ -764,6 +795,7 @@ static void set_def(lddmm_ctx &c) {
   c.adjoint_all = adjoint_all_impl<D, ORDER>;
   c.pers_blocks = pers_blocks_impl<D, ORDER>;
   c.small_clusters = small_clusters_impl<D, ORDER>;
+  c.group_blocks = group_blocks_impl<D, ORDER>;
   c.pers_clusters = pers_clusters_impl<D, ORDER>;
   c.probe_cluster = probe_cluster_impl<D, ORDER>;
 }
@@ -1757,6 +1789,7 @@ static int create_ctx(const lddmm_problem *probs, int num, const lddmm_config *c
         }
         CU(cudaMemsetAsync(c.sync, 0, sizeof(StepSync), c.stream));
       }
+      c.group_ok = cf.persistent == 0 && c.n_units <= c.group_blocks() * sms;
       if (cf.persistent == 0) {
         // the small form: one cluster per pair of at most 512 points, beyond which a CTA's
         // rows no longer fit its threads (at 200 points a step takes three quarters of the
@@ -1888,11 +1921,12 @@ extern "C" int lddmm_ctx_launch_config(const lddmm_ctx *c, int *o) {
 
 extern "C" int lddmm_ctx_launch_shape(const lddmm_ctx *c, int *o, int n) {
   if (!c || !o || n < 0) return LDDMM_ERR_ARG;
-  const long long v[12] = {c->S_shoot, c->S_adj, c->S_vfd, c->tpw_shoot, c->tpw_adj,
+  const long long v[13] = {c->S_shoot, c->S_adj, c->S_vfd, c->tpw_shoot, c->tpw_adj,
                            c->persistent ? (c->pers_kind == 1 ? 2 : 1) : 0, c->pers_C, c->pers_cl_ctas,
                            c->pers_ctas, c->pers_cl_share, c->pers_l2_share,
-                           c->persistent && c->pers_kind == 2 ? c->small_C : 0};
-  const int k = std::min(n, 12);
+                           c->persistent && c->pers_kind == 2 ? c->small_C : 0,
+                           c->persistent && c->pers_kind == 3 ? 1 : 0};
+  const int k = std::min(n, 13);
   for (int i = 0; i < k; ++i) o[i] = (int)v[i];
   return k;
 }
@@ -2626,7 +2660,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
   // per-step shooting and adjoint sweeps over one or two 64-row tiles per work item and a
   // cluster split S of 1, 2, 4 or 8 CTAs per item (3D Gaussian: gauss.cuh's and the general
   // ones); the varifold sweep over S = 1..8; and, for a batch on the persistent time-loop sweeps, their
-  // L2 and small forms (the cluster form where it is asked for) against T per-step launches
+  // L2, small and group forms (the cluster form where it is asked for) against T per-step launches
   // of the tuned shape.  Sizes given in the configuration are kept.  Every candidate gives the same
   // sums up to the order in which a cluster's partial sums are added (two-tile items
   // are bitwise one-tile items), so the choice affects time only.
@@ -2720,11 +2754,12 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
       }, ms);
     };
     err = reset_sync(c);
-    float mk[3] = {1e30f, 1e30f, 1e30f};
-    for (int kind = 0; kind <= 2 && err == cudaSuccess; ++kind) {
+    float mk[4] = {1e30f, 1e30f, 1e30f, 1e30f};
+    for (int kind = 0; kind <= 3 && err == cudaSuccess; ++kind) {
       if (kind == 0 && cf.persistent == 2) continue;
       if (kind == 1 && cf.persistent != 2) continue;
       if (kind == 2 && !c.small_C) continue;
+      if (kind == 3 && !c.group_ok) continue;
       c.pers_kind = kind;
       err = time_loops(&mk[kind]);
     }
@@ -2736,7 +2771,7 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
         return rc;
       }
     }
-    c.pers_kind = (int)(std::min_element(mk, mk + 3) - mk);
+    c.pers_kind = (int)(std::min_element(mk, mk + 4) - mk);
     if (err == cudaSuccess && cf.persistent == 0) {
       float ms = 0.0f;
       err = time_median(c, e0, e1, reps, [&]() {

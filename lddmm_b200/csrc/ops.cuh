@@ -94,6 +94,7 @@ struct ShootOp {
   static constexpr bool kPacked = true;
   static constexpr int JWP = (D == 3) ? 3 : 2;
   static constexpr int kUnroll = DefKernelOf<D, ORDER>::type::kUnroll;
+  static constexpr bool kGroupForm = D == 2 && ORDER == -1;  // persistent_group_kernel
   struct IData2 {
     float2 q[D];  // (row0, row1)
   };
@@ -361,6 +362,7 @@ struct AdjointOp {
   static constexpr bool kPacked = true;
   static constexpr int JWP = (D == 3) ? 6 : 4;
   static constexpr int kUnroll = DefKernelOf<D, ORDER>::type::kUnroll;
+  static constexpr bool kGroupForm = D == 2 && ORDER == -1;  // persistent_group_kernel
   struct IData2 {
     float2 q[D], l[D], r[D];  // (row0, row1)
   };

@@ -18,8 +18,8 @@
 //     results are bit-reproducible for a given plan.
 //
 // The cluster form (persistent_cluster_kernel) works on row groups of kGroup = 16 rows in
-// rounds of two segments (persist_round), the small form on whole pairs of a few hundred
-// points.
+// rounds of two segments (persist_round), the group form (persistent_group_kernel) on one such
+// group per CTA, the small form on whole pairs of a few hundred points.
 //
 // Grid barrier: a monotonically increasing arrival count (fire-and-forget atomic
 // add) that the CTAs poll against (step + 1) x grid.  When a launch ends, each CTA
@@ -461,6 +461,70 @@ __global__ void __launch_bounds__(kPersistWarps * 32, 2)
             if (lane < 2) o.write_group(0, row0 / kGroup + 2 * warp + lane, lane ? 0.0 : en);
           }
         }
+      }
+    }
+    if (!grid_barrier(sy, (unsigned)(s + 1) * gridDim.x, (unsigned)s)) return;
+  }
+  grid_depart(sy);
+  stamp_exit(sy, dir > 0 ? 0 : 1);
+  pdl_trigger();
+}
+
+// ---------------------------------------------------------------------------------
+// Group form: one whole 16-row group per CTA, no group cut, so that a step ends with the
+// warps' sums, the finalisation and the grid barrier.  For a few hundred to a few thousand
+// points of a cheap kernel, where a step is its latency and the combine of the 64-row tiles'
+// parts a third of it: 2D Gaussian, us per shooting / adjoint step, 64-row tiles -> this: 400
+// points 4.25 / 4.40 -> 3.16 / 3.80, 640 points 4.28 / 4.48 -> 3.53 / 4.21, 8 pairs of 500
+// 4.97 / 5.73 -> 3.89 / 5.05.
+// Beyond one group per resident CTA, or with a costlier pair, the tiles are faster (2D Matern
+// at 500 points: 5.8 / 6.2 us on tiles, 9.9 / 10.4 in whole groups).
+
+template <class Op>
+__global__ void __launch_bounds__(kPersistWarps * 32, 2)
+    persistent_group_kernel(Op op, const int2 *units, int T, int dir, StepSync *sy) {
+  constexpr int JW = Op::JW, NA = Op::NA, NW = kPersistWarps;
+  __shared__ float4 s_j[NW][JW][kSub];
+  __shared__ double s_red[1][NW][kGroup][NA];
+  __shared__ PairDesc s_pd[1];
+  __shared__ int s_uinf[1][2];
+  __shared__ int4 s_seg[1];
+  pdl_wait();
+  stamp_entry(sy, dir > 0 ? 0 : 1);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int2 un = units[blockIdx.x];
+  if (threadIdx.x == 0) {
+    s_uinf[0][0] = un.x | (un.y << 16);
+    s_uinf[0][1] = op.active(un.x);
+    s_pd[0] = op.pd[un.x];
+    s_seg[0] = make_int4(0, 0, op.pd[un.x].Npad, 0);
+  }
+  __syncthreads();
+  const int row = un.y * kGroup + lane;
+  for (int s = 0; s < T; ++s) {
+    Op o = op;
+    o.set_step(dir > 0 ? s : T - 1 - s);
+    persist_round(o, 1, s_seg, s_uinf, s_pd, s_j, s_red);
+    o.pd = s_pd;
+    const bool fin = warp == 0 && lane < kGroup && s_uinf[0][1];
+    typename Op::FData F;  // finalize operands, in flight during the barrier
+    if (fin) o.fin_load(0, row, F);
+    __syncthreads();
+    if (fin) {
+      double v[NA];
+#pragma unroll
+      for (int a = 0; a < NA; ++a) {
+        double x = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) x += s_red[0][w][lane][a];
+        v[a] = x;
+      }
+      double en = o.finalize(0, row, v, F);
+      if (Op::kTileSum) {
+#pragma unroll
+        for (int off = kGroup / 2; off > 0; off >>= 1)
+          en += __shfl_xor_sync(0xffffu, en, off);
+        if (lane == 0) o.write_group(0, un.y, en);
       }
     }
     if (!grid_barrier(sy, (unsigned)(s + 1) * gridDim.x, (unsigned)s)) return;

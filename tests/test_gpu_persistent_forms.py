@@ -141,3 +141,27 @@ def test_the_small_form_is_not_the_rule_beyond_one_wave():
     with api.Context([problem.circle_to_square(500, 40, 0.5)] * 16, autotune=False) as ctx:
         shape = ctx.launch_shape()
     assert shape["persistent"] == 1 and shape["small_ctas"] == 0
+
+
+@pytest.mark.parametrize("sizes", [(400,), (500,), (513,), (640,), (500, 17, 497)])
+def test_whole_row_groups_against_the_oracle(oracle, sizes):
+    """2D Gaussian pairs of a few hundred points, tuned: whole 16-row groups, one per CTA (on one
+    pair of 500 points a seventh faster than the next form).  Tolerance 1e-5, that of every FP32
+    sum of the library; bit for bit the same on a second call."""
+    from lddmm_b200 import api, problem
+
+    Ps = [problem.circle_to_square(n, 40, 0.5) for n in sizes]
+    for P in Ps:
+        P.knl_order = -1
+    alp = [np.random.default_rng(P.nde_num).normal(size=P.var_num) * 0.02 for P in Ps]
+    with api.Context(Ps) as ctx:
+        shape = ctx.launch_shape()
+        f, g = ctx.objgrd(np.concatenate(alp))
+        f2, g2 = ctx.objgrd(np.concatenate(alp))
+    assert sizes != (500,) or shape["groups"], shape
+    assert np.array_equal(f, f2) and np.array_equal(g, g2)
+    g = np.split(g, np.cumsum([P.var_num for P in Ps])[:-1])
+    for k, P in enumerate(Ps):
+        fo, go = oracle.objgrd(P, alp[k])
+        assert abs(f[k] - fo) <= TOL * abs(fo)
+        assert rel(g[k], go) < TOL
