@@ -2597,7 +2597,9 @@ static std::string tune_key(const lddmm_ctx &c, const lddmm_config &cf) {
   add(cf.persistent); add((int)c.use);
   for (const PairDesc &d : c.hpd) {
     add(d.Npad); add(d.Edpad); add(d.Etpad);
-    // the kernel widths: they decide what the sweeps with a distance test skip
+    // the kernel widths: they decide what the sweeps with a distance test skip (not worth
+    // trial sweeps for a single sum)
+    if (c.use != Use::kRegistration) continue;
     for (double w : {d.pd_fac, d.dc_fac}) {
       long long b;
       std::memcpy(&b, &w, sizeof(b));

@@ -126,3 +126,23 @@ def test_tuned_batch_of_small_gaussian_pairs():
     for form in (1, -1):
         assert np.allclose(out[form][0], out[0][0], rtol=1e-6)
         assert mrel(out[form][1], out[0][1]) < 1e-5
+
+
+@pytest.mark.parametrize("kind", ["multiply", "dq"])
+def test_single_sums_of_another_width_are_not_tuned_again(kind):
+    """One sum per call: the trial sweeps of a size serve every kernel width."""
+    import time
+
+    from lddmm_b200 import api
+
+    q, a = np.random.default_rng(3).normal(size=(2, 8900, 3))
+
+    def seconds(width):
+        t0 = time.perf_counter()
+        api.multiplyKernel(q, a, -1, width) if kind == "multiply" else \
+            api.dqKernel(q, a, a, -1, width)
+        return time.perf_counter() - t0
+
+    seconds(0.3)
+    again = min(seconds(0.3) for _ in range(3))
+    assert min(seconds(w) for w in (0.31, 0.32, 0.33)) < 2.0 * again
