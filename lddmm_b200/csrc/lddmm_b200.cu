@@ -2755,10 +2755,13 @@ static int autotune(lddmm_ctx &c, const lddmm_config &cf) {
         return e == cudaSuccess ? c.adjoint_all(c, c.GT) : e;
       }, ms);
     };
-    // (of big batches the first four steps: a first context of 20,000 Matern landmarks is
-    // created in 82 ms instead of 168)
+    // (of 1e8 pairs and more per step, the first four steps: a first context of 20,000 Matern
+    // landmarks is created in 82 ms instead of 168.  With fewer pairs a step is short against
+    // the persistent launch, which only the whole loop repays)
     const int steps = c.T;
-    if (c.n_units > 592) c.T = std::min(c.T, 4);
+    double pairs = 0.0;
+    for (const PairDesc &d : c.hpd) pairs += (double)d.Npad * d.Npad;
+    if (pairs >= 1e8) c.T = std::min(c.T, 4);
     err = reset_sync(c);
     float mk[4] = {1e30f, 1e30f, 1e30f, 1e30f};
     for (int kind = 0; kind <= 3 && err == cudaSuccess; ++kind) {
